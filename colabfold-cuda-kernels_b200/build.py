@@ -1,10 +1,10 @@
 """Builds libcolabfold_cuda_kernels.so for sm_100a in-tree, next to the Python lookup package.
 
     python colabfold-cuda-kernels_b200/build.py [--force]
-    python colabfold-cuda-kernels_b200/build.py --diag CCK_TRACE=1 [--diag CCK_STAGE_REC=1] -o PATH
+    python colabfold-cuda-kernels_b200/build.py --diag CCK_TRACE=1 -o PATH
 
-The second form builds a diagnostics variant of the same sources somewhere else (event trace of one CTA,
-stage records): never the library that the lookup package hands out.
+The second form builds a diagnostics variant of the same sources somewhere else (the event trace of one
+CTA): never the library that the lookup package hands out.
 
 Set CCK_FFI_INCLUDE_DIR to a directory holding xla/ffi/api/ffi.h to also compile the XLA FFI handler
 `MkSample` (csrc/ffi_handler.cu); without it the library exports the plain C ABI only.

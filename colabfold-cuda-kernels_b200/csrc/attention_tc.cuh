@@ -5,13 +5,13 @@
 // group of four softmax warps (one thread per query row), so that the bubbles of one item (its
 // prologue and epilogue, the waits inside a chunk) are filled by the other item's arithmetic on the
 // same SM sub-partitions. Roles:
-//   warps 0 and 10, one thread each   TMA of track 0 and of track 1: the Q tile of an item (128 x 64
+//   warps 0 and 10   TMA of track 0 and of track 1: the Q tile of an item (128 x 64
 //                        columns of QKVG of which 48 are used); per chunk of 64 keys the K tile and the
 //                        transposed V tile from VT into a 3-deep ring (a chunk's tiles are asked for one
 //                        chunk ahead and stay until its P·V is done), and the 128 x 64 tile of pair
 //                        logits into a 2-deep ring of its own, released as soon as the softmax threads
 //                        have read it
-//   warps 1 and 11, one thread each   tcgen05.mma of track 0 and of track 1. One wait per chunk: once
+//   warps 1 and 11   tcgen05.mma of track 0 and of track 1. One wait per chunk: once
 //                        the group's P of chunk g is complete, O += P·V of chunk g (128 x 48, K = 64,
 //                        P read from TMEM) and S = Q·Kᵀ of chunk g + 2 (128 x 64, K = 48) into the S
 //                        buffer that chunk g has just left go out back to back, so S is always a chunk
@@ -106,29 +106,6 @@ __device__ inline void attn_tc_init() {
     }
 }
 
-// has the phase with this parity completed? Never blocks.
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// D[tmem] (+)= A[tmem] · B[smem]ᵀ: A's 128 rows are the TMEM lanes, a 32-bit column holds two
-// consecutive k (16 bf16 of k = 8 columns)
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        :
-        : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 // 16 f32 columns of this warp's 32 TMEM lanes, without the wait
 __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
@@ -201,128 +178,136 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
     const uint32_t tmem = ctl->tmem_base;
     const bool flow = p.flow;
 
-    if ((warp == 0 || warp == kTcTmaWarp1) && lane == 0) {
-        // ---- TMA producer of one track. Issue order: the chunk's pair logits, then K and V of the
-        // chunk after it (their slots free up in that order), then, after an item's last chunk, the
-        // next item's Q tile (free once every Q·Kᵀ of the item is done).
-        const int t = warp != 0;
-        const int n = tc_track_items(first, items, t);
+    if (warp == 0 || warp == kTcTmaWarp1) {
+        // ---- TMA producer of one track (the whole warp passes here, one lane issues: ptx.cuh). Issue order:
+        // the chunk's pair logits, then K and V of the chunk after it (their slots free up in that order),
+        // then, after an item's last chunk, the next item's Q tile (free once every Q·Kᵀ of the item is done).
+        const int t = uni(warp != 0);
+        const int n = uni(tc_track_items(first, items, t)), nchunks = uni(chunks);
         if (n > 0) {
+            const uint32_t el = elect_one();
             TcTrackBars& B = bars->t[t];
-            char* base = sm + t * kTcTrackBytes;
+            const uint32_t base = uni(smem_u32(sm + t * kTcTrackBytes)), bar0 = uni(smem_u32(&B));
+            auto bar = [&](uint64_t& x) { return bar0 + uint32_t(reinterpret_cast<char*>(&x) - reinterpret_cast<char*>(&B)); };
             const CUtensorMap* mqk = &L.tmap[TM_T_QK];
             const CUtensorMap* mvt = &L.tmap[TM_T_VT];
             const CUtensorMap* mpl = &L.tmap[TM_T_PLG];
             const unsigned int qkvg_done = (epoch + 1) * (unsigned int)(gd_table()[GD_TOK_QKVG].nt * kWorkWarps); // (the counters count on through the launch)
-            const uint32_t j0 = bars->items[t], g0 = bars->chunks[t];
-            CCK_TRACE_BEGIN(t);
+            const uint32_t j0 = uni(bars->items[t]), g0 = uni(bars->chunks[t]);
+            const int rows_n = uni(N);
+            CCK_TRACE_BEGIN_IF(t, el);
             int ready = -1; // the sample whose rows of QKVG are known to be complete
-            auto wait_rows = [&](const TcItem& ti) {
-                if (flow && ti.s != ready) {
+            // the item whose tiles are being asked for, as map coordinates
+            int is = 0, ih = 0, qrow = 0, brow = 0;
+            auto set_item = [&](int j) {
+                const TcItem ti = tc_item(tc_track_item(first, t, j), S, qblocks, flow);
+                is = uni(ti.s), ih = uni(ti.h);
+                qrow = is * rows_n + uni(ti.qb) * kTcRows, brow = uni((b * kHeads + ti.h) * npb + ti.qb * kTcRows);
+                if (flow && is != ready) {
                     // every column tile of QKVG over the sample's rows (q, k, v and the gate), and over the
                     // next sample's rows that the last chunk of keys reaches into (masked, but read)
-                    flow_wait(flow_cnt(p, FC_QKVG), ti.s * N / kBM, (min(ti.s * N + np, S * N) - 1) / kBM, qkvg_done, &ctl->abort);
-                    ready = ti.s;
+                    flow_wait(flow_cnt(p, FC_QKVG), is * N / kBM, (min(is * N + np, S * N) - 1) / kBM, qkvg_done, &ctl->abort);
+                    __syncwarp();
+                    ready = is;
                 }
             };
-            auto load_q = [&](const TcItem& ti, uint32_t jg) {
+            auto load_q = [&](uint32_t jg) {
                 mbar_wait(&B.q_empty, (jg & 1) ^ 1, &ctl->abort);
-                mbar_expect_tx(&B.q_full, kTcQBytes);
-                tma_load_2d(base, mqk, ti.h * kHeadD, ti.s * N + ti.qb * kTcRows, &B.q_full);
-                tma_load_2d(base + kTcQBytes / 2, mqk, ti.h * kHeadD, ti.s * N + ti.qb * kTcRows + 64, &B.q_full);
+                mbar_expect_tx_el(el, bar(B.q_full), kTcQBytes);
+                tma_load_2d_el(el, base, mqk, ih * kHeadD, qrow, bar(B.q_full));
+                tma_load_2d_el(el, base + kTcQBytes / 2, mqk, ih * kHeadD, qrow + 64, bar(B.q_full));
             };
-            auto load_kv = [&](const TcItem& ti, int c, uint32_t g) {
-                const uint32_t st = g % kTcKvStages, par = (g / kTcKvStages) & 1;
-                mbar_wait(&B.kv_empty[st], par ^ 1, &ctl->abort);
-                char* ks = base + kTcKvOff + st * kTcKvBytes;
-                mbar_expect_tx(&B.kv_full[st], kTcKvBytes);
-                tma_load_2d(ks, mqk, kTokC + ti.h * kHeadD, ti.s * N + c * kTcKeys, &B.kv_full[st]);
-                tma_load_2d(ks + kTcKBytes, mvt, c * kTcKeys, (ti.s * kHeads + ti.h) * kHeadD, &B.kv_full[st]);
+            uint32_t kst = g0 % kTcKvStages, kpar = (g0 / kTcKvStages) & 1; // the next K|V slot and its phase parity
+            auto load_kv = [&](int c) {
+                mbar_wait(&B.kv_empty[kst], kpar ^ 1, &ctl->abort);
+                const uint32_t ks = base + kTcKvOff + kst * kTcKvBytes, kb = bar(B.kv_full[0]) + 8 * kst;
+                mbar_expect_tx_el(el, kb, kTcKvBytes);
+                tma_load_2d_el(el, ks, mqk, kTokC + ih * kHeadD, is * rows_n + c * kTcKeys, kb);
+                tma_load_2d_el(el, ks + kTcKBytes, mvt, c * kTcKeys, (is * kHeads + ih) * kHeadD, kb);
+                if (++kst == kTcKvStages) {
+                    kst = 0, kpar ^= 1;
+                }
             };
-            auto load_bias = [&](const TcItem& ti, int c, uint32_t g) {
-                const uint32_t st = g % kTcBiasStages, par = (g / kTcBiasStages) & 1;
+            auto load_bias = [&](int c, uint32_t g) {
+                const uint32_t st = g % kTcBiasStages, par = (g / kTcBiasStages) & 1, bb = bar(B.b_full[0]) + 8 * st;
                 mbar_wait(&B.b_empty[st], par ^ 1, &ctl->abort);
-                mbar_expect_tx(&B.b_full[st], kTcBiasBytes);
-                tma_load_2d(base + kTcBiasOff + st * kTcBiasBytes, mpl, c * kTcKeys, (b * kHeads + ti.h) * npb + ti.qb * kTcRows, &B.b_full[st]);
+                mbar_expect_tx_el(el, bb, kTcBiasBytes);
+                tma_load_2d_el(el, base + kTcBiasOff + st * kTcBiasBytes, mpl, c * kTcKeys, brow, bb);
             };
-            TcItem cur = tc_item(tc_track_item(first, t, 0), S, qblocks, flow);
             if (t == 1 && p.attn_skew > 0) { // a test's skew between the pipelines: results must not depend on it
                 const long long t0 = clock64();
                 while (clock64() - t0 < p.attn_skew + 37 * int(blockIdx.x % 64)) {
                 }
+                __syncwarp();
             }
-            wait_rows(cur);
-            load_kv(cur, 0, g0);
-            load_q(cur, j0);
-            CCK_STAMP(0, true);
+            set_item(0);
+            load_kv(0);
+            load_q(j0);
             uint32_t g = g0;
 #pragma unroll 1
             for (int j = 0; j < n; j++) {
 #pragma unroll 1
-                for (int c = 0; c < chunks; c++, g++) {
-                    load_bias(cur, c, g);
+                for (int c = 0; c < nchunks; c++, g++) {
+                    load_bias(c, g);
                     CCK_TRACE_EV(0x10 + t, g - g0);
-                    if (c + 1 < chunks) {
-                        load_kv(cur, c + 1, g + 1);
+                    if (c + 1 < nchunks) {
+                        load_kv(c + 1);
                         CCK_TRACE_EV(0x12 + t, g + 1 - g0);
                     } else if (j + 1 < n) {
-                        cur = tc_item(tc_track_item(first, t, j + 1), S, qblocks, flow);
-                        wait_rows(cur);
-                        load_kv(cur, 0, g + 1);
-                        load_q(cur, j0 + j + 1);
+                        set_item(j + 1);
+                        load_kv(0);
+                        load_q(j0 + j + 1);
                     }
                 }
             }
             CCK_TRACE_END();
         }
-    } else if ((warp == 1 || warp == kTcMmaWarp1) && lane == 0) {
-        // ---- MMA issuer of one track. One wait per chunk: when the group's P of chunk i is complete (and
-        // with it everybody has read S of chunk i), O (+)= P·V of chunk i and S of chunk i + 2 go out
-        // back to back. Everything an MMA needs is prepared: descriptors differ by constants.
-        const int t = warp != 1;
-        const int n = tc_track_items(first, items, t), total = n * chunks;
+    } else if (warp == 1 || warp == kTcMmaWarp1) {
+        // ---- MMA issuer of one track (the whole warp, one lane issues). One wait per chunk: when the group's
+        // P of chunk i is complete (and with it everybody has read S of chunk i), O (+)= P·V of chunk i and S
+        // of chunk i + 2 go out back to back. Everything an MMA needs is prepared: descriptors differ by constants.
+        const int t = uni(warp != 1);
+        const int n = uni(tc_track_items(first, items, t)), nchunks = uni(chunks), total = n * nchunks;
         if (total > 0) {
+            const uint32_t el = elect_one();
             TcTrackBars& B = bars->t[t];
-            char* base = sm + t * kTcTrackBytes;
-            const uint32_t tt = tmem + t * kTcTrackCols;
+            const uint32_t base = uni(smem_u32(sm + t * kTcTrackBytes)), bar0 = uni(smem_u32(&B));
+            auto bar = [&](uint64_t& x) { return bar0 + uint32_t(reinterpret_cast<char*>(&x) - reinterpret_cast<char*>(&B)); };
+            const uint32_t tt = uni(tmem) + t * kTcTrackCols;
             const uint32_t idesc_s = umma_idesc_bf16(kTcRows, kTcKeys), idesc_o = umma_idesc_bf16(kTcRows, kHeadD);
-            const uint32_t j0 = bars->items[t], g0 = bars->chunks[t];
-            const uint64_t dq = umma_desc_sw128(smem_u32(base)), dk0 = umma_desc_sw128(smem_u32(base + kTcKvOff));
+            const uint32_t j0 = uni(bars->items[t]), g0 = uni(bars->chunks[t]);
+            const uint64_t dq = umma_desc_sw128(base), dk0 = umma_desc_sw128(base + kTcKvOff);
             constexpr uint64_t kStageStep = kTcKvBytes >> 4, kVStep = kTcKBytes >> 4; // in the descriptor's address units
-            // the next S to issue: chunk number within the phase, its chunk within the item, its item
+            // the next S to issue: chunk number within the phase, its chunk within the item, its item, its K|V slot
             int qk_i = 0, qk_c = 0, qk_j = 0;
-            uint32_t qk_g = g0;
+            uint32_t qk_g = g0, qk_st = g0 % kTcKvStages, qk_par = (g0 / kTcKvStages) & 1;
             // S of the next chunk = Q·Kᵀ. Its S buffer was read by the whole group (the caller has seen the
             // group's P of the chunk two before complete, or the phase has just begun).
             auto issue_qk = [&]() {
-                const uint32_t st = qk_g % kTcKvStages;
                 if (qk_c == 0) {
                     mbar_wait(&B.q_full, (j0 + uint32_t(qk_j)) & 1, &ctl->abort);
                 }
-                mbar_wait(&B.kv_full[st], (qk_g / kTcKvStages) & 1, &ctl->abort);
-                CCK_STAMP(1, true);
+                mbar_wait(&B.kv_full[qk_st], qk_par, &ctl->abort);
                 tc_fence_after();
-                const uint64_t dk = dk0 + st * kStageStep;
-#pragma unroll
-                for (int kk = 0; kk < kHeadD / 16; kk++) {
-                    umma_bf16(tt + kTcS + (qk_g & 1) * 64, dq + 2 * kk, dk + 2 * kk, idesc_s, kk != 0);
-                }
-                umma_commit(&B.s_full[qk_g & 1]);
+                umma_bf16_k48_el(el, tt + kTcS + (qk_g & 1) * 64, dq, dk0 + qk_st * kStageStep, idesc_s);
+                umma_commit_el(el, bar(B.s_full[0]) + 8 * (qk_g & 1));
                 qk_i++, qk_g++;
-                if (++qk_c == chunks) {
-                    umma_commit(&B.q_empty); // every Q·Kᵀ of the item is issued
+                if (++qk_st == kTcKvStages) {
+                    qk_st = 0, qk_par ^= 1;
+                }
+                if (++qk_c == nchunks) {
+                    umma_commit_el(el, bar(B.q_empty)); // every Q·Kᵀ of the item is issued
                     qk_c = 0, qk_j++;
                 }
             };
-            // S stays two chunks ahead of the softmax. Within the current item the thread waits for what a
+            // S stays two chunks ahead of the softmax. Within the current item the warp waits for what a
             // chunk needs (K lands well ahead); a chunk of the next item goes out ahead only if its Q and K
             // are there already (its sample's rows of QKVG may still be in the making), else when that item starts.
             auto pump = [&](int upto, int item) {
                 while (qk_i < upto && qk_i < total) {
                     if (qk_j != item) {
-                        const bool ready = mbar_test(&B.kv_full[qk_g % kTcKvStages], (qk_g / kTcKvStages) & 1) &&
-                                           (qk_c != 0 || mbar_test(&B.q_full, (j0 + uint32_t(qk_j)) & 1));
-                        if (!ready) {
+                        const bool ready = mbar_test(&B.kv_full[qk_st], qk_par) && (qk_c != 0 || mbar_test(&B.q_full, (j0 + uint32_t(qk_j)) & 1));
+                        if (!uni(int(ready))) {
                             break;
                         }
                     }
@@ -330,32 +315,30 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                 }
             };
             tc_fence_after();
-            uint32_t g = g0;
+            uint32_t g = g0, st = g0 % kTcKvStages;
             int i = 0;
-            CCK_TRACE_BEGIN(2 + t);
+            CCK_TRACE_BEGIN_IF(2 + t, el);
 #pragma unroll 1
             for (int j = 0; j < n; j++) {
                 pump(i + 2, j);
 #pragma unroll 1
-                for (int c = 0; c < chunks; c++, g++, i++) {
-                    const uint32_t bi = g & 1, st = g % kTcKvStages;
+                for (int c = 0; c < nchunks; c++, g++, i++) {
+                    const uint32_t bi = g & 1;
                     mbar_wait(&B.p_full[bi], (g >> 1) & 1, &ctl->abort);
                     tc_fence_after();
                     CCK_TRACE_EV(0x20 + t, i);
-                    const uint64_t dv = dk0 + st * kStageStep + kVStep;
-#pragma unroll
-                    for (int kk = 0; kk < kTcKeys / 16; kk++) {
-                        umma_bf16_ts(tt + kTcO, tt + kTcP + bi * 32 + 8 * kk, dv + 2 * kk, idesc_o, (c | kk) != 0);
-                    }
-                    umma_commit(&B.pv_done[bi]);
-                    umma_commit(&B.kv_empty[st]);
+                    umma_bf16_ts_k64_el(el, tt + kTcO, tt + kTcP + bi * 32, dk0 + st * kStageStep + kVStep, idesc_o, c);
+                    umma_commit_el(el, bar(B.pv_done[0]) + 8 * bi);
+                    umma_commit_el(el, bar(B.kv_empty[0]) + 8 * st);
                     CCK_TRACE_EV(0x22 + t, i);
-                    if (c + 1 == chunks) {
-                        umma_commit(&B.o_full); // the item's O is complete
+                    if (c + 1 == nchunks) {
+                        umma_commit_el(el, bar(B.o_full)); // the item's O is complete
                     }
-                    CCK_STAMP(2, false);
                     pump(i + 3, j);
                     CCK_TRACE_EV(0x24 + t, i);
+                    if (++st == kTcKvStages) {
+                        st = 0;
+                    }
                 }
             }
             CCK_TRACE_END();
@@ -555,9 +538,6 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                 pend_lo = s * N + qb * kTcRows, pend_hi = min(pend_lo + kTcRows, (s + 1) * N) - 1;
             }
             CCK_TRACE_EV(0x3e + t, j);
-            if (threadIdx.x == kWorkWarp0 * 32) {
-                CCK_STAMP(4, false);
-            }
         }
         publish(); // (also: this warp's stores have landed before the phase ends)
         CCK_TRACE_END();

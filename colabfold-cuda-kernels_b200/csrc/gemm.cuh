@@ -1,33 +1,38 @@
 // The dense GEMM engine: C = A·Wᵀ with bf16 operands and f32 accumulation on the 5th-generation
-// tensor cores. Per CTA: one thread feeds a 4-stage shared-memory ring with TMA tile loads, one
-// thread issues tcgen05.mma into a double-buffered TMEM accumulator (2 x 256 columns), and four
-// warps drain finished accumulators with tcgen05.ld and apply the fused epilogue, so the epilogue
-// of tile i overlaps the main loop of tile i+1. Tiles are 128 x bn (bn = 64..256) x 64.
+// tensor cores. Per CTA: one warp feeds a shared-memory ring with TMA tile loads, one warp issues
+// tcgen05.mma into a double-buffered TMEM accumulator (2 x 256 columns), and eight warps drain finished
+// accumulators with tcgen05.ld and apply the fused epilogue, so the epilogue of tile i overlaps the main
+// loop of tile i+1. Tiles are 128 x bn (bn = 64..256) x 64.
+// A main loop runs at the rate of its MMAs when both roles issue from warp-uniform code (ptx.cuh): measured
+// inside the kernel, a k-block went from some 590 cycles at any width to 265 (bn = 128) and 525 (bn = 256).
 //
 // The epilogue kinds restate the reference's (src/diffusion/gemm.cuh:156-325) on a
 // one-thread-per-row accumulator layout.
 #pragma once
 
-#ifndef CCK_EPI_DB
-#define CCK_EPI_DB 0
-#endif
-// CCK_STAGE_REC=1 builds a diagnostics variant: every CTA stamps the moments of its roles inside a
-// phase (first TMA issued, first operands landed, last MMA issued, last accumulator seen, epilogue
-// done, barrier reached, barrier left) and the sums per phase kind are read with mk_stage_rec
-#ifndef CCK_STAGE_REC
-#define CCK_STAGE_REC 0
-#endif
 
 #include "params.cuh"
 #include "ptx.cuh"
 
 namespace cck {
 
-constexpr int kBM = 128, kBK = 64, kStages = 4, kMaxBN = 256;
-constexpr int kStageA = kBM * kBK * 2;        // 16 KB
-constexpr int kStageB = kMaxBN * kBK * 2;     // 32 KB
-constexpr int kStageBytes = kStageA + kStageB;
-constexpr int kPipeBytes = kStages * kStageBytes; // 192 KB
+constexpr int kBM = 128, kBK = 64, kMaxBN = 256;
+constexpr int kStageA = kBM * kBK * 2; // 16 KB
+constexpr int kPipeBytes = 192 << 10;
+// The operand ring: a slot holds one k-block of A and of W. Its size follows the column tile, so that a
+// narrow tile has more k-blocks in flight: the way of a k-block (request, L2, MMA, slot free again) takes
+// some 2200 cycles whatever its width, and with four slots of any width a tile of 64 or 128 columns ran at
+// that time / 4 = 590 cycles per k-block, where its MMAs take 245 or 290.
+constexpr int kMaxSlots = 8;
+__host__ __device__ constexpr int ring_slots(int bn) {
+    return bn > 128 ? 4 : bn > 64 ? 6 : kMaxSlots;
+}
+__host__ __device__ constexpr int ring_slot_bytes(int bn) {
+    return kStageA + bn * kBK * 2;
+}
+static_assert(ring_slots(256) * ring_slot_bytes(256) <= kPipeBytes && ring_slots(192) * ring_slot_bytes(192) <= kPipeBytes &&
+                  ring_slots(128) * ring_slot_bytes(128) <= kPipeBytes && ring_slots(64) * ring_slot_bytes(64) <= kPipeBytes,
+              "the ring outgrew its part of shared memory");
 constexpr int kTmemCols = 512;
 // Warp roles in the tensor-core phases: warp 0 holds the TMA thread, warp 1 the MMA thread, warps
 // 2..9 are the workers that read TMEM (accumulator epilogues, attention softmax). A warp may only
@@ -47,30 +52,14 @@ __device__ __forceinline__ int work_group() {
 
 // shared-memory control block
 struct SmemCtl {
-    uint64_t full[kStages], empty[kStages]; // TMA -> MMA, MMA -> TMA
+    uint64_t full[kMaxSlots], empty[kMaxSlots]; // TMA -> MMA, MMA -> TMA
     uint64_t tfull[2], tempty[2];           // MMA -> epilogue, epilogue -> MMA
     uint32_t tmem_base;
     volatile int abort;
     volatile int quit;                      // the launch has failed somewhere: leave the schedule
     unsigned long long t0;                  // end of the previous phase, ns (timing record, CTA 0)
-#if CCK_STAGE_REC
-    unsigned long long stamp[16], phase_t0;
-#endif
+    int ring_bn;                            // the column tile that the ring's slots are laid out for (TMA thread)
 };
-#if CCK_STAGE_REC
-__device__ unsigned long long g_stage_rec[32][16];
-// SM clock cycles: cheap to read, comparable within one CTA
-__device__ __forceinline__ unsigned long long stage_now() {
-    return (unsigned long long)clock64();
-}
-#define CCK_STAMP(i, first_only)                                                          \
-    do {                                                                                  \
-        SmemCtl* c_ = smem_ctl();                                                         \
-        if (!(first_only) || c_->stamp[i] == 0) c_->stamp[i] = stage_now();               \
-    } while (0)
-#else
-#define CCK_STAMP(i, first_only) do { } while (0)
-#endif
 
 // CCK_TRACE=n builds another diagnostics variant: threads of CTA n - 1 write (cycle, event, value)
 // records of what they pass, each role into its own 2048 slots (no atomics, one store per event), over
@@ -102,17 +91,19 @@ __device__ unsigned int g_barwait[kBarWaitSlots][160]; // [grid barrier][CTA]: c
     do {                                                       \
         if (tr_n_ != 0xffffffffu) g_trace_n[tr_role_] = tr_n_; \
     } while (0)
-#define CCK_TRACE_ONE(role, code, val) \
-    do {                               \
-        CCK_TRACE_BEGIN(role);         \
-        CCK_TRACE_EV(code, val);       \
-        CCK_TRACE_END();               \
+#define CCK_TRACE_ONE_IF(role, code, val, cond) \
+    do {                                        \
+        CCK_TRACE_BEGIN_IF(role, cond);         \
+        CCK_TRACE_EV(code, val);                \
+        CCK_TRACE_END();                        \
     } while (0)
+#define CCK_TRACE_ONE(role, code, val) CCK_TRACE_ONE_IF(role, code, val, true)
 #else
 #define CCK_TRACE_BEGIN_IF(role, cond) do { } while (0)
 #define CCK_TRACE_BEGIN(role) do { } while (0)
 #define CCK_TRACE_EV(code, val) do { } while (0)
 #define CCK_TRACE_END() do { } while (0)
+#define CCK_TRACE_ONE_IF(role, code, val, cond) do { } while (0)
 #define CCK_TRACE_ONE(role, code, val) do { } while (0)
 #endif
 
@@ -170,7 +161,7 @@ __device__ __forceinline__ void fail_launch(unsigned int code, unsigned int wher
 
 // per-thread pipeline positions, kept across phases for the whole launch
 struct Pipe {
-    uint32_t kb = 0;   // k-blocks produced (TMA thread) or consumed (MMA thread)
+    uint32_t ring = 0; // phase parity of each slot of the operand ring, as this role passes them
     uint32_t tile = 0; // accumulator tiles issued (MMA thread) or drained (worker threads)
 };
 
@@ -200,13 +191,13 @@ constexpr int kPiece = 16;
 __device__ __forceinline__ float* epi_stage() {
     return reinterpret_cast<float*>(smem_base() + kEpiOff + (warp_id() - kWorkWarp0) * kEpiStageBytes);
 }
-// row-per-lane values v[16 pc .. 16 pc + 15] -> column-per-lane t[i] (row l / 4 + 8i)
-template <int PC> __device__ __forceinline__ void epi_turn(float* st, const float (&v)[32], float4 (&t)[4]) {
+// row-per-lane values of 16 columns -> column-per-lane t[i] (row l / 4 + 8i)
+__device__ __forceinline__ void epi_turn(float* st, const float* v, float4 (&t)[4]) {
     const int l = lane_id();
     float4* w = reinterpret_cast<float4*>(st + l * kPiece);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        w[i ^ ((l >> 1) & 3)] = make_float4(v[16 * PC + 4 * i], v[16 * PC + 4 * i + 1], v[16 * PC + 4 * i + 2], v[16 * PC + 4 * i + 3]);
+        w[i ^ ((l >> 1) & 3)] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
     }
     __syncwarp();
     const int r = l >> 2, c = l & 3;
@@ -384,9 +375,6 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
                 bnext = c < g.bias_cols ? g.bias[c] : 0.f;
             }
             mbar_wait(tfull, tpar, abort);
-            if (threadIdx.x == kWorkWarp0 * 32) {
-                CCK_STAMP(3, false);
-            }
             tc_fence_after();
 #pragma unroll 1
             for (int u = gp; u < units; u += 2) {
@@ -463,9 +451,6 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
         epi_prefetch<E>(g, oc0 + 32 * gp, cur);
     }
     mbar_wait(tfull, tpar, abort);
-    if (threadIdx.x == kWorkWarp0 * 32) {
-        CCK_STAMP(3, false);
-    }
     tc_fence_after();
 #pragma unroll 1
     for (int u = gp; u < units; u += 2) {
@@ -506,9 +491,9 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
             }
             const EpiUnit eu = epi_unit<E>(g, oc);
             float4 t[4];
-            epi_turn<0>(st, v, t);
+            epi_turn(st, v, t);
             epi_store<E>(g, eu, r0, cl, t, cur.b[0]);
-            epi_turn<1>(st, v, t);
+            epi_turn(st, v + kPiece, t);
             epi_store<E>(g, eu, r0, kPiece + cl, t, cur.b[1]);
         }
         cur = nxt;
@@ -516,128 +501,68 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
 }
 
 // The gated residual update out = src + gate ⊙ C · rowmask. Everything it reads besides the
-// accumulator depends on addresses only, so it is fetched while the main loop runs: the residual
-// rows by cp.async into shared memory that the pipeline leaves free (these GEMMs have bn <= 128, so
-// the upper 16 KB of each stage's 32 KB weight slot is unused; each worker warp owns 8 KB of it,
-// 16 slots of 16 bytes per lane), the gates into registers (bf16) or beside the residual (f32,
-// bn <= 64).
+// accumulator depends on addresses only, so it is fetched into registers while the main loop runs: the
+// residual and the gates of 16 NP columns per warp (group 0 the tile's left half, group 1 its right one), 4
+// rows x 4 columns of a piece of 16 columns per lane. f32 gates (the atom GEMMs) come a piece ahead instead:
+// beside the residual they would not fit.
 constexpr int kResidMaxBnBf = 128, kResidMaxBnF32 = 64;
-__device__ __forceinline__ void cp_async16_cg(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.wait_all;" ::: "memory");
-}
-template <bool GF32>
-__device__ __forceinline__ void resid_tile(const GemmDesc& g, uint32_t acc, int row0, int col0, uint64_t* tfull, uint32_t tpar,
+template <bool GF32, int NP>
+__device__ __forceinline__ void resid_tile(const GemmDesc& g, const void* gate, uint32_t acc, int row0, int col0, uint64_t* tfull, uint32_t tpar,
                                            volatile int* abort) {
-    constexpr int kU = GF32 ? 1 : 2; // units of 32 columns per warp
-    const int q = work_quarter(), gp = work_group(), ww = warp_id() - kWorkWarp0;
+    const int q = work_quarter(), c0 = work_group() * NP * kPiece;
     const int r0 = row0 + q * 32 + (lane_id() >> 2), cl = 4 * (lane_id() & 3);
-    const uint32_t taddr = acc + (uint32_t(q * 32) << 16);
-    float4* area = reinterpret_cast<float4*>(smem_base() + (ww >> 1) * kStageBytes + kStageA + kStageB / 2 + (ww & 1) * 8192) + lane_id();
-    const float* src = static_cast<const float*>(g.out);
-    const int units = g.bn / 32;
-    float m[4];
-    const bf16* gp4[4]; // bf16 gates: this lane's four rows at the tile's first column
+    const uint32_t taddr = acc + (uint32_t(q * 32) << 16) + c0;
+    const int m = g.m, ldo = g.ldo;
+    float* const op = static_cast<float*>(g.out) + col0 + c0 + cl;
+    float4 x[NP][4];
+    float mask[4];
+    uint2 gb[GF32 ? 1 : NP][4];
+    float4 gf[2][4];
+    const char* gp[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const int row = min(r0 + 8 * i, g.m - 1), p = row % g.period;
-        m[i] = g.rowmask ? g.rowmask[p] : 1.f;
-        const float* sp = src + size_t(row) * g.ldo + col0 + cl;
-        const size_t go = size_t(p) * g.ldg + col0 + cl;
-        gp4[i] = static_cast<const bf16*>(g.gate) + go;
+        const int row = min(r0 + 8 * i, m - 1), p = row % g.period;
+        mask[i] = g.rowmask ? g.rowmask[p] : 1.f;
+        gp[i] = static_cast<const char*>(gate) + (size_t(p) * g.ldg + col0 + c0 + cl) * (GF32 ? 4 : 2);
 #pragma unroll
-        for (int k = 0; k < kU; k++) {
-            const int u = gp + 2 * k;
-            if (u < units) {
-#pragma unroll
-                for (int pc = 0; pc < 2; pc++) {
-                    const int c = 32 * u + kPiece * pc, slot = (k * 2 + pc) * 4 + i;
-                    cp_async16_cg(area + slot * 32, sp + c);
-                    if constexpr (GF32) {
-                        cp_async16_cg(area + (8 + slot) * 32, static_cast<const float*>(g.gate) + go + c);
-                    }
-                }
+        for (int k = 0; k < NP; k++) {
+            x[k][i] = __ldcg(reinterpret_cast<const float4*>(op + size_t(row) * ldo + kPiece * k));
+            if constexpr (!GF32) {
+                gb[k][i] = *reinterpret_cast<const uint2*>(gp[i] + 2 * kPiece * k);
             }
         }
-    }
-    // bf16 gates travel in registers, one piece ahead of their use
-    uint2 gcur[4], gnxt[4];
-    if constexpr (!GF32) {
-        if (gp < units) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                gcur[i] = *reinterpret_cast<const uint2*>(gp4[i] + 32 * gp);
-            }
+        if constexpr (GF32) {
+            gf[0][i] = *reinterpret_cast<const float4*>(gp[i]);
         }
     }
     mbar_wait(tfull, tpar, abort);
-    if (threadIdx.x == kWorkWarp0 * 32) {
-        CCK_STAMP(3, false);
-    }
     tc_fence_after();
-    cp_async_wait_all();
     float* st = epi_stage();
-    float* op = static_cast<float*>(g.out) + col0 + cl;
 #pragma unroll
-    for (int k = 0; k < kU; k++) {
-        const int u = gp + 2 * k;
-        if (u < units) {
-#pragma unroll
-            for (int pc = 0; pc < 2; pc++) {
-                const int c = 32 * u + kPiece * pc;
-                if constexpr (!GF32) {
-                    // the next piece of this warp: the unit's second piece, or the next unit's first
-                    const int cn = pc == 0 ? c + kPiece : c + 64 - kPiece;
-                    if (pc == 0 || u + 2 < units) {
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            gnxt[i] = *reinterpret_cast<const uint2*>(gp4[i] + cn);
-                        }
-                    }
-                }
-                float v[32]; // one piece: the first 16 are used
-                {
-                    float h[16];
-                    tmem_ld16(taddr + c, h);
-#pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        v[i] = h[i];
-                    }
-                }
-                float4 t[4];
-                epi_turn<0>(st, v, t);
+    for (int k = 0; k < NP; k++) {
+        if constexpr (GF32) {
+            if (k + 1 < NP) {
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    const int row = r0 + 8 * i;
-                    if (row < g.m) {
-                        const int slot = (k * 2 + pc) * 4 + i;
-                        const float4 x = area[slot * 32];
-                        float4 gt;
-                        if constexpr (GF32) {
-                            gt = area[(8 + slot) * 32];
-                        } else {
-                            gt = unpack_bf4(gcur[i]);
-                        }
-                        const float4 cc = t[i];
-                        *reinterpret_cast<float4*>(op + size_t(row) * g.ldo + c) =
-                            make_float4(x.x + gt.x * cc.x * m[i], x.y + gt.y * cc.y * m[i], x.z + gt.z * cc.z * m[i], x.w + gt.w * cc.w * m[i]);
-                    }
-                }
-                if constexpr (!GF32) {
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        gcur[i] = gnxt[i];
-                    }
+                    gf[(k + 1) & 1][i] = *reinterpret_cast<const float4*>(gp[i] + 4 * kPiece * (k + 1));
                 }
             }
         }
+        float h[16];
+        tmem_ld16(taddr + kPiece * k, h);
+        float4 t[4];
+        epi_turn(st, h, t);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int row = r0 + 8 * i;
+            if (row < m) {
+                const float4 gt = GF32 ? gf[k & 1][i] : unpack_bf4(gb[GF32 ? 0 : k][i]);
+                const float4 y = x[k][i], cc = t[i];
+                *reinterpret_cast<float4*>(op + size_t(row) * ldo + kPiece * k) =
+                    make_float4(y.x + gt.x * cc.x * mask[i], y.y + gt.y * cc.y * mask[i], y.z + gt.z * cc.z * mask[i], y.w + gt.w * cc.w * mask[i]);
+            }
+        }
     }
-    // What this warp read and wrote here with ordinary accesses (its staging area inside the pipeline
-    // stages, the turn through its epilogue stage) is shared memory that later TMA loads overwrite:
-    // order the two proxies.
-    fence_async_smem();
 }
 
 // tile t -> (row tile, column tile) without an integer division
@@ -681,13 +606,47 @@ __device__ __forceinline__ void flow_signal(unsigned int* cnt, int c0, int c1) {
         }
     }
 }
-// One thread waits until the counters [c0, c1] have reached target (bounded, as every wait here);
-// what it then reads through TMA is what the signalling warps wrote. The counters are read eight at
-// a time with relaxed loads (one L2 round trip for the batch, not one each) and one acquire fence
-// follows the last read.
+// One thread's wait for one counter, in single looks, so that it can do something else in between.
+// Bounded as every wait here: when it gives up, or the launch has failed elsewhere, ready() says true and
+// the abort flag is set.
+struct FlowWait {
+    const unsigned int* cnt;
+    unsigned int target, looks;
+    volatile int* abort;
+    long long t0;
+    __device__ __forceinline__ FlowWait(const unsigned int* c, unsigned int tgt, volatile int* ab) : cnt(c), target(tgt), looks(0), abort(ab) {
+        t0 = clock64();
+        if (*abort) { // a wait inside this CTA gave up earlier: tell the grid, which would otherwise wait for this CTA's units
+            fail_launch(ST_PIPE_TIMEOUT, 0);
+        }
+    }
+    __device__ __forceinline__ bool ready() {
+        if (ld_relaxed(cnt) >= target) {
+            return true;
+        }
+        return *abort || (++looks % 32 == 0 && given_up()); // (the status word is another way to L2: not at every look)
+    }
+    // another CTA gave up (its units will not come), or this wait ran out: the launch drains
+    __device__ __noinline__ bool given_up() {
+        if (ld_relaxed(&kp().ctl->status) == ST_OK && clock64() - t0 <= wait_limit()) {
+            return false;
+        }
+        fail_launch(ST_PIPE_TIMEOUT, 0);
+        *abort = 1;
+        return true;
+    }
+    // what the signalling warps wrote is visible to what follows: this thread's reads and TMA loads
+    __device__ __forceinline__ void acquire() {
+        fence_acq_rel_gpu();
+        fence_async_global();
+    }
+};
+// One thread waits until the counters [c0, c1] have reached target; what it then reads through TMA is what
+// the signalling warps wrote. The counters are read eight at a time with relaxed loads (one L2 round
+// trip for the batch, not one each) and one acquire fence follows the last read.
 __device__ __forceinline__ bool flow_wait(const unsigned int* cnt, int c0, int c1, unsigned int target, volatile int* abort) {
     const long long t0 = clock64();
-    unsigned int* status = &kp().ctl->status;
+    unsigned int looks = 0;
     if (*abort) { // a wait inside this CTA gave up earlier: tell the grid, which would otherwise wait for this CTA's units
         fail_launch(ST_PIPE_TIMEOUT, 0);
     }
@@ -710,7 +669,7 @@ __device__ __forceinline__ bool flow_wait(const unsigned int* cnt, int c0, int c
                 return false;
             }
             // another CTA gave up (its units will not come), or this wait ran out: the launch drains
-            if (ld_relaxed(status) != ST_OK || clock64() - t0 > wait_limit()) {
+            if (++looks % 32 == 0 && (ld_relaxed(&kp().ctl->status) != ST_OK || clock64() - t0 > wait_limit())) {
                 fail_launch(ST_PIPE_TIMEOUT, 0);
                 *abort = 1;
                 return false;
@@ -745,7 +704,6 @@ template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, con
     SmemCtl* ctl = smem_ctl();
     GemmDesc g = gd; // a private copy: stores through its pointers cannot alias it
     g.bias = g.bias ? g.bias + size_t(b) * g.bias_step : nullptr;
-    g.gate = static_cast<const char*>(g.gate) + (long long)(b)*g.gate_step;
     CCK_TRACE_BEGIN_IF(4, threadIdx.x == kWorkWarp0 * 32);
     CCK_TRACE_EV(0x70, E);
     for (int t = tb; t < te; t += ts, tile++) {
@@ -765,10 +723,13 @@ template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, con
                 }
                 __syncwarp();
             }
-            if (g.gate_f32) {
-                resid_tile<true>(g, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);
+            const char* gate = static_cast<const char*>(gd.gate) + (long long)(b)*gd.gate_step;
+            if (gd.gate_f32) {
+                resid_tile<true, 2>(gd, gate, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);
+            } else if (gd.bn == 128) {
+                resid_tile<false, 4>(gd, gate, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);
             } else {
-                resid_tile<false>(g, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);
+                resid_tile<false, 2>(gd, gate, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);
             }
         } else {
             epilogue_tile<E>(g, mo, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);
@@ -778,9 +739,6 @@ template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, con
         CCK_TRACE_EV(0x72, t); // the accumulator is read
         if (lane_id() == 0) {
             mbar_arrive(&ctl->tempty[buf]);
-            if (warp_id() == kWorkWarp0) {
-                CCK_STAMP(4, false);
-            }
         }
         if constexpr (E == EPI_BF16 || E == EPI_GLU || E == EPI_RESID) {
             if (const int sigc = gd.fl >> GF_SIG_SHIFT & GF_CNT_MASK) {
@@ -805,118 +763,184 @@ template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, con
 }
 
 // ---- the TMA and MMA roles over the tiles of one GEMM
-// Tiles tb, tb + ts, ... < te (tile t: rows (t % mt)·128, columns (t / mt)·bn) of descriptor gd
-// with block b of its stack applied; one thread each.
-// k-blocks [kb0, kb1) of tile t into the ring, from position kbc on
-__device__ __forceinline__ void produce_kblocks(const Launch& L, const GemmDesc& gd, int b, int t, int kb0, int kb1, uint32_t& kbc) {
-    char* sm = smem_base();
-    SmemCtl* ctl = smem_ctl();
-    const CUtensorMap* ma = &L.tmap[gd.map_a];
-    const CUtensorMap* mb = &L.tmap[gd.map_b];
-    const int ktiles = gd.ktiles, kwrap = gd.b_kwrap;
-    const uint32_t bytes = kStageA + uint32_t(gd.bn) * kBK * 2;
+// Tiles tb, tb + ts, ... < te of descriptor gd with block b of its stack applied; one warp each (what a
+// single lane must do is predicated, see ptx.cuh). Both roles take the ring's slots in order from slot 0 at
+// the start of a GEMM; a slot's phase parity is a bit of pipe.ring, so the number of slots may change from
+// one GEMM to the next.
+
+// Where a tile's operands lie: row of A's map (pair GEMM: row tile (q, key tile) starts at row q·ldn + k0
+// of PC) and row of W's map
+struct TileRows {
+    int a, b;
+};
+__device__ __forceinline__ TileRows tile_rows(const GemmDesc& gd, int b, int t) {
     int row0, col0;
     tile_coords(gd, t, row0, col0);
-    // pair GEMM: row tile (q, key tile) starts at row q·ldn + k0 of PC
-    const int arow = ktiles ? row0 / (ktiles * kBM) * gd.ldn + row0 % (ktiles * kBM) : gd.a_row0 + row0;
-    const int brow = gd.b_row0 + b * gd.b_step + col0;
-    for (int kb = kb0; kb < kb1; kb++, kbc++) {
-        const uint32_t s = kbc % kStages, par = (kbc / kStages) & 1;
-        mbar_wait(&ctl->empty[s], par ^ 1, &ctl->abort);
-        CCK_STAMP(10, true);
-        mbar_expect_tx(&ctl->full[s], bytes);
-        char* st = sm + s * kStageBytes;
-        const int ka = kb * kBK, kw = kwrap ? ka % kwrap : ka;
-        tma_load_2d(st, ma, ka, arow, &ctl->full[s]);
-        tma_load_2d(st + kStageA, mb, kw, brow, &ctl->full[s]);
-        CCK_STAMP(0, true);
+    TileRows r;
+    r.a = uni(gd.ktiles ? row0 / (gd.ktiles * kBM) * gd.ldn + row0 % (gd.ktiles * kBM) : gd.a_row0 + row0);
+    r.b = uni(gd.b_row0 + b * gd.b_step + col0);
+    return r;
+}
+// A GEMM with another column tile lays the ring out anew: what the slots hold must have been consumed.
+__device__ __forceinline__ void ring_layout(SmemCtl* ctl, uint32_t ring, int bn) {
+    if (uni(ctl->ring_bn) != bn) {
+        for (int s = 0; s < kMaxSlots; s++) {
+            mbar_wait(&ctl->empty[s], (ring >> s & 1) ^ 1, &ctl->abort);
+        }
+        __syncwarp();
+        ctl->ring_bn = bn;
+        __syncwarp();
     }
 }
-// The TMA role over this CTA's tiles of one GEMM. After a grid barrier the thread that saw the
-// barrier open runs it right there for the phase's first GEMM (ahead = true), before the rest of
-// the CTA has found its way to the operation: the ramp of the phase (operation fetch, role
-// dispatch) then runs under the loads' latency. pipe.tile of the producer thread (otherwise unused)
-// says that the next call has nothing left to do.
+// The weights of the first k-blocks of this CTA's first tile, asked for ahead of everything the tile has to
+// wait for (a grid barrier): they depend on nothing that the launch computes. Returns how many.
+__device__ CCK_PHASE_FN int gemm_prefetch_w(const Launch& L, Pipe& pipe, const GemmDesc& gd, int b, int tb, int te) {
+    if (tb >= te) {
+        return 0;
+    }
+    SmemCtl* ctl = smem_ctl();
+    const uint32_t el = elect_one(), ring = uni(pipe.ring);
+    const int bn = uni(gd.bn);
+    ring_layout(ctl, ring, bn);
+    const CUtensorMap* mb = &L.tmap[uni(gd.map_b)];
+    const uint32_t bytes = ring_slot_bytes(bn), w0 = uni(smem_u32(smem_base())) + kStageA, full = uni(smem_u32(&ctl->full[0]));
+    const int n = uni(min(gd.k / kBK, ring_slots(bn))), kwrap = uni(gd.b_kwrap ? gd.b_kwrap : 1 << 30), row = tile_rows(gd, b, tb).b;
+    for (int i = 0; i < n; i++) {
+        mbar_wait(&ctl->empty[i], (ring >> i & 1) ^ 1, &ctl->abort);
+        mbar_expect_tx_el(el, full + 8 * i, bytes);
+        const int k = i * kBK;
+        tma_load_2d_el(el, w0 + i * bytes, mb, k >= kwrap ? k - kwrap : k, row, full + 8 * i);
+    }
+    return n;
+}
+// The TMA role. `ahead`: run by the warp that saw a grid barrier open, right there, before the rest of the
+// CTA has found its way to the operation; pipe.tile of this warp (otherwise unused) then says that the
+// next call has nothing left to do. `have`: k-blocks of the first tile whose weights are already on their
+// way (gemm_prefetch_w). While a tile waits for the rows of A that it reads, its weights are fetched into
+// the slots that are free: when the rows are complete, only A's way is left.
 __device__ CCK_PHASE_FN void gemm_produce(const Launch& L, Pipe& pipe, const GemmDesc& gd, int b, int tb, int te, int ts, bool ahead,
-                                          unsigned int epoch) {
+                                          int have, unsigned int epoch) {
     if (pipe.tile) { // produced ahead
         pipe.tile = 0;
         return;
     }
-    const int kblocks = gd.k / kBK;
-    uint32_t kbc = pipe.kb;
-    CCK_TRACE_BEGIN(0);
-    CCK_TRACE_EV(0x50, gd.epi);
-    for (int t = tb; t < te; t += ts) {
-        if (const int depc = gd.fl >> GF_DEP_SHIFT & GF_CNT_MASK) { // until the rows of A that this tile reads are complete
-            int row0, col0;
-            tile_coords(gd, t, row0, col0);
-            const int rb = row0 / kBM;
-#if CCK_STAGE_REC
-            const long long fw0_ = clock64();
-#endif
-            flow_wait(flow_cnt(kp(), depc - 1), rb, rb, (epoch + 1) * flow_target(gd, depc - 1, rb, gd_table()[GD_TOK_W1].nt),
-                      &smem_ctl()->abort);
-#if CCK_STAGE_REC
-            atomicAdd(&g_stage_rec[28][3 + (depc - 1)], (unsigned long long)(clock64() - fw0_)); // row 28: 4 waits for TO, 5 waits for TC
-            atomicAdd(&g_stage_rec[28][6 + (depc - 1)], 1ull);                                  // 7, 8: how many
-#endif
+    if (tb < te) {
+        SmemCtl* ctl = smem_ctl();
+        const uint32_t el = elect_one();
+        const CUtensorMap* ma = &L.tmap[uni(gd.map_a)];
+        const CUtensorMap* mb = &L.tmap[uni(gd.map_b)];
+        const int bn = uni(gd.bn), kblocks = uni(gd.k / kBK), slots = ring_slots(bn), depc = uni(gd.fl >> GF_DEP_SHIFT & GF_CNT_MASK);
+        const int kwrap = uni(gd.b_kwrap ? gd.b_kwrap : 1 << 30);
+        const uint32_t bytes = ring_slot_bytes(bn), sm = uni(smem_u32(smem_base())), full = uni(smem_u32(&ctl->full[0])),
+                       empty = uni(smem_u32(&ctl->empty[0]));
+        uint32_t ring = uni(pipe.ring);
+        int s = 0;
+        have = uni(have), tb = uni(tb), te = uni(te), ts = uni(ts);
+        if (have == 0) {
+            ring_layout(ctl, ring, bn);
         }
-        CCK_TRACE_EV(0x52, t); // what the tile reads is complete
-        produce_kblocks(L, gd, b, t, 0, kblocks, kbc);
-        CCK_TRACE_EV(0x54, t); // every k-block is asked for
+        CCK_TRACE_BEGIN_IF(0, el);
+        CCK_TRACE_EV(0x50, gd.epi);
+        for (int t = tb; t < te; t += ts, have = 0) {
+            const TileRows r = tile_rows(gd, b, t);
+            if (depc) { // until the rows of A that this tile reads are complete
+                int row0, col0;
+                tile_coords(gd, t, row0, col0);
+                const int rb = row0 / kBM;
+                FlowWait w(flow_cnt(kp(), depc - 1) + rb, (epoch + 1) * flow_target(gd, depc - 1, rb, gd_table()[GD_TOK_W1].nt), &ctl->abort);
+                const int most = min(kblocks, slots);
+                int f = s + have < slots ? s + have : s + have - slots; // the slot of k-block `have`
+                while (!uni(int(w.ready()))) {
+                    if (have < most && uni(int(mbar_test_a(empty + 8 * f, (ring >> f & 1) ^ 1)))) {
+                        mbar_expect_tx_el(el, full + 8 * f, bytes);
+                        const int k = have * kBK;
+                        tma_load_2d_el(el, sm + f * bytes + kStageA, mb, k >= kwrap ? k - kwrap : k, r.b, full + 8 * f);
+                        have++;
+                        f = f + 1 < slots ? f + 1 : 0;
+                    }
+                }
+                w.acquire();
+            }
+            CCK_TRACE_EV(0x52, t); // what the tile reads is complete
+            for (int kb = 0; kb < kblocks; kb++) {
+                const uint32_t st = sm + s * bytes, bar = full + 8 * s;
+                const int k = kb * kBK;
+                if (kb >= have) {
+                    mbar_wait(&ctl->empty[s], (ring >> s & 1) ^ 1, &ctl->abort);
+                    mbar_expect_tx_el(el, bar, bytes);
+                    tma_load_2d_el(el, st + kStageA, mb, k >= kwrap ? k - kwrap : k, r.b, bar);
+                }
+                tma_load_2d_el(el, st, ma, k, r.a, bar);
+                ring ^= 1u << s;
+                s = s + 1 < slots ? s + 1 : 0;
+            }
+            CCK_TRACE_EV(0x54, t); // every k-block is asked for
+        }
+        CCK_TRACE_END();
+        pipe.ring = ring;
     }
-    CCK_TRACE_END();
-    pipe.kb = kbc;
     pipe.tile = ahead;
 }
 __device__ CCK_PHASE_FN void gemm_issue(Pipe& pipe, const GemmDesc& gd, int tb, int te, int ts) {
-    char* sm = smem_base();
+    if (tb >= te) {
+        return;
+    }
     SmemCtl* ctl = smem_ctl();
-    const int bn = gd.bn, kblocks = gd.k / kBK;
-    const uint32_t idesc = umma_idesc_bf16(kBM, bn);
-    uint32_t kbc = pipe.kb, tile = pipe.tile;
-    CCK_TRACE_BEGIN(2);
+    const uint32_t el = elect_one();
+    const int bn = uni(gd.bn), kblocks = uni(gd.k / kBK), slots = ring_slots(bn);
+    const uint32_t idesc = umma_idesc_bf16(kBM, bn), tmem = uni(ctl->tmem_base), full = uni(smem_u32(&ctl->full[0])),
+                   empty = uni(smem_u32(&ctl->empty[0])), tfull = uni(smem_u32(&ctl->tfull[0]));
+    uint32_t ring = uni(pipe.ring), tile = uni(pipe.tile);
+    tb = uni(tb), te = uni(te), ts = uni(ts);
+    // the operands' descriptors differ from slot to slot by the slot's size (in units of 16 bytes)
+    const uint64_t d0 = umma_desc_sw128(uni(smem_u32(smem_base()))), step = uint64_t(ring_slot_bytes(bn) >> 4);
+    int s = 0;
+    uint64_t da = d0;
+    CCK_TRACE_BEGIN_IF(2, el);
     CCK_TRACE_EV(0x60, gd.epi);
     for (int t = tb; t < te; t += ts, tile++) {
         const uint32_t buf = tile & 1, tpar = (tile >> 1) & 1;
         mbar_wait(&ctl->tempty[buf], tpar ^ 1, &ctl->abort);
-        tc_fence_after();
         CCK_TRACE_EV(0x62, t); // the accumulator buffer is free
-        const uint32_t acc = ctl->tmem_base + buf * kMaxBN;
-        for (int kb = 0; kb < kblocks; kb++, kbc++) {
-            const uint32_t s = kbc % kStages, par = (kbc / kStages) & 1;
-            mbar_wait(&ctl->full[s], par, &ctl->abort);
-            CCK_STAMP(1, true);
+        const uint32_t acc = tmem + buf * kMaxBN;
+        bool landed = false;
+        for (int kb = 0; kb < kblocks; kb++) {
+            if (!landed) {
+                mbar_wait(&ctl->full[s], ring >> s & 1, &ctl->abort);
+            }
             tc_fence_after();
             if (kb == 0) {
                 CCK_TRACE_EV(0x64, t); // the first operands have landed
             }
-            const uint32_t sa = smem_u32(sm + s * kStageBytes), sb = sa + kStageA;
-            const uint64_t da = umma_desc_sw128(sa), db = umma_desc_sw128(sb);
-#pragma unroll
-            for (int kk = 0; kk < kBK / 16; kk++) {
-                // 16 bf16 = 32 bytes along k inside the 128-byte swizzle row: +2 in the address field
-                umma_bf16(acc, da + 2 * kk, db + 2 * kk, idesc, (kb | kk) != 0);
+            const uint64_t d = da;
+            const int cs = s;
+            ring ^= 1u << s;
+            if (++s < slots) {
+                da += step;
+            } else {
+                s = 0, da = d0;
             }
-            umma_commit(&ctl->empty[s]);
+            // (the next k-block's barrier is looked at under this one's MMAs: a wait that passes costs 88 cycles)
+            landed = kb + 1 < kblocks && mbar_test_a(full + 8 * s, ring >> s & 1);
+            umma_bf16_kblock_el(el, acc, d, d + (kStageA >> 4), idesc, kb);
+            umma_commit_el(el, empty + 8 * cs);
         }
-        umma_commit(&ctl->tfull[buf]);
-        CCK_STAMP(2, false);
+        umma_commit_el(el, tfull + 8 * buf);
         CCK_TRACE_EV(0x66, t); // the tile's last MMA is issued
     }
     CCK_TRACE_END();
-    pipe.kb = kbc, pipe.tile = tile;
+    pipe.ring = ring, pipe.tile = tile;
 }
 
 // once per launch, by the whole CTA: barriers and the TMEM allocation
 __device__ inline void gemm_init() {
     SmemCtl* ctl = smem_ctl();
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kStages; i++) {
+        for (int i = 0; i < kMaxSlots; i++) {
             mbar_init(&ctl->full[i], 1);
             mbar_init(&ctl->empty[i], 1);
         }
+        ctl->ring_bn = 0;
         for (int i = 0; i < 2; i++) {
             mbar_init(&ctl->tfull[i], 1);
             mbar_init(&ctl->tempty[i], kWorkWarps);

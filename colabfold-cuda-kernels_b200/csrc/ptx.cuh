@@ -68,7 +68,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// The same with a suspend-time hint (ns): the thread sleeps in hardware until the phase completes or
+// has the phase with this parity completed? Never blocks.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// mbar_try_wait with a suspend-time hint (ns): the thread sleeps in hardware until the phase completes or
 // the time is over, instead of coming back to spin. A waiting thread then leaves its SM
 // sub-partition's issue slots to the warps that share it.
 __device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parity, uint32_t ns) {
@@ -82,6 +94,92 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parit
         : "memory");
     return ok != 0;
 }
+// ---- Instructions for a role that a whole warp runs. Every lane passes the same loop; what must happen once is
+// predicated on one elected lane (`el`) inside the statement instead of sitting in a one-lane branch. The
+// operands of tcgen05 and TMA instructions live in the uniform register file, which the compiler feeds
+// directly only where control flow is warp-uniform: in a branch of one thread a k-block of four
+// tcgen05.mma, a wait and a commit took 541 cycles to issue whatever its width, in this form 260 at 128 columns
+// (the rate of the tensor pipe) and 500 at 256; a wait and two TMA loads 309 against 253.
+// uni(): the value of lane 0, which the compiler then knows to be the same in all lanes
+__device__ __forceinline__ int uni(int v) {
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+__device__ __forceinline__ uint32_t uni(uint32_t v) {
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+__device__ __forceinline__ bool mbar_test_a(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void mbar_expect_tx_el(uint32_t el, uint32_t bar, uint32_t bytes) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t"
+        "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar),
+        "r"(bytes), "r"(el)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_el(uint32_t el, uint32_t smem_dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+        "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
+        :
+        : "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(el)
+        : "memory");
+}
+// one k-block of 64: four MMAs of K = 16 (32 bytes along k inside the 128-byte swizzle row: +2 in the
+// descriptors' address field); the first one accumulates if `acc` is not zero
+__device__ __forceinline__ void umma_bf16_kblock_el(uint32_t el, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, e;\n\t.reg .b64 a, b;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\tsetp.eq.b32 q, 0, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "add.u64 a, %1, 2;\n\tadd.u64 b, %2, 2;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, q;\n\t"
+        "add.u64 a, %1, 4;\n\tadd.u64 b, %2, 4;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, q;\n\t"
+        "add.u64 a, %1, 6;\n\tadd.u64 b, %2, 6;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, q;\n\t}"
+        :
+        : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(acc), "r"(el)
+        : "memory");
+}
+// three MMAs of K = 16: a head of 48
+__device__ __forceinline__ void umma_bf16_k48_el(uint32_t el, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, e;\n\t.reg .b64 a, b;\n\t"
+        "setp.ne.b32 e, %4, 0;\n\tsetp.eq.b32 q, 0, 0;\n\tsetp.ne.b32 p, 0, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "add.u64 a, %1, 2;\n\tadd.u64 b, %2, 2;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, q;\n\t"
+        "add.u64 a, %1, 4;\n\tadd.u64 b, %2, 4;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, q;\n\t}"
+        :
+        : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(el)
+        : "memory");
+}
+// four MMAs of K = 16 with A in tensor memory (16 bf16 of k are 8 columns)
+__device__ __forceinline__ void umma_bf16_ts_k64_el(uint32_t el, uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, e;\n\t.reg .b64 b;\n\t.reg .b32 a;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\tsetp.eq.b32 q, 0, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "add.u32 a, %1, 8;\n\tadd.u64 b, %2, 2;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, q;\n\t"
+        "add.u32 a, %1, 16;\n\tadd.u64 b, %2, 4;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, q;\n\t"
+        "add.u32 a, %1, 24;\n\tadd.u64 b, %2, 6;\n\t@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, q;\n\t}"
+        :
+        : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc), "r"(el)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit_el(uint32_t el, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+        "r"(el)
+        : "memory");
+}
+
 // Waits for the phase with the given parity. Returns false if it gave up; *abort (shared memory)
 // is then set so that every later wait of the CTA returns at once.
 #ifndef CCK_WAIT_HINT_NS

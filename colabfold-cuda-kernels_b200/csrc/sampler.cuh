@@ -73,116 +73,91 @@ __device__ __noinline__ bool grid_barrier(const Launch& L, int end_kind) {
     const bool stop = (end_kind & 3) == END_PHASE && p.dbg_stop > 0 && r.phase + 1 >= p.dbg_stop;
     fence_async_global(); // this thread's global writes, for TMA reads of other CTAs in later phases
     __syncthreads();
-    // Thread 0 waits for the grid; its warp then releases the CTA through a named barrier (the warp
-    // arrives as a whole and does not wait: a warp-level barrier instruction counts 32 arrivals
-    // however many of its lanes run it, so the warp must not be split between arrive and sync),
-    // after which thread 0 runs the next GEMM's TMA role while the others find their way there.
-    int gemm_id = -1, gemm_b = 0;
-    bool open = true;
-    if (threadIdx.x == 0) {
+    // Warp 0 waits for the grid (its first thread does); it then releases the CTA through a named barrier
+    // (the warp arrives as a whole and does not wait: a warp-level barrier instruction counts 32
+    // arrivals however many of its lanes run it, so the warp must not be split between arrive and sync),
+    // after which it runs the next GEMM's TMA role while the others find their way there.
+    if (warp_id() == 0) {
         SmemCtl* sc = smem_ctl();
-#if CCK_STAGE_REC
-        sc->stamp[5] = stage_now();
-#endif
-        if (sc->abort) { // a wait of this CTA gave up in the phase that ends here
-            fail_launch(ST_PIPE_TIMEOUT, r.syncs);
-        }
-        const unsigned int target = (r.syncs + 1) * gridDim.x + (unsigned int)p.barrier_extra;
-        CCK_TRACE_ONE(6, 0x84, kind);
+        CCK_TRACE_ONE_IF(6, 0x84, kind, threadIdx.x == 0);
 #if CCK_TRACE
         const long long tw0_ = clock64();
 #endif
-        red_release_add(&p.ctl->barrier, 1u);
+        if (threadIdx.x == 0) {
+            if (sc->abort) { // a wait of this CTA gave up in the phase that ends here
+                fail_launch(ST_PIPE_TIMEOUT, r.syncs);
+            }
+            red_release_add(&p.ctl->barrier, 1u);
+        }
+        __syncwarp();
         // while the arrival travels: is the next operation a GEMM? (the program's control
-        // operations followed without their side effects)
+        // operations followed without their side effects; a GEMM that waits for other units never follows
+        // a barrier.) Its first weights can be on their way: the other warps have left the phase, nobody
+        // touches the ring's shared memory.
+        int gemm_id = -1, gemm_b = 0, have = 0;
         if (!stop) {
             const Program& prog = *reinterpret_cast<const Program*>(smem_base() + kProgOff);
             Flow f{r.pc, r.blk, r.step, r.ret, r.second};
             const Op op = flow_next(prog, p, f);
-            if (op.fn == FN_GEMM) { // (a GEMM that waits for other units never follows a barrier: nothing to wait for here)
+            if (op.fn == FN_GEMM) {
                 gemm_id = op.a0, gemm_b = op.b == kLoopB ? f.blk : op.b;
+                const GemmDesc& g = gd_table()[gemm_id];
+                have = gemm_prefetch_w(L, r.pipe, g, gemm_b, blockIdx.x, g.tiles);
             }
         }
-        const long long t0 = clock64();
-        for (;;) {
-            const unsigned int v = ld_acquire(&p.ctl->barrier);
-            if (v & kBarrierPoison) { // some CTA has recorded a failure: nobody waits for anybody any more
-                sc->abort = 1, sc->quit = 1;
-                open = false;
-                break;
-            }
-            if (v >= target) {
-                break;
-            }
-            if (clock64() - t0 > wait_limit()) {
-                fail_launch(ST_BARRIER_TIMEOUT, r.syncs);
-                sc->abort = 1, sc->quit = 1;
-                open = false;
-                break;
-            }
-            __nanosleep(20);
-        }
-        CCK_TRACE_ONE(6, 0x86, kind);
-#if CCK_TRACE
-        if (r.syncs < kBarWaitSlots) { // every CTA: how long it waited at this barrier (the last to arrive waits least)
-            g_barwait[r.syncs][blockIdx.x] = (unsigned int)(clock64() - tw0_) | (unsigned int)kind << 24;
-        }
-#endif
-#if CCK_STAGE_REC
-        {
-            const unsigned long long t = stage_now();
-            if (sc->phase_t0) {
-                for (int i = 0; i < 14; i++) {
-                    if (i != 6 && i != 7 && sc->stamp[i] >= sc->phase_t0) {
-                        atomicAdd(&g_stage_rec[kind][i], sc->stamp[i] - sc->phase_t0);
-                    }
+        bool open = true;
+        if (threadIdx.x == 0) {
+            const unsigned int target = (r.syncs + 1) * gridDim.x + (unsigned int)p.barrier_extra;
+            const long long t0 = clock64();
+            for (;;) {
+                const unsigned int v = ld_acquire(&p.ctl->barrier);
+                if (v & kBarrierPoison) { // some CTA has recorded a failure: nobody waits for anybody any more
+                    sc->abort = 1, sc->quit = 1;
+                    break;
                 }
-                atomicAdd(&g_stage_rec[kind][6], t - sc->phase_t0);
-                atomicAdd(&g_stage_rec[kind][7], 1ull);
+                if (v >= target) {
+                    break;
+                }
+                if (clock64() - t0 > wait_limit()) {
+                    fail_launch(ST_BARRIER_TIMEOUT, r.syncs);
+                    sc->abort = 1, sc->quit = 1;
+                    break;
+                }
+                __nanosleep(20);
             }
-            for (int i = 0; i < 16; i++) {
-                sc->stamp[i] = 0;
+            CCK_TRACE_ONE(6, 0x86, kind);
+#if CCK_TRACE
+            if (r.syncs < kBarWaitSlots) { // every CTA: how long it waited at this barrier (the last to arrive waits least)
+                g_barwait[r.syncs][blockIdx.x] = (unsigned int)(clock64() - tw0_) | (unsigned int)kind << 24;
             }
-            sc->phase_t0 = t;
-        }
 #endif
-        if (p.timing && blockIdx.x == 0) {
-            const unsigned long long t = now_ns();
-            if (sc->t0) {
-                // accumulated in shared memory, written out when the kernel ends: a global
-                // read-modify-write here would delay CTA 0, and with it the grid, in every phase
-                unsigned long long* acc = reinterpret_cast<unsigned long long*>(smem_base() + kCtlOff + kTimingOff);
-                acc[2 * kind] += t - sc->t0;
-                acc[2 * kind + 1] += 1;
+            if (p.timing && blockIdx.x == 0) {
+                const unsigned long long t = now_ns();
+                if (sc->t0) {
+                    // accumulated in shared memory, written out when the kernel ends: a global
+                    // read-modify-write here would delay CTA 0, and with it the grid, in every phase
+                    unsigned long long* acc = reinterpret_cast<unsigned long long*>(smem_base() + kCtlOff + kTimingOff);
+                    acc[2 * kind] += t - sc->t0;
+                    acc[2 * kind + 1] += 1;
+                }
+                sc->t0 = t;
             }
-            sc->t0 = t;
+            open = !sc->abort;
         }
-        open = open && !sc->abort;
-    }
-    if (warp_id() == 0) {
         __syncwarp();
         asm volatile("barrier.cta.arrive 6, %0;" ::"n"(kThreads) : "memory");
-        if (threadIdx.x == 0 && open && gemm_id >= 0) {
-            fence_async_global(); // the other CTAs' writes of the phase just ended, for this thread's TMA reads
+        open = __shfl_sync(0xffffffffu, int(open), 0);
+        if (open && gemm_id >= 0) {
+            fence_async_global(); // the other CTAs' writes of the phase just ended, for this warp's TMA reads
             const GemmDesc& g = gd_table()[gemm_id];
-            gemm_produce(L, r.pipe, g, gemm_b, blockIdx.x, g.tiles, gridDim.x, true, 0); // the rotation starts at 0 after a barrier
+            gemm_produce(L, r.pipe, g, gemm_b, blockIdx.x, g.tiles, gridDim.x, true, have, 0); // the rotation starts at 0 after a barrier
         }
         __syncwarp();
     } else {
         asm volatile("barrier.cta.sync 6, %0;" ::"n"(kThreads) : "memory");
     }
     r.syncs++;
-#if CCK_STAGE_REC
-    if (threadIdx.x == 0) {
-        smem_ctl()->stamp[11] = stage_now();
-    }
-#endif
     fence_async_global();
-#if CCK_STAGE_REC
-    if (threadIdx.x == 0) {
-        smem_ctl()->stamp[8] = stage_now();
-    }
-#endif
     r.d.start = 0;
     r.phase += (end_kind & 3) == END_PHASE;
     return stop || smem_ctl()->quit; // (written before the named barrier that released this thread)
@@ -382,17 +357,10 @@ __device__ __forceinline__ void run_gemm(const Launch& L, Run& r, Deal& d, int i
     const GemmDesc& g = gd_table()[id];
     const int tiles = g.tiles, tb = d.first(), ts = gridDim.x;
     const int warp = warp_id();
-    if (threadIdx.x == 0) {
-        CCK_STAMP(9, true);
-    }
     if (warp == 0) {
-        if (lane_id() == 0) {
-            gemm_produce(L, r.pipe, g, b, tb, tiles, ts, false, epoch);
-        }
+        gemm_produce(L, r.pipe, g, b, tb, tiles, ts, false, 0, epoch);
     } else if (warp == 1) {
-        if (lane_id() == 0) {
-            gemm_issue(r.pipe, g, tb, tiles, ts);
-        }
+        gemm_issue(r.pipe, g, tb, tiles, ts);
     } else if (warp < kAuxWarp0) {
         const uint32_t tile = r.pipe.tile;
         const CUtensorMap* mo = g.map_o >= 0 ? &L.tmap[g.map_o] : nullptr;
@@ -436,9 +404,6 @@ __device__ __forceinline__ void run_op(const Launch& L, Run& r, const Op op) {
     const KP& p = kp();
     const int b = op.b == kLoopB ? r.blk : op.b, step = r.step;
     Deal& d = r.d;
-    if (threadIdx.x == 0) {
-        CCK_STAMP(12, true);
-    }
     switch (op.fn) {
     case FN_GEMM:
         run_gemm(L, r, d, op.a0, b, flow_epoch(p, r));
@@ -530,8 +495,8 @@ __device__ __forceinline__ void run_op(const Launch& L, Run& r, const Op op) {
     default: // FN_CTA_SYNC
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        CCK_STAMP(13, false);
+    if (op.fn != FN_GEMM && op.fn != FN_CTA_SYNC) {
+        fence_async_smem(); // what this thread did in the scratch area, before TMA loads fill the ring there
     }
 }
 
@@ -572,14 +537,6 @@ extern "C" __global__ void __launch_bounds__(cck::kThreads, 1) cck_sampler_kerne
     gd_build();
     gemm_init();
     attn_tc_init();
-#if CCK_STAGE_REC
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < 16; i++) {
-            smem_ctl()->stamp[i] = 0;
-        }
-        smem_ctl()->phase_t0 = 0;
-    }
-#endif
     __syncthreads();
     // The schedule state of each thread lives in shared memory, not on its stack: the acquire of
     // every grid barrier empties L1, and state kept in local memory would then cost an L2 round
