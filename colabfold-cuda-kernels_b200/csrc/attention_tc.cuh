@@ -186,6 +186,7 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
         const int n = uni(tc_track_items(first, items, t)), nchunks = uni(chunks);
         if (n > 0) {
             const uint32_t el = elect_one();
+            const uint64_t policy = l2_policy(S == 1); // the pair logits: one sample reads them once, several meet in L2
             TcTrackBars& B = bars->t[t];
             const uint32_t base = uni(smem_u32(sm + t * kTcTrackBytes)), bar0 = uni(smem_u32(&B));
             auto bar = [&](uint64_t& x) { return bar0 + uint32_t(reinterpret_cast<char*>(&x) - reinterpret_cast<char*>(&B)); };
@@ -232,7 +233,7 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                 const uint32_t st = g % kTcBiasStages, par = (g / kTcBiasStages) & 1, bb = bar(B.b_full[0]) + 8 * st;
                 mbar_wait(&B.b_empty[st], par ^ 1, &ctl->abort);
                 mbar_expect_tx_el(el, bb, kTcBiasBytes);
-                tma_load_2d_el(el, base + kTcBiasOff + st * kTcBiasBytes, mpl, c * kTcKeys, brow, bb);
+                tma_load_2d_hint_el(el, base + kTcBiasOff + st * kTcBiasBytes, mpl, c * kTcKeys, brow, bb, policy);
             };
             if (t == 1 && p.attn_skew > 0) { // a test's skew between the pipelines: results must not depend on it
                 const long long t0 = clock64();

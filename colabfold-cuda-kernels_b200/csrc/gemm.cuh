@@ -792,6 +792,15 @@ __device__ __forceinline__ void ring_layout(SmemCtl* ctl, uint32_t ring, int bn)
         __syncwarp();
     }
 }
+// A sampling step of the smallest fold reads 400 MB of weights, which push everything else out of the 126 MB of
+// L2: inputs, intermediate rows and the kernel's own code (half a megabyte, most of it run once per step)
+// then come from HBM. Where few row tiles share a weight tile, within microseconds, the weights are marked as
+// the first to leave: 1.20 -> 1.11 ms per step at 32 x 1, 1.37 -> 1.34 at 61 x 5. With many row tiles that
+// loses the weights between two of them (5.37 -> 5.51 ms at 1024 x 5).
+constexpr int kOnceRowTiles = 24;
+__device__ __forceinline__ uint64_t weights_policy(const GemmDesc& gd) {
+    return l2_policy(uni(gd.mt) <= kOnceRowTiles);
+}
 // The weights of the first k-blocks of this CTA's first tile, asked for ahead of everything the tile has to
 // wait for (a grid barrier): they depend on nothing that the launch computes. Returns how many.
 __device__ CCK_PHASE_FN int gemm_prefetch_w(const Launch& L, Pipe& pipe, const GemmDesc& gd, int b, int tb, int te) {
@@ -800,6 +809,7 @@ __device__ CCK_PHASE_FN int gemm_prefetch_w(const Launch& L, Pipe& pipe, const G
     }
     SmemCtl* ctl = smem_ctl();
     const uint32_t el = elect_one(), ring = uni(pipe.ring);
+    const uint64_t policy = weights_policy(gd);
     const int bn = uni(gd.bn);
     ring_layout(ctl, ring, bn);
     const CUtensorMap* mb = &L.tmap[uni(gd.map_b)];
@@ -809,7 +819,7 @@ __device__ CCK_PHASE_FN int gemm_prefetch_w(const Launch& L, Pipe& pipe, const G
         mbar_wait(&ctl->empty[i], (ring >> i & 1) ^ 1, &ctl->abort);
         mbar_expect_tx_el(el, full + 8 * i, bytes);
         const int k = i * kBK;
-        tma_load_2d_el(el, w0 + i * bytes, mb, k >= kwrap ? k - kwrap : k, row, full + 8 * i);
+        tma_load_2d_hint_el(el, w0 + i * bytes, mb, k >= kwrap ? k - kwrap : k, row, full + 8 * i, policy);
     }
     return n;
 }
@@ -827,6 +837,7 @@ __device__ CCK_PHASE_FN void gemm_produce(const Launch& L, Pipe& pipe, const Gem
     if (tb < te) {
         SmemCtl* ctl = smem_ctl();
         const uint32_t el = elect_one();
+        const uint64_t policy = weights_policy(gd);
         const CUtensorMap* ma = &L.tmap[uni(gd.map_a)];
         const CUtensorMap* mb = &L.tmap[uni(gd.map_b)];
         const int bn = uni(gd.bn), kblocks = uni(gd.k / kBK), slots = ring_slots(bn), depc = uni(gd.fl >> GF_DEP_SHIFT & GF_CNT_MASK);
@@ -854,7 +865,7 @@ __device__ CCK_PHASE_FN void gemm_produce(const Launch& L, Pipe& pipe, const Gem
                     if (have < most && uni(int(mbar_test_a(empty + 8 * f, (ring >> f & 1) ^ 1)))) {
                         mbar_expect_tx_el(el, full + 8 * f, bytes);
                         const int k = have * kBK;
-                        tma_load_2d_el(el, sm + f * bytes + kStageA, mb, k >= kwrap ? k - kwrap : k, r.b, full + 8 * f);
+                        tma_load_2d_hint_el(el, sm + f * bytes + kStageA, mb, k >= kwrap ? k - kwrap : k, r.b, full + 8 * f, policy);
                         have++;
                         f = f + 1 < slots ? f + 1 : 0;
                     }
@@ -868,7 +879,7 @@ __device__ CCK_PHASE_FN void gemm_produce(const Launch& L, Pipe& pipe, const Gem
                 if (kb >= have) {
                     mbar_wait(&ctl->empty[s], (ring >> s & 1) ^ 1, &ctl->abort);
                     mbar_expect_tx_el(el, bar, bytes);
-                    tma_load_2d_el(el, st + kStageA, mb, k >= kwrap ? k - kwrap : k, r.b, bar);
+                    tma_load_2d_hint_el(el, st + kStageA, mb, k >= kwrap ? k - kwrap : k, r.b, bar, policy);
                 }
                 tma_load_2d_el(el, st, ma, k, r.a, bar);
                 ring ^= 1u << s;

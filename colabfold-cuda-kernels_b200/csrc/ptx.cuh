@@ -133,6 +133,21 @@ __device__ __forceinline__ void tma_load_2d_el(uint32_t el, uint32_t smem_dst, c
         : "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(el)
         : "memory");
 }
+// the same with an L2 policy: what is read once and not soon again is the first to leave
+__device__ __forceinline__ uint64_t l2_policy(bool once) {
+    uint64_t first, normal;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(normal));
+    return once ? first : normal;
+}
+__device__ __forceinline__ void tma_load_2d_hint_el(uint32_t el, uint32_t smem_dst, const CUtensorMap* map, int x, int y, uint32_t bar, uint64_t policy) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+        "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %6;\n\t}"
+        :
+        : "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(el), "l"(policy)
+        : "memory");
+}
 // one k-block of 64: four MMAs of K = 16 (32 bytes along k inside the 128-byte swizzle row: +2 in the
 // descriptors' address field); the first one accumulates if `acc` is not zero
 __device__ __forceinline__ void umma_bf16_kblock_el(uint32_t el, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t acc) {
