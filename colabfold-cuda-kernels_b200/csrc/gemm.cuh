@@ -593,7 +593,7 @@ constexpr int kMaxGd = kGdBytes / int(sizeof(GemmDesc));
 
 // ---- completion counters between operations of one phase (FlowCnt)
 __device__ __forceinline__ unsigned int* flow_cnt(const KP& p, int which) {
-    return p.flow_cnt + which * p.flow_n;
+    return p.flow_cnt + which * p.flow_n * kFlowPitch;
 }
 // The calling warp's part of a unit is stored: its lanes' writes (and lane 0's TMA stores, which the
 // caller has waited for) are published with one release add per counter in [c0, c1].
@@ -602,7 +602,7 @@ __device__ __forceinline__ void flow_signal(unsigned int* cnt, int c0, int c1) {
     __syncwarp();
     if (lane_id() == 0) {
         for (int c = c0; c <= c1; c++) {
-            red_release_add(cnt + c, 1u);
+            red_release_add(cnt + c * kFlowPitch, 1u);
         }
     }
 }
@@ -655,7 +655,7 @@ __device__ __forceinline__ bool flow_wait(const unsigned int* cnt, int c0, int c
             unsigned int v[8];
 #pragma unroll
             for (int i = 0; i < 8; i++) {
-                v[i] = b0 + i <= c1 ? ld_relaxed(cnt + b0 + i) : target;
+                v[i] = b0 + i <= c1 ? ld_relaxed(cnt + (b0 + i) * kFlowPitch) : target;
             }
             bool ok = true;
 #pragma unroll
@@ -858,7 +858,7 @@ __device__ CCK_PHASE_FN void gemm_produce(const Launch& L, Pipe& pipe, const Gem
                 int row0, col0;
                 tile_coords(gd, t, row0, col0);
                 const int rb = row0 / kBM;
-                FlowWait w(flow_cnt(kp(), depc - 1) + rb, (epoch + 1) * flow_target(gd, depc - 1, rb, gd_table()[GD_TOK_W1].nt), &ctl->abort);
+                FlowWait w(flow_cnt(kp(), depc - 1) + rb * kFlowPitch, (epoch + 1) * flow_target(gd, depc - 1, rb, gd_table()[GD_TOK_W1].nt), &ctl->abort);
                 const int most = min(kblocks, slots);
                 int f = s + have < slots ? s + have : s + have - slots; // the slot of k-block `have`
                 while (!uni(int(w.ready()))) {

@@ -171,7 +171,7 @@ static int make_template(Template& t, int S, int Nb, int NSb, int nsteps, uint32
     want[B_AGT] = ra * kTokC * f;
     want[B_VT] = size_t(S) * kTokC * t.np * h;
     t.flow_n = int(cdiv(int(rt), kBM)) + 1;
-    want[B_FLOW] = size_t(kFlowCnts) * t.flow_n * sizeof(unsigned int);
+    want[B_FLOW] = size_t(kFlowCnts) * t.flow_n * kFlowPitch * sizeof(unsigned int);
     size_t off = align_up(sizeof(Control), kAlign);
     for (int b = 0; b < kNumBufs; b++) {
         t.off[b] = off, t.bytes[b] = want[b];

@@ -51,6 +51,10 @@ struct Bufs {
 // launch waits for (e + 1) times what one block adds.
 enum FlowCnt { FC_QKVG, FC_TO, FC_TC, FC_ACT1, FC_ACT2, FC_TX, kFlowCnts };
 
+// A counter has a 128-byte line of its own: many CTAs poll it while others add to it, and neighbours in one line
+// would share that traffic.
+constexpr int kFlowPitch = 32;
+
 // control words at the head of the workspace, zeroed before every launch
 struct Control {
     unsigned int barrier; // arrivals of the grid barrier, monotonic; kBarrierPoison is set with the status

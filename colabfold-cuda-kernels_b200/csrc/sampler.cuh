@@ -337,7 +337,7 @@ __device__ CCK_PHASE_FN void pair_fill_pads(const KP& p, Deal& d) {
         }
     }
     if (p.flow) { // the completion counters of the token blocks' chains
-        for (size_t i = tid; i < size_t(kFlowCnts) * p.flow_n; i += nth) {
+        for (size_t i = tid; i < size_t(kFlowCnts) * p.flow_n * kFlowPitch; i += nth) {
             p.flow_cnt[i] = 0;
         }
     }
