@@ -24,8 +24,8 @@
 //                        when that store has landed, under the next item's first chunk.
 // O stays in TMEM for the whole item: P·V accumulates over the chunks. The exponentials of a row are
 // taken against a reference value that follows the row's running maximum lazily: it moves only when
-// the maximum has grown by more than 2^8 (a warp decides together, since TMEM accesses are
-// warp-wide), and then the row's O and sum are rescaled in place before the chunk's P is handed over.
+// a chunk's exponentials add up to more than 2^8 (a warp decides together, since TMEM accesses are
+// warp-wide), and then the row's O and sum are rescaled in place and the chunk's exponentials taken again.
 // Until then P may reach 2^8 instead of 1, which changes nothing in bf16 or f32 but the exponent.
 // Math as the reference's token attention (src/diffusion/attention.cuh:145-249): logits in base 2,
 // P rounded to bf16 before P·V, row sums from the unrounded P.
@@ -43,7 +43,9 @@ static_assert(kTcRows == kBM, "one softmax thread per row of a 128-row UMMA");
 static_assert(kTcWarps == kAttnItemWarps, "the completion counters of TO count the warps of an item");
 constexpr int kTcTmaWarp1 = kAuxWarp0, kTcMmaWarp1 = kAuxWarp0 + 1; // the second track's TMA and MMA threads
 constexpr int kTcKvStages = 3, kTcBiasStages = 2;
-constexpr float kTcLazy = 8.f; // the exponentials' reference value trails the running maximum by up to 2^8
+// The exponentials' reference value trails the running maximum by up to 2^8: an exponential above that makes its
+// chunk's sum exceed it too.
+constexpr float kTcLazySum = 256.f;
 constexpr int kTcKBytes = kTcKeys * 128;          // 8 KB: 64 keys x 64 columns
 constexpr int kTcVBytes = kHeadD * 128;           // 6 KB: 48 head dims x 64 keys
 constexpr int kTcKvBytes = kTcKBytes + kTcVBytes; // 14 KB
@@ -106,6 +108,14 @@ __device__ inline void attn_tc_init() {
     }
 }
 
+// two f32 plus the two bf16 of a word
+__device__ __forceinline__ float2 add_bf2(uint32_t w, float2 x) {
+    float2 y;
+    asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tadd.rn.f32.bf16 %0, lo, %3;\n\tadd.rn.f32.bf16 %1, hi, %4;\n\t}"
+        : "=f"(y.x), "=f"(y.y)
+        : "r"(w), "f"(x.x), "f"(x.y));
+    return y;
+}
 // 16 f32 columns of this warp's 32 TMEM lanes, without the wait
 __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
@@ -399,50 +409,84 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                     }
                     cp_async_commit();
                 }
-                uint32_t s0[32], s1[32]; // the row's scores of the chunk's first and second 32 keys
-                tmem_ld32_issue(tt + kTcS + bi * 64, s0);
-                tmem_ld32_issue(tt + kTcS + bi * 64 + 32, s1);
-                // the row's 64 pair logits: 8 swizzled 16-byte pieces of the tile
                 mbar_wait(&B.b_full[bst], (g / kTcBiasStages) & 1, &ctl->abort);
-                const char* brow = base + kTcBiasOff + bst * kTcBiasBytes + row_in * 128;
-                tmem_ld_wait(s0);
-                tmem_ld_wait(s1);
-                float mxp[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}; // four chains, so that the maxima do not serialise
-                // scores in base 2 with the pair logits added, in place; the chunk's maximum
-                auto add_bias = [&](uint32_t(&sr)[32], int hf) {
+                const char* brow = base + kTcBiasOff + bst * kTcBiasBytes + row_in * 128; // the row's 64 pair logits: 8 swizzled 16-byte pieces
+                // One pass over the chunk: exponentials of the scores (base 2, pair logits added) against the
+                // reference value m, P = 2^(score - m) as bf16 to TMEM (16 keys are 8 columns), and their sum. A
+                // warp issues an instruction every two cycles or so, and eight warps of softmax are what
+                // the SM has: the pass is as short as it can be. The pair logits are added as they are (a mixed
+                // f32 + bf16 addition instead of unpacking), and only an item's first chunk looks for its
+                // maximum: later ones take the reference of the chunks before on trust. Where a score has
+                // outgrown it by 2^kTcLazy, its exponential alone makes the sum say so; the pass is then repeated.
+                // The chunk's P buffer held P of chunk g - 2. That chunk's P·V was issued before this chunk's
+                // Q·Kᵀ, by the same warp, and the commit behind s_full covers everything issued before it:
+                // having seen S, the buffer is free.
+                auto row_max = [&]() {
+                    float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll 1
+                    for (int hf = 0; hf < 2; hf++) {
+                        uint32_t sr[32];
+                        tmem_ld32_issue(tt + kTcS + bi * 64 + 32 * hf, sr);
+                        tmem_ld_wait(sr);
 #pragma unroll
-                    for (int jj = 0; jj < 4; jj++) {
-                        const uint4 bw = *reinterpret_cast<const uint4*>(brow + (((4 * hf + jj) ^ (row_in & 7)) << 4));
-                        const uint32_t w[4] = {bw.x, bw.y, bw.z, bw.w};
+                        for (int jj = 0; jj < 4; jj++) {
+                            const uint4 bw = *reinterpret_cast<const uint4*>(brow + (((4 * hf + jj) ^ (row_in & 7)) << 4));
+                            const uint32_t w[4] = {bw.x, bw.y, bw.z, bw.w};
 #pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            const int i = 8 * jj + 2 * k;
-                            const float2 a = __ffma2_rn(make_float2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), scale2,
-                                                        make_float2(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xFFFF0000u)));
-                            sr[i] = __float_as_uint(a.x), sr[i + 1] = __float_as_uint(a.y);
-                            mxp[k] = max3(mxp[k], a.x, a.y);
+                            for (int k = 0; k < 4; k++) {
+                                const float2 x = add_bf2(w[k], __fmul2_rn(make_float2(__uint_as_float(sr[8 * jj + 2 * k]), __uint_as_float(sr[8 * jj + 2 * k + 1])), scale2));
+                                mx[k & 1] = max3(mx[k & 1], x.x, x.y);
+                            }
                         }
                     }
+                    return fmaxf(mx[0], mx[1]);
                 };
-                add_bias(s0, 0);
-                add_bias(s1, 1);
-                // The tile is in registers: its slot may be refilled. The refill is a TMA write (async proxy)
-                // over what this thread has just read with ordinary loads: the proxy fence orders the two.
-                fence_async_smem();
-                mbar_arrive(&B.b_empty[bst]);
-                const float mx = max3(mxp[0], mxp[1], fmaxf(mxp[2], mxp[3]));
-                CCK_TRACE_EV(0x34 + t, g - g0);
                 if (c == 0) {
-                    m = mx;
-                } else if (__any_sync(0xffffffffu, mx > m + kTcLazy)) {
+                    m = row_max();
+                }
+                float chunk_l;
+                for (;;) {
+                    const float2 neg_m = make_float2(-m, -m);
+                    float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+                    for (int hf = 0; hf < 2; hf++) {
+                        uint32_t sr[32];
+                        tmem_ld32_issue(tt + kTcS + bi * 64 + 32 * hf, sr);
+                        tmem_ld_wait(sr);
+#pragma unroll
+                        for (int jj = 0; jj < 2; jj++) {
+                            uint32_t pk[8];
+#pragma unroll
+                            for (int q4 = 0; q4 < 2; q4++) {
+                                const uint4 bw = *reinterpret_cast<const uint4*>(brow + (((4 * hf + 2 * jj + q4) ^ (row_in & 7)) << 4));
+                                const uint32_t w[4] = {bw.x, bw.y, bw.z, bw.w};
+#pragma unroll
+                                for (int k = 0; k < 4; k++) {
+                                    const int i = 16 * jj + 8 * q4 + 2 * k;
+                                    const float2 x = add_bf2(w[k], __ffma2_rn(make_float2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), scale2, neg_m));
+                                    const float2 e = make_float2(ex2_fast(x.x), ex2_fast(x.y));
+                                    sum2[k & 1] = __fadd2_rn(sum2[k & 1], e);
+                                    pk[4 * q4 + k] = pack_bf2(e.x, e.y);
+                                }
+                            }
+                            tmem_st8(tt + kTcP + bi * 32 + 16 * hf + 8 * jj, pk);
+                        }
+                    }
+                    chunk_l = (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
+                    if (c == 0 || !__any_sync(0xffffffffu, !(chunk_l <= kTcLazySum))) {
+                        break;
+                    }
                     // The reference value moves: the rows of this warp rescale what they have accumulated
                     // (every lane, by its own factor: TMEM accesses are warp-wide). O is current once the
                     // previous chunk's P·V is done, and the next P·V waits for this chunk's P.
-                    const float mn = fmaxf(m, mx), f = ex2_fast(m - mn);
+                    const float mn = fmaxf(m, row_max());
+                    if (!__any_sync(0xffffffffu, mn > m)) { // (a large sum of small exponentials)
+                        break;
+                    }
+                    const float f = ex2_fast(m - mn);
                     m = mn, l *= f;
                     mbar_wait(&B.pv_done[bi ^ 1], ((g - 1) >> 1) & 1, &ctl->abort);
                     tc_fence_after();
-                    // (16 columns at a time: the chunk's 64 scores are live in registers beside them)
 #pragma unroll 1
                     for (int i = 0; i < kHeadD; i += 16) {
                         uint32_t r[16];
@@ -455,29 +499,12 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                         tmem_st16(tt + kTcO + i, r);
                     }
                 }
-                // The chunk's P buffer held P of chunk g - 2. That chunk's P·V was issued before this chunk's
-                // Q·Kᵀ, by the same thread, and the commit behind s_full covers everything issued before it:
-                // having seen S, the buffer is free.
-                const float2 neg_m = make_float2(-m, -m);
-                float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-                // P = 2^(score - reference) as bf16: 16 keys are 8 columns
-                auto exp_store = [&](const uint32_t(&sr)[32], int hf) {
-#pragma unroll
-                    for (int jj = 0; jj < 2; jj++) {
-                        uint32_t pk[8];
-#pragma unroll
-                        for (int k = 0; k < 8; k++) {
-                            const float2 x = __fadd2_rn(make_float2(__uint_as_float(sr[16 * jj + 2 * k]), __uint_as_float(sr[16 * jj + 2 * k + 1])), neg_m);
-                            const float2 e = make_float2(ex2_fast(x.x), ex2_fast(x.y));
-                            sum2[k & 1] = __fadd2_rn(sum2[k & 1], e);
-                            pk[k] = pack_bf2(e.x, e.y);
-                        }
-                        tmem_st8(tt + kTcP + bi * 32 + 16 * hf + 8 * jj, pk);
-                    }
-                };
-                exp_store(s0, 0);
-                exp_store(s1, 1);
-                l += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
+                l += chunk_l;
+                // The tile of pair logits has been used: its slot may be refilled. The refill is a TMA write (async
+                // proxy) over what this thread has read with ordinary loads: the proxy fence orders the two.
+                fence_async_smem();
+                mbar_arrive(&B.b_empty[bst]);
+                CCK_TRACE_EV(0x34 + t, g - g0);
                 tmem_st_wait();
                 tc_fence_before();
                 mbar_arrive(&B.p_full[bi]);
