@@ -33,12 +33,13 @@ __host__ __device__ inline PhiloxWords philox(uint32_t c0, uint32_t c1, uint32_t
     }
     return s;
 }
+// (Out of line: one copy of some 250 instructions instead of four per caller, whose code is fetched anew every step.)
 // Four standard normals of one counter: Box-Muller on word pairs (0, 1) and (2, 3), uniforms from the
 // 24 high bits, the first of a pair kept away from zero
 struct Normals4 {
     float z[4];
 };
-__device__ inline Normals4 philox_normals(uint32_t idx, uint32_t step, uint32_t sample, uint32_t stream, uint32_t k0, uint32_t k1) {
+__device__ __noinline__ Normals4 philox_normals(uint32_t idx, uint32_t step, uint32_t sample, uint32_t stream, uint32_t k0, uint32_t k1) {
     const PhiloxWords s = philox(idx, step, sample, stream, k0, k1);
     constexpr float kInv24 = 1.0f / 16777216.f, kTwoPi = 6.2831853071795864f;
     Normals4 n;
@@ -89,16 +90,16 @@ struct RigidMotion {
     }
 };
 __device__ inline RigidMotion random_rigid(uint32_t step, uint32_t sample, uint32_t k0, uint32_t k1) {
-    const Normals4 a = philox_normals(0, step, sample, STREAM_AUGMENT, k0, k1);
-    const Normals4 b = philox_normals(1, step, sample, STREAM_AUGMENT, k0, k1);
-    const Normals4 c = philox_normals(2, step, sample, STREAM_AUGMENT, k0, k1);
-    const V3 first{a.z[0], a.z[1], a.z[2]}, second{a.z[3], b.z[0], b.z[1]};
+    // (a whole warp calls: lane i forms the normals of counter i % 4)
+    const Normals4 n = philox_normals(lane_id() & 3, step, sample, STREAM_AUGMENT, k0, k1);
+    auto z = [&](int counter, int i) { return __shfl_sync(0xffffffffu, n.z[i], counter); };
+    const V3 first{z(0, 0), z(0, 1), z(0, 2)}, second{z(0, 3), z(1, 0), z(1, 1)};
     RigidMotion m;
     m.e0 = first / length_floored(first);
     const V3 rest = second - dot(second, m.e0) * m.e0;
     m.e1 = rest / length_floored(rest);
     m.e2 = cross(m.e0, m.e1);
-    m.t = V3{b.z[2], b.z[3], c.z[0]};
+    m.t = V3{z(1, 2), z(1, 3), z(2, 0)};
     return m;
 }
 

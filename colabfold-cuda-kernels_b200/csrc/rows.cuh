@@ -97,52 +97,51 @@ __device__ __forceinline__ void rows_done(Deal& d, int rows) {
 
 // ---- conditioning
 
-// ntv = LN_affine(cos(2π(¼ ln(t/σd)·w + b))) @ WN on one CTA (reference: src/diffusion/rows.cuh:168-200)
+// ntv = LN_affine(cos(2π(¼ ln(t/σd)·w + b))) @ WN (reference: src/diffusion/rows.cuh:168-200), four columns per
+// CTA: every CTA forms the 256 Fourier features, thread k holds feature k's share of the four columns. (One
+// CTA walking all columns took 256 dependent steps: most of this phase's 7.5 us at 32 x 1 and 24 us at 512 x 5.)
+constexpr int kNoiseCols = 4;
 __device__ CCK_PHASE_FN void noise_vector(const KP& p, Deal& d, float t) {
-    if (d.first() == 0) {
-        float* e = reinterpret_cast<float*>(smem_base());
-        float* red = e + kFourier;
-        const float lt = 0.25f * logf(t / kSigmaData);
-        const int k = threadIdx.x; // one thread per Fourier feature; the warps past them add zeros
+    const int items = p.cs / kNoiseCols;
+    for (int it = d.first(); it < items; it += gridDim.x) {
+        float* red = reinterpret_cast<float*>(smem_base()); // [2 + kNoiseCols][kWarps]
+        const int k = threadIdx.x, lane = lane_id(), warp = warp_id(); // one thread per Fourier feature; the warps past them add zeros
         const bool on = k < kFourier;
+        const float lt = 0.25f * logf(t / kSigmaData);
+        const float4 w = on ? *reinterpret_cast<const float4*>(p.tw.wn + size_t(k) * p.cs + kNoiseCols * it) : make_float4(0.f, 0.f, 0.f, 0.f);
         const float x = on ? cosf(2.f * 3.14159265358979323846f * (lt * p.tw.fourier_w[k] + p.tw.fourier_b[k])) : 0.f;
-        float s = warp_sum(x);
-        if (lane_id() == 0) {
-            red[warp_id()] = s;
-        }
-        __syncthreads();
-        s = 0.f;
-        for (int w = 0; w < kWarps; w++) {
-            s += red[w];
-        }
-        const float mean = s / kFourier;
-        __syncthreads();
-        float q = warp_sum(on ? (x - mean) * (x - mean) : 0.f);
-        if (lane_id() == 0) {
-            red[warp_id()] = q;
-        }
-        __syncthreads();
-        q = 0.f;
-        for (int w = 0; w < kWarps; w++) {
-            q += red[w];
-        }
-        const float rstd = 1.f / sqrtf(q / kFourier + kLnEps);
-        if (on) {
-            e[k] = (x - mean) * rstd * p.tw.noise_ln[k] + p.tw.noise_lno[k];
-        }
-        __syncthreads();
-        for (int c = threadIdx.x; c < p.cs; c += kThreads) {
-            float acc = 0.f;
-            for (int j = 0; j < kFourier; j++) {
-                acc += e[j] * p.tw.wn[j * p.cs + c];
+        auto cta_sum = [&](float v, float* slot) {
+            v = warp_sum(v);
+            if (lane == 0) {
+                slot[warp] = v;
             }
-            p.buf.ntv[c] = acc;
+            __syncthreads();
+            float s = 0.f;
+            for (int i = 0; i < kWarps; i++) {
+                s += slot[i];
+            }
+            return s;
+        };
+        const float mean = cta_sum(x, red) / kFourier;
+        const float rstd = 1.f / sqrtf(cta_sum(on ? (x - mean) * (x - mean) : 0.f, red + kWarps) / kFourier + kLnEps);
+        const float e = on ? (x - mean) * rstd * p.tw.noise_ln[k] + p.tw.noise_lno[k] : 0.f;
+        const float4 part = make_float4(warp_sum(e * w.x), warp_sum(e * w.y), warp_sum(e * w.z), warp_sum(e * w.w));
+        if (lane == 0) {
+            *reinterpret_cast<float4*>(red + 2 * kWarps + kNoiseCols * warp) = part;
+        }
+        __syncthreads();
+        if (threadIdx.x < kNoiseCols) {
+            float acc = 0.f;
+            for (int i = 0; i < kWarps; i++) {
+                acc += red[2 * kWarps + kNoiseCols * i + threadIdx.x];
+            }
+            p.buf.ntv[kNoiseCols * it + threadIdx.x] = acc;
         }
         __syncthreads();
     }
-    d.advance(1);
+    d.advance(items);
 }
-static_assert(kThreads >= kFourier, "noise_vector maps one thread to one Fourier feature");
+static_assert(kThreads >= kFourier && (2 * kWarps) % 4 == 0, "noise_vector maps one thread to one Fourier feature; its partial sums are read as float4");
 
 // SCT = bf16(LN(sc)·S + O); the first call also forms sc = SC_BASE + ntv
 // (reference: src/diffusion/rows.cuh:202-222). cs = 384.
@@ -369,28 +368,35 @@ __device__ CCK_PHASE_FN void token_final_ln(const KP& p, Deal& d, unsigned int e
 __device__ CCK_PHASE_FN void aggr_gather(const KP& p, Deal& d) {
     const int rows = p.S * p.N;
     for (int r = row_first(d); r < rows; r += row_step()) {
-        const int s = r / p.N, n = r % p.N;
+        const int s = r / p.N, n = r % p.N, lane = lane_id();
+        // the token's slots, one per lane; then its atoms' rows two at a time, in slot order (a slot per step, each
+        // waiting for its index and then for its row, was 24 trips to L2: 24 -> 20 us at 512 x 5, 10 -> 7.7 at 32 x 1)
+        const float wl = lane < kSlots ? p.geo.tam[n * kSlots + lane] : 0.f;
+        const int al = lane < kSlots ? p.geo.q2ta[n * kSlots + lane] : -1;
+        const RowV<6> se = load_f32<6>(p.buf.se + size_t(n) * kTokC);
+        const float wsum = warp_sum(wl);
+        const float* agt = p.buf.agt + size_t(s) * p.A * kTokC;
         RowV<6> sum;
 #pragma unroll
         for (int j = 0; j < 6; j++) {
             sum.v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        float wsum = 0.f;
-        for (int j = 0; j < kSlots; j++) {
-            const float w = p.geo.tam[n * kSlots + j];
-            const int a = p.geo.q2ta[n * kSlots + j];
-            wsum += w;
-            if (a >= 0) {
-                const RowV<6> v = load_f32<6>(p.buf.agt + (size_t(s) * p.A + a) * kTokC);
+        unsigned int left = __ballot_sync(0xffffffffu, al >= 0);
+        while (left) {
+            const int j0 = __ffs(left) - 1;
+            left &= left - 1;
+            const int j1 = left ? __ffs(left) - 1 : j0; // (none left: the same row once more, with weight 0)
+            const float w0 = __shfl_sync(0xffffffffu, wl, j0), w1 = left ? __shfl_sync(0xffffffffu, wl, j1) : 0.f;
+            const RowV<6> v0 = load_f32<6>(agt + size_t(__shfl_sync(0xffffffffu, al, j0)) * kTokC);
+            const RowV<6> v1 = load_f32<6>(agt + size_t(__shfl_sync(0xffffffffu, al, j1)) * kTokC);
+            left &= left - 1;
 #pragma unroll
-                for (int k = 0; k < 6; k++) {
-                    sum.v[k].x += w * v.v[k].x, sum.v[k].y += w * v.v[k].y;
-                    sum.v[k].z += w * v.v[k].z, sum.v[k].w += w * v.v[k].w;
-                }
+            for (int k = 0; k < 6; k++) {
+                sum.v[k].x = sum.v[k].x + w0 * v0.v[k].x + w1 * v1.v[k].x, sum.v[k].y = sum.v[k].y + w0 * v0.v[k].y + w1 * v1.v[k].y;
+                sum.v[k].z = sum.v[k].z + w0 * v0.v[k].z + w1 * v1.v[k].z, sum.v[k].w = sum.v[k].w + w0 * v0.v[k].w + w1 * v1.v[k].w;
             }
         }
         const float inv = 1.f / fmaxf(wsum, 1e-10f);
-        const RowV<6> se = load_f32<6>(p.buf.se + size_t(n) * kTokC);
 #pragma unroll
         for (int k = 0; k < 6; k++) {
             sum.v[k] = make_float4(sum.v[k].x * inv + se.v[k].x, sum.v[k].y * inv + se.v[k].y,
