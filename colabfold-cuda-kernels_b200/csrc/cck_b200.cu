@@ -470,7 +470,7 @@ int mk_gemm_test(const uint16_t* A, const uint16_t* W, float* C, int M, int N, i
         cudaFree(da), cudaFree(dw), cudaFree(dc), cudaFree(ctl);
         return 1;
     }
-    int bn = (tile == 64 || tile == 128 || tile == 256) && N % tile == 0 ? tile : choose_bn(M, N, dev.sms);
+    int bn = (tile == 64 || tile == 128 || tile == 256) && N % tile == 0 ? tile : choose_bn(M, N, K / kBK, dev.sms);
     Launch L;
     memset(&L, 0, sizeof L);
     L.kp.ctl = ctl, L.kp.wait_cycles = kWaitCycles;

@@ -7,6 +7,7 @@
 // synchronised on the operator path.
 #pragma once
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -274,10 +275,13 @@ static int encode_rows_store_map(CUtensorMap* m, const void* base, size_t rows, 
     return E_OK;
 }
 
-// the column tile of a GEMM: the widest of 256/128/64 that divides n, unless a narrower one needs
-// fewer whole rounds over the grid (weighted by width)
-// (GLU GEMMs whose units have 96 rows take 192 or 96)
-inline int choose_bn(size_t m, int n, int grid, int max_bn = kMaxBN, int unit = 64) {
+// The column tile of a GEMM with m rows, n columns and kblocks k-blocks: 256, 128 or 64 (GLU GEMMs whose units have
+// 96 rows: 192 or 96), the one with the least estimated time of the CTA that has most tiles. Measured: with the
+// whole grid loading, a k-block arrives at 83 bytes per cycle; an epilogue takes about 18 cycles a column and
+// overlaps the next tile's main loop, except the last one; going from one tile to the next costs some 1500.
+// (Choosing by rounds and width alone gave 256 columns where 13 row tiles x 12 column tiles need two rounds
+// of the grid for 8 tiles, 320 x 5: 2.46 -> 2.28 ms per step, and 128 where that is bound by the loads, 1024 x 5: 5.32 -> 5.04.)
+inline int choose_bn(size_t m, int n, int kblocks, int grid, int max_bn = kMaxBN, int unit = 64) {
     int best = unit;
     double best_cost = 1e300;
     for (int bn = 4 * unit; bn >= unit; bn /= 2) {
@@ -285,7 +289,8 @@ inline int choose_bn(size_t m, int n, int grid, int max_bn = kMaxBN, int unit = 
             continue;
         }
         const size_t tiles = (m + kBM - 1) / kBM * size_t(n / bn);
-        const double cost = double((tiles + grid - 1) / grid) * (bn + 24);
+        const double kblock = (kStageA + bn * kBK * 2) / 83.0, epi = 18.0 * bn;
+        const double cost = double((tiles + grid - 1) / grid) * (std::max(kblocks * kblock, epi) + 1500) + epi;
         if (cost < best_cost) {
             best_cost = cost, best = bn;
         }
@@ -605,7 +610,8 @@ static int make_launch(Launch& L, const Template& t, const Device& dev, const vo
         {TM_B_DEC_W2, IN_DEC_W2, 3 * kAtomC, kAtomHidden, ra, kAtomC, kResidMaxBnF32},
     };
     for (const BMap& m : bmaps) {
-        const int bn = choose_bn(m.m, m.n, dev.sms, m.max_bn, m.unit);
+        const int kb = int(m.cols / kBK) * (m.id == TM_B_ENC_W1 || m.id == TM_B_DEC_W1 ? 2 : 1); // (hi | lo inputs: W1 of the atoms twice)
+        const int bn = choose_bn(m.m, m.n, kb, dev.sms, m.max_bn, m.unit);
         p.bn[m.id] = bn;
         if (int e = encode_map(&L.tmap[m.id], in[m.in], m.rows, m.cols, m.cols, bn)) {
             return e;
