@@ -621,7 +621,7 @@ struct FlowWait {
         }
     }
     __device__ __forceinline__ bool ready() {
-        if (ld_relaxed(cnt) >= target) {
+        if (ld_acquire(cnt) >= target) { // (an acquire at every look, so that no fence, which takes as long as a look, follows the last)
             return true;
         }
         return *abort || (++looks % 32 == 0 && given_up()); // (the status word is another way to L2: not at every look)
@@ -637,34 +637,19 @@ struct FlowWait {
     }
     // what the signalling warps wrote is visible to what follows: this thread's reads and TMA loads
     __device__ __forceinline__ void acquire() {
-        fence_acq_rel_gpu();
         fence_async_global();
     }
 };
-// One thread waits until the counters [c0, c1] have reached target; what it then reads through TMA is what
-// the signalling warps wrote. The counters are read eight at a time with relaxed loads (one L2 round
-// trip for the batch, not one each) and one acquire fence follows the last read.
+// One thread waits until the counters [c0, c1] have reached target, one after the other; what it then reads is what
+// the signalling warps wrote.
 __device__ __forceinline__ bool flow_wait(const unsigned int* cnt, int c0, int c1, unsigned int target, volatile int* abort) {
     const long long t0 = clock64();
     unsigned int looks = 0;
     if (*abort) { // a wait inside this CTA gave up earlier: tell the grid, which would otherwise wait for this CTA's units
         fail_launch(ST_PIPE_TIMEOUT, 0);
     }
-    for (int b0 = c0; b0 <= c1; b0 += 8) {
-        for (;;) {
-            unsigned int v[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                v[i] = b0 + i <= c1 ? ld_relaxed(cnt + (b0 + i) * kFlowPitch) : target;
-            }
-            bool ok = true;
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                ok = ok && v[i] >= target;
-            }
-            if (ok) {
-                break;
-            }
+    for (int c = c0; c <= c1; c++) {
+        while (ld_acquire(cnt + c * kFlowPitch) < target) {
             if (*abort) {
                 return false;
             }
@@ -674,10 +659,8 @@ __device__ __forceinline__ bool flow_wait(const unsigned int* cnt, int c0, int c
                 *abort = 1;
                 return false;
             }
-            __nanosleep(20);
         }
     }
-    fence_acq_rel_gpu();
     fence_async_global();
     return true;
 }
