@@ -187,6 +187,8 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
     const int warp = warp_id(), lane = lane_id(), first = d.first();
     const uint32_t tmem = ctl->tmem_base;
     const bool flow = p.flow;
+    const int alt = flow ? int(epoch & 1) : 0; // which of the two buffers holds this block's q, k, v and gates
+    const bf16* const qkvg = alt ? p.buf.qkvg2 : p.buf.qkvg;
 
     if (warp == 0 || warp == kTcTmaWarp1) {
         // ---- TMA producer of one track (the whole warp passes here, one lane issues: ptx.cuh). Issue order:
@@ -200,8 +202,8 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
             TcTrackBars& B = bars->t[t];
             const uint32_t base = uni(smem_u32(sm + t * kTcTrackBytes)), bar0 = uni(smem_u32(&B));
             auto bar = [&](uint64_t& x) { return bar0 + uint32_t(reinterpret_cast<char*>(&x) - reinterpret_cast<char*>(&B)); };
-            const CUtensorMap* mqk = &L.tmap[TM_T_QK];
-            const CUtensorMap* mvt = &L.tmap[TM_T_VT];
+            const CUtensorMap* mqk = &L.tmap[TM_T_QK + alt];
+            const CUtensorMap* mvt = &L.tmap[TM_T_VT + alt];
             const CUtensorMap* mpl = &L.tmap[TM_T_PLG];
             const unsigned int qkvg_done = (epoch + 1) * (unsigned int)(gd_table()[GD_TOK_QKVG].nt * kWorkWarps); // (the counters count on through the launch)
             const uint32_t j0 = uni(bars->items[t]), g0 = uni(bars->chunks[t]);
@@ -405,7 +407,7 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                     for (int i = 0; i < kTcOutPieces; i++) {
                         const int pc = i * 32 + lane, r = pc / kTcOutPieces, o = pc % kTcOutPieces;
                         const size_t grow = size_t(s) * N + min(qb * kTcRows + q * 32 + r, N - 1);
-                        cp_async16(stage + r * kTcOutPitch + o * 16, p.buf.qkvg + grow * kQKVG + 3 * kTokC + h * kHeadD + o * 8, true);
+                        cp_async16(stage + r * kTcOutPitch + o * 16, qkvg + grow * kQKVG + 3 * kTokC + h * kHeadD + o * 8, true);
                     }
                     cp_async_commit();
                 }

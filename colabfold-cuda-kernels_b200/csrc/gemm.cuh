@@ -666,10 +666,10 @@ __device__ __forceinline__ bool flow_wait(const unsigned int* cnt, int c0, int c
 }
 // Arrivals that complete row block rb of a GEMM's A (descriptor g, depc set) in one token block. TO:
 // the attention items of every block of 128 queries (per sample of g.period rows) that the rows
-// touch, 16 heads x 4 warps each. TC: the column tiles of W1 over these rows, 8 warps each. TX: the
+// touch, 16 heads x 4 warps each. TC: the column tiles of W1 over these rows, 8 warps each. TX, TX0: the
 // adaLN rows of the block.
 __device__ __forceinline__ unsigned int flow_target(const GemmDesc& g, int which, int rb, int w1_tiles) {
-    if (which == FC_TX) {
+    if (which == FC_TX || which == FC_TX0) {
         return (unsigned int)(min(kBM, g.m - rb * kBM));
     }
     if (which != FC_TO) {
@@ -687,6 +687,11 @@ template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, con
     SmemCtl* ctl = smem_ctl();
     GemmDesc g = gd; // a private copy: stores through its pointers cannot alias it
     g.bias = g.bias ? g.bias + size_t(b) * g.bias_step : nullptr;
+    if constexpr (E == EPI_BF16) {
+        if ((gd.fl & GF_ALT) && (epoch & 1)) {
+            g.out = kp().buf.qkvg2, g.vt = kp().buf.vt2;
+        }
+    }
     CCK_TRACE_BEGIN_IF(4, threadIdx.x == kWorkWarp0 * 32);
     CCK_TRACE_EV(0x70, E);
     for (int t = tb; t < te; t += ts, tile++) {
@@ -695,14 +700,13 @@ template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, con
         const uint32_t buf = tile & 1, tpar = (tile >> 1) & 1;
         const uint32_t acc = ctl->tmem_base + buf * kMaxBN;
         if constexpr (E == EPI_RESID) {
-            // The epilogue fetches the residual rows ahead, under the main loop. Where the operation that
-            // wrote them last shares this phase (W2: the rows come from WO, no barrier since), they are
-            // final once the tile's own dependency is met: WO's tiles over the rows came before the adaLN
-            // rows, W1's tiles and so the counter that the tile's TMA thread waits for as well.
-            if ((gd.fl >> GF_DEP_SHIFT & GF_CNT_MASK) == 1 + FC_TC) {
+            // The epilogue fetches the residual rows ahead, under the main loop. On completion counters the
+            // operation that wrote them last may still be running elsewhere: W2 of the block before for WO, which
+            // the attention's adaLN rows have waited for; WO for W2, which came before W1's tiles.
+            if (const int depc = gd.fl >> GF_DEP_SHIFT & GF_CNT_MASK) {
                 if (lane_id() == 0) {
-                    flow_wait(flow_cnt(kp(), FC_TC), row0 / kBM, row0 / kBM, (epoch + 1) * flow_target(gd, FC_TC, row0 / kBM, gd_table()[GD_TOK_W1].nt),
-                              &ctl->abort);
+                    const int which = depc == 1 + FC_TO ? FC_TX0 : FC_TC, rb = row0 / kBM;
+                    flow_wait(flow_cnt(kp(), which), rb, rb, (epoch + 1) * flow_target(gd, which, rb, gd_table()[GD_TOK_W1].nt), &ctl->abort);
                 }
                 __syncwarp();
             }

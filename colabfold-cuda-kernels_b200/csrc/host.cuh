@@ -53,6 +53,10 @@ inline int fail(int code, const std::string& msg) {
     return code;
 }
 
+// the token blocks on completion counters: not with PARALLEL or QKNORM, whose blocks have other phases
+inline bool flow_allowed(uint32_t flags) {
+    return !(flags & (F_PARALLEL | F_QKNORM));
+}
 // Everything that depends only on the shapes: model widths and the workspace layout
 struct Template {
     int S, Nb, NSb, nsteps;
@@ -173,6 +177,9 @@ static int make_template(Template& t, int S, int Nb, int NSb, int nsteps, uint32
     want[B_VT] = size_t(S) * kTokC * t.np * h;
     t.flow_n = int(cdiv(int(rt), kBM)) + 1;
     want[B_FLOW] = size_t(kFlowCnts) * t.flow_n * kFlowPitch * sizeof(unsigned int);
+    if (flow_allowed(flags)) { // the second buffers of the token blocks' chains
+        want[B_QKVG2] = want[B_QKVG], want[B_VT2] = want[B_VT];
+    }
     size_t off = align_up(sizeof(Control), kAlign);
     for (int b = 0; b < kNumBufs; b++) {
         t.off[b] = off, t.bytes[b] = want[b];
@@ -321,9 +328,6 @@ struct ProgramWriter {
 // operations chained by completion counters (FlowCnt) instead of barriers. Not with PARALLEL or QKNORM, whose blocks have other phases; not in a debug run that
 // stops at a phase of the reference's schedule, which counts the barriers.
 constexpr uint32_t kProgFlow = 1u << 30;
-inline bool flow_allowed(uint32_t flags) {
-    return !(flags & (F_PARALLEL | F_QKNORM));
-}
 static void write_denoise(ProgramWriter& w, uint32_t flags) {
     const bool qkn = flags & F_QKNORM, par = flags & F_PARALLEL;
     const bool flow = (flags & kProgFlow) && flow_allowed(flags);
@@ -387,8 +391,8 @@ static void write_denoise(ProgramWriter& w, uint32_t flags) {
         w.op(FN_TOK_ATTN, 0, kLoopB, END_PHASE, K_T_ATTN);
         w.gemm(GD_TOK_WO, kLoopB, END_PHASE, K_T_WO);
     } else if (flow) {
-        w.op(FN_TOK_ADALN, TM_ATTN_SCALE, kLoopB, END_PHASE, K_T_W2);
-        w.gemm(GD_TOK_QKVG, kLoopB);
+        w.op(FN_TOK_ADALN, TM_ATTN_SCALE, kLoopB, END_ARRIVE, K_T_W2);
+        w.gemm(GD_TOK_QKVG, kLoopB); // a tile waits for the adaLN rows of its block of 128
         w.op(FN_CTA_SYNC);
         w.op(FN_TOK_ATTN, 0, kLoopB);
         w.op(FN_CTA_SYNC);
@@ -536,7 +540,7 @@ static int make_launch(Launch& L, const Template& t, const Device& dev, const vo
     b.sct = BH(B_SCT), b.scln0 = BH(B_SCLN0), b.scbf = BH(B_SCBF), b.sch = BH(B_SCH), b.mods = BH(B_MODS);
     b.ao = BH(B_AO), b.abf = BH(B_ABF), b.aqg = BH(B_AQG), b.akv = BH(B_AKV), b.tx = BH(B_TX), b.qkvg = BH(B_QKVG);
     b.to = BH(B_TO), b.tc = BH(B_TC), b.plg = BH(B_PLG), b.axq = BH(B_AXQ), b.axk = BH(B_AXK), b.axhl = BH(B_AXHL);
-    b.aca = BH(B_ACA), b.vt = BH(B_VT), b.tx2 = t.flags & F_PARALLEL ? BH(B_TX2) : b.tx;
+    b.aca = BH(B_ACA), b.vt = BH(B_VT), b.qkvg2 = BH(B_QKVG2), b.vt2 = BH(B_VT2), b.tx2 = t.flags & F_PARALLEL ? BH(B_TX2) : b.tx;
     p.flow_cnt = reinterpret_cast<unsigned int*>(ws + t.off[B_FLOW]);
     p.ctl = reinterpret_cast<Control*>(ws);
 
@@ -558,11 +562,13 @@ static int make_launch(Launch& L, const Template& t, const Device& dev, const vo
         }
     }
     // token attention: Q/K tiles of QKVG (64 columns x 64 rows), VT tiles (64 keys x 48 dims), bias tiles
-    if (int e = encode_map(&L.tmap[TM_T_QK], b.qkvg, rt, kQKVG, kQKVG, 64)) {
-        return e;
-    }
-    if (int e = encode_map(&L.tmap[TM_T_VT], b.vt, size_t(t.S) * kTokC, size_t(t.np), size_t(t.np), kHeadD)) {
-        return e;
+    for (int alt = 0; alt <= (p.flow ? 1 : 0); alt++) {
+        if (int e = encode_map(&L.tmap[TM_T_QK + alt], alt ? b.qkvg2 : b.qkvg, rt, kQKVG, kQKVG, 64)) {
+            return e;
+        }
+        if (int e = encode_map(&L.tmap[TM_T_VT + alt], alt ? b.vt2 : b.vt, size_t(t.S) * kTokC, size_t(t.np), size_t(t.np), kHeadD)) {
+            return e;
+        }
     }
     if (int e = encode_map(&L.tmap[TM_T_PLG], b.plg, size_t(t.nb) * kPairHeads * t.np, size_t(t.np), size_t(t.np), 128)) {
         return e;
@@ -577,7 +583,7 @@ static int make_launch(Launch& L, const Template& t, const Device& dev, const vo
         const void* base;
         size_t rows, cols;
     } omaps[] = {
-        {TM_O_QKVG, b.qkvg, rt, kQKVG}, {TM_O_AQG, b.aqg, ra, 2 * kAtomC}, {TM_O_AKV, b.akv, ra, 2 * kAtomC},
+        {TM_O_QKVG, b.qkvg, rt, kQKVG}, {TM_O_QKVG2, p.flow ? b.qkvg2 : b.qkvg, rt, kQKVG}, {TM_O_AQG, b.aqg, ra, 2 * kAtomC}, {TM_O_AKV, b.akv, ra, 2 * kAtomC},
         {TM_O_TC, b.tc, rt, kTokHidden}, {TM_O_ACA, b.aca, ra, kAtomHidden}, {TM_O_SCH, b.sch, size_t(N), 2 * cs},
         {TM_O_MODS, b.mods, nb * kTokModSlots * N, kTokC},
     };

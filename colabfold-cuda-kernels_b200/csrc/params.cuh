@@ -18,8 +18,8 @@ namespace cck {
     X(B_WQKVG) X(B_WO) X(B_W1) X(B_W2) X(B_WTB) X(B_WAGGR) X(B_PLW)                                \
     X(B_ENC_WQG) X(B_ENC_WKV) X(B_ENC_WO) X(B_ENC_W1) X(B_ENC_W2)                                  \
     X(B_DEC_WQG) X(B_DEC_WKV) X(B_DEC_WO) X(B_DEC_W1) X(B_DEC_W2)                                  \
-    X(T_QK) X(T_VT) X(T_PLG) X(T_TO)                                                                    \
-    X(O_QKVG) X(O_AQG) X(O_AKV) X(O_TC) X(O_ACA) X(O_SCH) X(O_MODS)
+    X(T_QK) X(T_QK2) X(T_VT) X(T_VT2) X(T_PLG) X(T_TO)                                                                    \
+    X(O_QKVG) X(O_QKVG2) X(O_AQG) X(O_AKV) X(O_TC) X(O_ACA) X(O_SCH) X(O_MODS)
 #define CCK_ENUM(name) TM_##name,
 enum TMap { CCK_TMAPS(CCK_ENUM) kNumTMaps };
 #undef CCK_ENUM
@@ -40,17 +40,18 @@ struct Geo {
 struct Bufs {
     float *pos, *xn, *out, *cen, *ntv, *sc, *se, *qa, *skip, *act, *tb, *upd, *agt, *grad, *kab;
     bf16 *sct, *scln0, *scbf, *sch, *mods, *ao, *abf, *aqg, *akv, *tx, *qkvg, *to, *tc, *plg;
-    bf16 *axq, *axk, *axhl, *aca, *vt, *tx2;
+    bf16 *axq, *axk, *axhl, *aca, *vt, *tx2, *qkvg2, *vt2;
 };
-// A token block runs without a grid barrier inside it: QKVG -> attention -> WO -> adaLN -> W1 -> W2,
-// and the adaLN rows of the next block (or the final LayerNorm) follow W2 in the same way; the one
-// barrier of a block stands between those rows and QKVG. A unit of a later operation waits for the
-// units it reads, counted per block of 128 token rows: every worker warp adds one when its part of a
-// unit has been stored (TX: every adaLN row of the transition's input adds one). The counters are
-// zeroed at the start of a launch and count on through it: a unit of the e-th token block of the
+// The token blocks run without grid barriers: adaLN -> QKVG -> attention -> WO -> adaLN -> W1 -> W2, and the adaLN
+// rows of the next block (or the final LayerNorm) follow W2 in the same way. A unit of a later operation
+// waits for the units it reads, counted per block of 128 token rows: every worker warp adds one when its part of a
+// unit has been stored (TX0, TX: every adaLN row of the attention's and of the transition's input adds one). The
+// counters are zeroed at the start of a launch and count on through it: a unit of the e-th token block of the
 // launch waits for (e + 1) times what one block adds.
-enum FlowCnt { FC_QKVG, FC_TO, FC_TC, FC_ACT1, FC_ACT2, FC_TX, kFlowCnts };
-
+// What a block writes while units of the block before may still be reading: only QKVG and VT, which the attention
+// items of a whole sample read. They alternate between two buffers: what the one of the block before last held
+// has been read when this block's rows exist, since every row went through that block's attention.
+enum FlowCnt { FC_QKVG, FC_TO, FC_TC, FC_ACT1, FC_ACT2, FC_TX, FC_TX0, kFlowCnts };
 // A counter has a 128-byte line of its own: many CTAs poll it while others add to it, and neighbours in one line
 // would share that traffic.
 constexpr int kFlowPitch = 32;
@@ -128,8 +129,9 @@ __host__ __device__ inline int gd_atom(int side, int which) {
 
 // ---- the phase program: the host writes the schedule as a list of operations, the kernel
 // interprets it. An operation runs one function over the grid; `end` says what follows it: nothing
-// (the next operation shares the phase), a sub-phase barrier of this implementation, or a barrier
-// that also counts as a phase of the reference's schedule (src/diffusion/sampler.cuh:99-230).
+// (the next operation shares the phase), a sub-phase barrier of this implementation, a barrier that also
+// counts as a phase of the reference's schedule (src/diffusion/sampler.cuh:99-230), or an arrival at the
+// barrier that nobody waits for (the next full barrier counts it).
 enum Fn : unsigned char {
     FN_GEMM,          // a0: descriptor, b
     FN_POS_INIT, FN_PAIR_PADS, FN_POS_CENTRE, FN_POS_AUGMENT, FN_POS_UPDATE, FN_POS_OUT_ONCE, FN_POS_OUTPUT,
@@ -152,7 +154,7 @@ enum Fn : unsigned char {
     FN_RET,
     FN_END,
 };
-enum OpEnd : unsigned char { END_NONE, END_SUB, END_PHASE };
+enum OpEnd : unsigned char { END_NONE, END_SUB, END_PHASE, END_ARRIVE };
 constexpr unsigned char kLoopB = 255; // b comes from the token-block loop
 struct Op {
     unsigned char fn, a0, b, end_kind; // end_kind: OpEnd in the low two bits, the phase kind above them
@@ -179,10 +181,10 @@ enum Epi : int {
     EPI_PAIR,  // token pair logits into PLG
 };
 
-// nfast: tile t is (row tile t / nt, column tile t % nt) instead of (t % mt, t / mt); sig: 1 + the
+// alt: the output alternates between two buffers from token block to token block; nfast: tile t is (row tile t / nt, column tile t % nt) instead of (t % mt, t / mt); sig: 1 + the
 // completion counters (FlowCnt) that finished tiles are reported to; dep: 1 + the completion
 // counters that a tile's rows of A wait for (0: none)
-enum GdFlag { GF_NFAST = 1, GF_SIG_SHIFT = 4, GF_DEP_SHIFT = 8, GF_CNT_MASK = 15 };
+enum GdFlag { GF_NFAST = 1, GF_ALT = 2, GF_SIG_SHIFT = 4, GF_DEP_SHIFT = 8, GF_CNT_MASK = 15 };
 struct GemmDesc {
     int map_a, map_b; // tensor maps
     int map_o;        // the output's store map, or -1: plain stores

@@ -284,16 +284,14 @@ __device__ CCK_HOT_FN void token_adaln(const KP& p, Deal& d, int b, int slot, un
     if (p.flow) {
         // the attention's input follows W2 of the block before, the transition's input WO of this block
         FlowRows f = flow_rows(p, rows, slot == TM_ATTN_SCALE ? FC_ACT2 : FC_ACT1, epoch + (slot != TM_ATTN_SCALE));
-        unsigned int* tx_done = flow_cnt(p, FC_TX);
+        unsigned int* tx_done = flow_cnt(p, slot == TM_ATTN_SCALE ? FC_TX0 : FC_TX);
         for (int r = f.r0; r < f.r1; r += kWarps) {
             AdaRow a0;
             adaln_load_mods(a0, p, ms, mo, r); // (nothing to wait for: they travel while the counter is awaited)
             flow_row_wait(f, r);
             a0.x = load_f32_cg<6>(p.buf.act + size_t(r) * kTokC);
             adaln_finish(a0, p, r);
-            if (slot != TM_ATTN_SCALE) { // W1's tiles over the row's block of 128 wait for its rows
-                flow_signal(tx_done, r / kBM, r / kBM);
-            }
+            flow_signal(tx_done, r / kBM, r / kBM); // the tiles of QKVG or W1 over the row's block of 128 wait for its rows
         }
         return;
     }

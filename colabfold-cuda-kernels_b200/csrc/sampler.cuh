@@ -233,8 +233,8 @@ __device__ inline GemmDesc gemm_tok(const KP& p, int b, int which) {
     }
     if (p.flow) { // blocks of 128 rows complete in order, and the units that read them start early
         const int sig = 1 + (which == TG_QKVG ? FC_QKVG : which == TG_WO ? FC_ACT1 : which == TG_W1 ? FC_TC : FC_ACT2);
-        const int dep = which == TG_WO ? 1 + FC_TO : which == TG_W1 ? 1 + FC_TX : which == TG_W2 ? 1 + FC_TC : 0;
-        g.fl = GF_NFAST | sig << GF_SIG_SHIFT | dep << GF_DEP_SHIFT;
+        const int dep = 1 + (which == TG_QKVG ? FC_TX0 : which == TG_WO ? FC_TO : which == TG_W1 ? FC_TX : FC_TC);
+        g.fl = GF_NFAST | (which == TG_QKVG ? GF_ALT : 0) | sig << GF_SIG_SHIFT | dep << GF_DEP_SHIFT;
     }
     return g;
 }
@@ -329,6 +329,9 @@ __device__ CCK_PHASE_FN void pair_fill_pads(const KP& p, Deal& d) {
         const size_t v = size_t(p.S) * kTokC * pad;
         for (size_t i = tid; i < v; i += nth) {
             p.buf.vt[(i / pad) * p.npb + p.N + i % pad] = 0;
+            if (p.flow) {
+                p.buf.vt2[(i / pad) * p.npb + p.N + i % pad] = 0;
+            }
         }
         const size_t tables = size_t(p.nb) * kPairHeads, m = tables * pad * p.np;
         for (size_t i = tid; i < m; i += nth) {
@@ -342,9 +345,11 @@ __device__ CCK_PHASE_FN void pair_fill_pads(const KP& p, Deal& d) {
         }
     }
     const size_t row0 = size_t(p.S) * p.N, row1 = min(size_t(p.S) * p.Nb, row0 + kTcKeys);
-    uint4* z = reinterpret_cast<uint4*>(p.buf.qkvg + row0 * kQKVG);
-    for (size_t i = tid; i < (row1 - row0) * kQKVG / 8; i += nth) {
-        z[i] = make_uint4(0, 0, 0, 0);
+    for (int alt = 0; alt <= (p.flow ? 1 : 0); alt++) {
+        uint4* z = reinterpret_cast<uint4*>((alt ? p.buf.qkvg2 : p.buf.qkvg) + row0 * kQKVG);
+        for (size_t i = tid; i < (row1 - row0) * kQKVG / 8; i += nth) {
+            z[i] = make_uint4(0, 0, 0, 0);
+        }
     }
     (void)d;
 }
@@ -363,7 +368,7 @@ __device__ __forceinline__ void run_gemm(const Launch& L, Run& r, Deal& d, int i
         gemm_issue(r.pipe, g, tb, tiles, ts);
     } else if (warp < kAuxWarp0) {
         const uint32_t tile = r.pipe.tile;
-        const CUtensorMap* mo = g.map_o >= 0 ? &L.tmap[g.map_o] : nullptr;
+        const CUtensorMap* mo = g.map_o >= 0 ? &L.tmap[g.map_o + ((g.fl & GF_ALT) ? epoch & 1 : 0)] : nullptr;
         switch (g.epi) {
         case EPI_BF16:
             worker_tiles<EPI_BF16>(g, mo, b, tile, tb, tiles, ts, epoch);
@@ -562,7 +567,13 @@ extern "C" __global__ void __launch_bounds__(cck::kThreads, 1) cck_sampler_kerne
             CCK_TRACE_ONE(6, 0x82, op.fn);
         }
         r.pc++;
-        if ((op.end_kind & 3) != END_NONE && grid_barrier(L, op.end_kind)) {
+        if ((op.end_kind & 3) == END_ARRIVE) {
+            // this CTA's part is done; whoever has to know more waits for completion counters
+            if (threadIdx.x == 0) {
+                atomicAdd(&kp().ctl->barrier, 1u);
+            }
+            r.syncs++;
+        } else if ((op.end_kind & 3) != END_NONE && grid_barrier(L, op.end_kind)) {
             break;
         }
     }
