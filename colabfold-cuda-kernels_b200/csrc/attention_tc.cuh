@@ -9,8 +9,7 @@
 //                        columns of QKVG of which 48 are used); per chunk of 64 keys the K tile and the
 //                        transposed V tile from VT into a 3-deep ring (a chunk's tiles are asked for one
 //                        chunk ahead and stay until its P·V is done), and the 128 x 64 tile of pair
-//                        logits into a 2-deep ring of its own, released as soon as the softmax threads
-//                        have read it
+//                        logits into a 2-deep ring of its own, released with the P that came of it
 //   warps 1 and 11   tcgen05.mma of track 0 and of track 1. One wait per chunk: once
 //                        the group's P of chunk g is complete, O += P·V of chunk g (128 x 48, K = 64,
 //                        P read from TMEM) and S = Q·Kᵀ of chunk g + 2 (128 x 64, K = 48) into the S
@@ -42,7 +41,7 @@ constexpr int kTcRows = kTcWarps * 32;            // query rows per item = softm
 static_assert(kTcRows == kBM, "one softmax thread per row of a 128-row UMMA");
 static_assert(kTcWarps == kAttnItemWarps, "the completion counters of TO count the warps of an item");
 constexpr int kTcTmaWarp1 = kAuxWarp0, kTcMmaWarp1 = kAuxWarp0 + 1; // the second track's TMA and MMA threads
-constexpr int kTcKvStages = 3, kTcBiasStages = 2;
+constexpr int kTcKvStages = 3, kTcBiasStages = 2; // (pair logits: one slot per chunk parity, as S and P)
 // The exponentials' reference value trails the running maximum by up to 2^8: an exponential above that makes its
 // chunk's sum exceed it too.
 constexpr float kTcLazySum = 256.f;
@@ -70,8 +69,7 @@ static_assert(kTcTracks * kTcTrackCols <= kTmemCols, "two tracks share the CTA's
 struct TcTrackBars {
     uint64_t q_full, q_empty;                             // TMA -> MMA; MMA (every Q·Kᵀ of the item done) -> TMA
     uint64_t kv_full[kTcKvStages], kv_empty[kTcKvStages]; // TMA -> MMA; MMA (P·V of the chunk done) -> TMA
-    uint64_t b_full[kTcBiasStages], b_empty[kTcBiasStages]; // TMA -> softmax; softmax (tile read) -> TMA
-    uint64_t s_full[2], p_full[2];                        // MMA -> softmax; softmax (P stored, O rescaled) -> MMA
+    uint64_t s_full[2], p_full[2];                        // MMA (S) and TMA (pair logits) -> softmax; softmax (P stored, O rescaled, pair logits read) -> MMA, TMA
     uint64_t pv_done[2];                                  // MMA (P·V of the chunk done: O is current, for a rescale)
     uint64_t o_full;                                      // MMA (the item's last P·V done) -> softmax
 };
@@ -95,11 +93,8 @@ __device__ inline void attn_tc_init() {
             for (int i = 0; i < kTcKvStages; i++) {
                 mbar_init(&tb.kv_full[i], 1), mbar_init(&tb.kv_empty[i], 1);
             }
-            for (int i = 0; i < kTcBiasStages; i++) {
-                mbar_init(&tb.b_full[i], 1), mbar_init(&tb.b_empty[i], kTcRows);
-            }
             for (int i = 0; i < 2; i++) {
-                mbar_init(&tb.s_full[i], 1), mbar_init(&tb.p_full[i], kTcRows), mbar_init(&tb.pv_done[i], 1);
+                mbar_init(&tb.s_full[i], 2), mbar_init(&tb.p_full[i], kTcRows), mbar_init(&tb.pv_done[i], 1);
             }
             mbar_init(&tb.o_full, 1);
             b->items[t] = 0, b->chunks[t] = 0;
@@ -242,8 +237,9 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                 }
             };
             auto load_bias = [&](int c, uint32_t g) {
-                const uint32_t st = g % kTcBiasStages, par = (g / kTcBiasStages) & 1, bb = bar(B.b_full[0]) + 8 * st;
-                mbar_wait(&B.b_empty[st], par ^ 1, &ctl->abort);
+                // (the slot's last reader is through when P of the chunk two before is there)
+                const uint32_t st = g & 1, bb = bar(B.s_full[0]) + 8 * st;
+                mbar_wait(&B.p_full[st], ((g >> 1) & 1) ^ 1, &ctl->abort);
                 mbar_expect_tx_el(el, bb, kTcBiasBytes);
                 tma_load_2d_hint_el(el, base + kTcBiasOff + st * kTcBiasBytes, mpl, c * kTcKeys, brow, bb, policy);
             };
@@ -390,9 +386,9 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
             float m = 0.f, l = 0.f; // the reference value of the row's exponentials, the row sum against it
 #pragma unroll 1
             for (int c = 0; c < chunks; c++, g++) {
-                const uint32_t bi = g & 1, bpar = (g >> 1) & 1, bst = g % kTcBiasStages;
+                const uint32_t bi = g & 1, bpar = (g >> 1) & 1;
                 CCK_TRACE_EV(0x30 + t, g - g0);
-                mbar_wait(&B.s_full[bi], bpar, &ctl->abort);
+                mbar_wait(&B.s_full[bi], bpar, &ctl->abort); // the scores and the pair logits (one wait: one that passes costs 90 cycles)
                 tc_fence_after();
                 CCK_TRACE_EV(0x32 + t, g - g0);
                 if (c == 0) {
@@ -411,8 +407,7 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                     }
                     cp_async_commit();
                 }
-                mbar_wait(&B.b_full[bst], (g / kTcBiasStages) & 1, &ctl->abort);
-                const char* brow = base + kTcBiasOff + bst * kTcBiasBytes + row_in * 128; // the row's 64 pair logits: 8 swizzled 16-byte pieces
+                const char* brow = base + kTcBiasOff + bi * kTcBiasBytes + row_in * 128; // the row's 64 pair logits: 8 swizzled 16-byte pieces
                 // One pass over the chunk: exponentials of the scores (base 2, pair logits added) against the
                 // reference value m, P = 2^(score - m) as bf16 to TMEM (16 keys are 8 columns), and their sum. A
                 // warp issues an instruction every two cycles or so, and eight warps of softmax are what
@@ -502,11 +497,10 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                     }
                 }
                 l += chunk_l;
-                // The tile of pair logits has been used: its slot may be refilled. The refill is a TMA write (async
+                CCK_TRACE_EV(0x34 + t, g - g0);
+                // The tile of pair logits has been used, too: its slot may be refilled. The refill is a TMA write (async
                 // proxy) over what this thread has read with ordinary loads: the proxy fence orders the two.
                 fence_async_smem();
-                mbar_arrive(&B.b_empty[bst]);
-                CCK_TRACE_EV(0x34 + t, g - g0);
                 tmem_st_wait();
                 tc_fence_before();
                 mbar_arrive(&B.p_full[bi]);
