@@ -398,9 +398,7 @@ static void write_denoise(ProgramWriter& w, uint32_t flags) {
         w.op(FN_CTA_SYNC);
         w.gemm(GD_TOK_WO, kLoopB);
         w.op(FN_TOK_ADALN, TM_TRANS_SCALE, kLoopB); // its rows wait for WO's tiles over them
-        // (WO's epilogue keeps the residual rows it fetched ahead in the upper halves of the ring's
-        // weight slots, which W1's 256-column tiles fill: every warp of the CTA is through with WO first)
-        w.op(FN_CTA_SYNC);
+        w.op(FN_CTA_SYNC, 1); // (nothing is restaged here: the roles go on into W1 as each is through)
         w.gemm(GD_TOK_W1, kLoopB); // a tile waits for the adaLN rows of its block of 128
         w.gemm(GD_TOK_W2, kLoopB); // the next block's adaLN rows (or the final LayerNorm's) wait for its tiles
     } else {

@@ -147,7 +147,7 @@ enum Fn : unsigned char {
     FN_TOK_ATTN, FN_TOK_FINAL_LN, FN_DEC_INIT,
     FN_TOK_QKNORM,    // QKNORM: b
     FN_ATOM_QKNORM,   // QKNORM: a0: side, b
-    FN_CTA_SYNC,      // the GEMM roles rejoin before the CTA restages shared memory
+    FN_CTA_SYNC,      // a0 = 0: the GEMM roles rejoin before the CTA restages shared memory; 1: a place where they need not
     FN_BLOCK_NEXT,    // next token block: jump to operation a0 while blocks remain
     FN_STEP_NEXT,     // next sampling step: jump to operation a0 while steps remain
     FN_CALL,          // the denoiser subroutine at operation a0; b = 1: at σ instead of t̂ (Heun's second call)

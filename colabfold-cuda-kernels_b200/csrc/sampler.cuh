@@ -498,7 +498,9 @@ __device__ __forceinline__ void run_op(const Launch& L, Run& r, const Op op) {
         atom_qknorm(p, d, op.a0 ? p.dec : p.enc, b);
         break;
     default: // FN_CTA_SYNC
-        __syncthreads();
+        if (op.a0 == 0) {
+            __syncthreads();
+        }
     }
     if (op.fn != FN_GEMM && op.fn != FN_CTA_SYNC) {
         fence_async_smem(); // what this thread did in the scratch area, before TMA loads fill the ring there
