@@ -261,8 +261,11 @@ struct FlowRows {
 };
 __device__ __forceinline__ FlowRows flow_rows(const KP& p, int rows, int which, unsigned int gemms_done) {
     FlowRows f;
-    const int per = cdiv(rows, int(gridDim.x));
-    f.r0 = min(rows, int(blockIdx.x) * per) + warp_id(), f.r1 = min(rows, (int(blockIdx.x) + 1) * per), f.ok = -1;
+    // Where a warp has a row or two, the first go to the two warps without a role in the GEMMs, which are there first;
+    // the roles' own warps get on with the next operation (390-1900 rows: 1.5%). With three rows and more to a warp,
+    // 1024 x 5, that order took 2% longer.
+    const int per = cdiv(rows, int(gridDim.x)), rank = per <= 2 * kWarps ? (warp_id() + kWarps - kAuxWarp0) % kWarps : warp_id();
+    f.r0 = min(rows, int(blockIdx.x) * per) + rank, f.r1 = min(rows, (int(blockIdx.x) + 1) * per), f.ok = -1;
     f.cnt = flow_cnt(p, which);
     f.target = gemms_done * (unsigned int)(gd_table()[which == FC_ACT1 ? GD_TOK_WO : GD_TOK_W2].nt * kWorkWarps);
     return f;
