@@ -236,12 +236,12 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                     kst = 0, kpar ^= 1;
                 }
             };
-            auto load_bias = [&](int c, uint32_t g) {
+            auto load_bias = [&](int c, int row, uint32_t g) {
                 // (the slot's last reader is through when P of the chunk two before is there)
                 const uint32_t st = g & 1, bb = bar(B.s_full[0]) + 8 * st;
                 mbar_wait(&B.p_full[st], ((g >> 1) & 1) ^ 1, &ctl->abort);
                 mbar_expect_tx_el(el, bb, kTcBiasBytes);
-                tma_load_2d_hint_el(el, base + kTcBiasOff + st * kTcBiasBytes, mpl, c * kTcKeys, brow, bb, policy);
+                tma_load_2d_hint_el(el, base + kTcBiasOff + st * kTcBiasBytes, mpl, c * kTcKeys, row, bb, policy);
             };
             if (t == 1 && p.attn_skew > 0) { // a test's skew between the pipelines: results must not depend on it
                 const long long t0 = clock64();
@@ -249,24 +249,29 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                 }
                 __syncwarp();
             }
-            set_item(0);
-            load_kv(0);
-            load_q(j0);
-            uint32_t g = g0;
+            // (one loop over all chunks, so that each of the loads above is there once: this function's loops share an
+            // instruction cache, and eight warps of softmax want most of it)
+            const int total = n * nchunks;
+            int j = 0, c = 0, bias_c = 0, bias_row = 0;
 #pragma unroll 1
-            for (int j = 0; j < n; j++) {
-#pragma unroll 1
-                for (int c = 0; c < nchunks; c++, g++) {
-                    load_bias(c, g);
-                    CCK_TRACE_EV(0x10 + t, g - g0);
-                    if (c + 1 < nchunks) {
-                        load_kv(c + 1);
-                        CCK_TRACE_EV(0x12 + t, g + 1 - g0);
-                    } else if (j + 1 < n) {
-                        set_item(j + 1);
-                        load_kv(0);
-                        load_q(j0 + j + 1);
+            for (int i = 0; i <= total; i++) {
+                if (i > 0) {
+                    load_bias(bias_c, bias_row, g0 + uint32_t(i - 1));
+                    CCK_TRACE_EV(0x10 + t, i - 1);
+                }
+                if (i < total) {
+                    if (c == 0) {
+                        set_item(j);
                     }
+                    load_kv(c);
+                    CCK_TRACE_EV(0x12 + t, i);
+                    if (c == 0) {
+                        load_q(j0 + uint32_t(j));
+                    }
+                }
+                bias_c = c, bias_row = brow;
+                if (++c == nchunks) {
+                    c = 0, j++;
                 }
             }
             CCK_TRACE_END();
@@ -324,30 +329,26 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                 }
             };
             tc_fence_after();
-            uint32_t g = g0, st = g0 % kTcKvStages;
-            int i = 0;
+            uint32_t st = g0 % kTcKvStages;
+            int j = 0, c = 0;
             CCK_TRACE_BEGIN_IF(2 + t, el);
 #pragma unroll 1
-            for (int j = 0; j < n; j++) {
+            for (int i = 0; i < total; i++) {
                 pump(i + 2, j);
-#pragma unroll 1
-                for (int c = 0; c < nchunks; c++, g++, i++) {
-                    const uint32_t bi = g & 1;
-                    mbar_wait(&B.p_full[bi], (g >> 1) & 1, &ctl->abort);
-                    tc_fence_after();
-                    CCK_TRACE_EV(0x20 + t, i);
-                    umma_bf16_ts_k64_el(el, tt + kTcO, tt + kTcP + bi * 32, dk0 + st * kStageStep + kVStep, idesc_o, c);
-                    umma_commit_el(el, bar(B.pv_done[0]) + 8 * bi);
-                    umma_commit_el(el, bar(B.kv_empty[0]) + 8 * st);
-                    CCK_TRACE_EV(0x22 + t, i);
-                    if (c + 1 == nchunks) {
-                        umma_commit_el(el, bar(B.o_full)); // the item's O is complete
-                    }
-                    pump(i + 3, j);
-                    CCK_TRACE_EV(0x24 + t, i);
-                    if (++st == kTcKvStages) {
-                        st = 0;
-                    }
+                const uint32_t g = g0 + uint32_t(i), bi = g & 1;
+                mbar_wait(&B.p_full[bi], (g >> 1) & 1, &ctl->abort);
+                tc_fence_after();
+                CCK_TRACE_EV(0x20 + t, i);
+                umma_bf16_ts_k64_el(el, tt + kTcO, tt + kTcP + bi * 32, dk0 + st * kStageStep + kVStep, idesc_o, c);
+                umma_commit_el(el, bar(B.pv_done[0]) + 8 * bi);
+                umma_commit_el(el, bar(B.kv_empty[0]) + 8 * st);
+                CCK_TRACE_EV(0x22 + t, i);
+                if (++st == kTcKvStages) {
+                    st = 0;
+                }
+                if (++c == nchunks) {
+                    umma_commit_el(el, bar(B.o_full)); // the item's O is complete
+                    c = 0, j++;
                 }
             }
             CCK_TRACE_END();
