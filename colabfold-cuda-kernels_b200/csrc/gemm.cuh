@@ -593,7 +593,7 @@ constexpr int kMaxGd = kGdBytes / int(sizeof(GemmDesc));
 
 // ---- completion counters between operations of one phase (FlowCnt)
 __device__ __forceinline__ unsigned int* flow_cnt(const KP& p, int which) {
-    return p.flow_cnt + which * p.flow_n * kFlowPitch;
+    return p.flow_cnt + (which < kFlowTok ? which * p.flow_n : kFlowTok * p.flow_n + (which - kFlowTok) * p.flow_na) * kFlowPitch;
 }
 // The calling warp's part of a unit is stored: its lanes' writes (and lane 0's TMA stores, which the
 // caller has waited for) are published with one release add per counter in [c0, c1].
@@ -666,14 +666,14 @@ __device__ __forceinline__ bool flow_wait(const unsigned int* cnt, int c0, int c
 }
 // Arrivals that complete row block rb of a GEMM's A (descriptor g, depc set) in one token block. TO:
 // the attention items of every block of 128 queries (per sample of g.period rows) that the rows
-// touch, 16 heads x 4 warps each. TC: the column tiles of W1 over these rows, 8 warps each. TX, TX0: the
-// adaLN rows of the block.
-__device__ __forceinline__ unsigned int flow_target(const GemmDesc& g, int which, int rb, int w1_tiles) {
-    if (which == FC_TX || which == FC_TX0) {
+// touch, 16 heads x 4 warps each. TC: the column tiles of W1 over these rows, 8 warps each. ACA: the same of the atoms. TX,
+// TX0, AX, AXT: the rows of the block.
+__device__ __forceinline__ unsigned int flow_target(const GemmDesc& g, int which, int rb) {
+    if (which == FC_TX || which == FC_TX0 || which == FC_AX || which == FC_AXT) {
         return (unsigned int)(min(kBM, g.m - rb * kBM));
     }
     if (which != FC_TO) {
-        return (unsigned int)(w1_tiles * kWorkWarps);
+        return (unsigned int)(gd_table()[which == FC_TC ? GD_TOK_W1 : GD_ENC_W1].nt * kWorkWarps);
     }
     const int lo = rb * kBM, hi = min(lo + kBM, g.m) - 1, qblocks = cdiv(g.period, kBM);
     const int ilo = lo / g.period * qblocks + lo % g.period / kBM, ihi = hi / g.period * qblocks + hi % g.period / kBM;
@@ -705,8 +705,8 @@ template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, con
             // the attention's adaLN rows have waited for; WO for W2, which came before W1's tiles.
             if (const int depc = gd.fl >> GF_DEP_SHIFT & GF_CNT_MASK) {
                 if (lane_id() == 0) {
-                    const int which = depc == 1 + FC_TO ? FC_TX0 : FC_TC, rb = row0 / kBM;
-                    flow_wait(flow_cnt(kp(), which), rb, rb, (epoch + 1) * flow_target(gd, which, rb, gd_table()[GD_TOK_W1].nt), &ctl->abort);
+                    const int which = depc == 1 + FC_TO ? FC_TX0 : depc - 1, rb = row0 / kBM;
+                    flow_wait(flow_cnt(kp(), which), rb, rb, (epoch + 1) * flow_target(gd, which, rb), &ctl->abort);
                 }
                 __syncwarp();
             }
@@ -845,7 +845,7 @@ __device__ CCK_PHASE_FN void gemm_produce(const Launch& L, Pipe& pipe, const Gem
                 int row0, col0;
                 tile_coords(gd, t, row0, col0);
                 const int rb = row0 / kBM;
-                FlowWait w(flow_cnt(kp(), depc - 1) + rb * kFlowPitch, (epoch + 1) * flow_target(gd, depc - 1, rb, gd_table()[GD_TOK_W1].nt), &ctl->abort);
+                FlowWait w(flow_cnt(kp(), depc - 1) + rb * kFlowPitch, (epoch + 1) * flow_target(gd, depc - 1, rb), &ctl->abort);
                 const int most = min(kblocks, slots);
                 int f = s + have < slots ? s + have : s + have - slots; // the slot of k-block `have`
                 while (!uni(int(w.ready()))) {

@@ -61,7 +61,7 @@ inline bool flow_allowed(uint32_t flags) {
 struct Template {
     int S, Nb, NSb, nsteps;
     uint32_t flags;
-    int steps, cs, nb, tw1, aw1, nk, plc, plx, np, flow_n;
+    int steps, cs, nb, tw1, aw1, nk, plc, plx, np, flow_n, flow_na;
     size_t off[kNumBufs], bytes[kNumBufs];
     size_t total;
 };
@@ -176,7 +176,8 @@ static int make_template(Template& t, int S, int Nb, int NSb, int nsteps, uint32
     want[B_AGT] = ra * kTokC * f;
     want[B_VT] = size_t(S) * kTokC * t.np * h;
     t.flow_n = int(cdiv(int(rt), kBM)) + 1;
-    want[B_FLOW] = size_t(kFlowCnts) * t.flow_n * kFlowPitch * sizeof(unsigned int);
+    t.flow_na = int(cdiv(int(ra), kBM));
+    want[B_FLOW] = (size_t(kFlowTok) * t.flow_n + size_t(kFlowAtom) * t.flow_na) * kFlowPitch * sizeof(unsigned int);
     if (flow_allowed(flags)) { // the second buffers of the token blocks' chains
         want[B_QKVG2] = want[B_QKVG], want[B_VT2] = want[B_VT];
     }
@@ -328,54 +329,94 @@ struct ProgramWriter {
 // operations chained by completion counters (FlowCnt) instead of barriers. Not with PARALLEL or QKNORM, whose blocks have other phases; not in a debug run that
 // stops at a phase of the reference's schedule, which counts the barriers.
 constexpr uint32_t kProgFlow = 1u << 30;
+// the pieces of an atom block on completion counters (side 0 encoder, 1 decoder)
+static void write_atom_projections(ProgramWriter& w, int side, int b) {
+    w.op(FN_ATOM_LN_QK, side, b, END_ARRIVE);
+    w.gemm(gd_atom(side, AG_QG), b), w.gemm(gd_atom(side, AG_KV), b);
+}
+static void write_atom_transition(ProgramWriter& w, int side, int b) {
+    w.gemm(gd_atom(side, AG_WO), b, END_ARRIVE);
+    w.op(FN_ATOM_LN_T, side, b, END_ARRIVE);
+    w.gemm(gd_atom(side, AG_W1), b, END_ARRIVE);
+    w.gemm(gd_atom(side, AG_W2), b, END_ARRIVE);
+}
 static void write_denoise(ProgramWriter& w, uint32_t flags) {
     const bool qkn = flags & F_QKNORM, par = flags & F_PARALLEL;
     const bool flow = (flags & kProgFlow) && flow_allowed(flags);
-    // conditioning + atom encoder + aggregation
-    w.op(FN_NOISE_INIT, 0, 0, END_PHASE, K_INIT);
-    for (int b = 0; b < kAtomBlocks; b++) {
-        if (b < 2) {
-            w.op(FN_SC_LN, b);
-        } else {
-            w.op(FN_SC_PREP);
+    if (flow) {
+        // Atom encoder: one phase from an attention's output to the next projections. The conditioning, one operation
+        // per phase, rides along.
+        w.op(FN_NOISE_INIT, 0, 0, END_PHASE, K_INIT);
+        w.op(FN_SC_LN, 0);
+        write_atom_projections(w, 0, 0);
+        w.op(FN_CTA_SYNC, 1, 0, END_PHASE, K_A_PROJ);
+        for (int b = 0; b < kAtomBlocks; b++) {
+            if (b == 0) {
+                w.gemm(GD_ST_W1_0);
+            } else if (b == 1) {
+                w.op(FN_SC_LN, 1);
+            } else {
+                w.gemm(GD_ST_W2_1);
+            }
+            w.op(FN_CTA_SYNC);
+            w.op(FN_ATOM_ATTN, 0, b, END_PHASE, K_A_ATTN);
+            write_atom_transition(w, 0, b);
+            if (b + 1 < kAtomBlocks) {
+                write_atom_projections(w, 0, b + 1);
+                w.gemm(b == 0 ? GD_ST_W2_0 : GD_ST_W1_1, 0, END_PHASE, K_A_W2);
+            } else {
+                w.op(FN_ATOM_TAIL_SKIP);
+                w.op(FN_SC_PREP, 0, 0, END_PHASE, K_A_W2);
+            }
         }
-        if (par) { // the transition's input comes from the block input too: both adaLN passes first
-            w.op(FN_ATOM_LN_QK, 0, b);
-            w.op(FN_ATOM_LN_T, 0, b, END_SUB, K_A_LN);
-        } else {
-            w.op(FN_ATOM_LN_QK, 0, b, END_SUB, K_A_LN);
+        w.gemm(GD_AGGR), w.gemm(GD_MODS_0), w.gemm(GD_MODS_1), w.gemm(GD_EMBED, 0, END_SUB, K_AGG_GEMM);
+    } else {
+        // conditioning + atom encoder + aggregation
+        w.op(FN_NOISE_INIT, 0, 0, END_PHASE, K_INIT);
+        for (int b = 0; b < kAtomBlocks; b++) {
+            if (b < 2) {
+                w.op(FN_SC_LN, b);
+            } else {
+                w.op(FN_SC_PREP);
+            }
+            if (par) { // the transition's input comes from the block input too: both adaLN passes first
+                w.op(FN_ATOM_LN_QK, 0, b);
+                w.op(FN_ATOM_LN_T, 0, b, END_SUB, K_A_LN);
+            } else {
+                w.op(FN_ATOM_LN_QK, 0, b, END_SUB, K_A_LN);
+            }
+            w.gemm(gd_atom(0, AG_QG), b);
+            if (qkn) { // LayerNorm of the q and k just written, before the phase ends
+                w.gemm(gd_atom(0, AG_KV), b, END_SUB, K_A_PROJ);
+                w.op(FN_ATOM_QKNORM, 0, b, END_PHASE, K_QKN);
+            } else {
+                w.gemm(gd_atom(0, AG_KV), b, END_PHASE, K_A_PROJ);
+            }
+            // the conditioning's GEMMs ride in the attention phase
+            if (b < 2) {
+                w.gemm(GD_ST_W1_0 + b);
+            } else {
+                w.gemm(GD_MODS_0), w.gemm(GD_MODS_1), w.gemm(GD_EMBED);
+            }
+            w.op(FN_CTA_SYNC);
+            w.op(FN_ATOM_ATTN, 0, b, END_PHASE, K_A_ATTN);
+            if (b < 2) {
+                w.gemm(GD_ST_W2_0 + b);
+            }
+            w.gemm(gd_atom(0, AG_WO), b, END_SUB, K_A_WO);
+            if (!par) {
+                w.op(FN_ATOM_LN_T, 0, b, END_SUB, K_A_LNT);
+            }
+            w.gemm(gd_atom(0, AG_W1), b, END_SUB, K_A_W1);
+            if (b + 1 < kAtomBlocks) {
+                w.gemm(gd_atom(0, AG_W2), b, END_PHASE, K_A_W2);
+            } else {
+                w.gemm(gd_atom(0, AG_W2), b, END_SUB, K_A_W2);
+                w.op(FN_ATOM_TAIL_SKIP, 0, 0, END_PHASE, K_A_TAIL);
+            }
         }
-        w.gemm(gd_atom(0, AG_QG), b);
-        if (qkn) { // LayerNorm of the q and k just written, before the phase ends
-            w.gemm(gd_atom(0, AG_KV), b, END_SUB, K_A_PROJ);
-            w.op(FN_ATOM_QKNORM, 0, b, END_PHASE, K_QKN);
-        } else {
-            w.gemm(gd_atom(0, AG_KV), b, END_PHASE, K_A_PROJ);
-        }
-        // the conditioning's GEMMs ride in the attention phase
-        if (b < 2) {
-            w.gemm(GD_ST_W1_0 + b);
-        } else {
-            w.gemm(GD_MODS_0), w.gemm(GD_MODS_1), w.gemm(GD_EMBED);
-        }
-        w.op(FN_CTA_SYNC);
-        w.op(FN_ATOM_ATTN, 0, b, END_PHASE, K_A_ATTN);
-        if (b < 2) {
-            w.gemm(GD_ST_W2_0 + b);
-        }
-        w.gemm(gd_atom(0, AG_WO), b, END_SUB, K_A_WO);
-        if (!par) {
-            w.op(FN_ATOM_LN_T, 0, b, END_SUB, K_A_LNT);
-        }
-        w.gemm(gd_atom(0, AG_W1), b, END_SUB, K_A_W1);
-        if (b + 1 < kAtomBlocks) {
-            w.gemm(gd_atom(0, AG_W2), b, END_PHASE, K_A_W2);
-        } else {
-            w.gemm(gd_atom(0, AG_W2), b, END_SUB, K_A_W2);
-            w.op(FN_ATOM_TAIL_SKIP, 0, 0, END_PHASE, K_A_TAIL);
-        }
+        w.gemm(GD_AGGR, 0, END_SUB, K_AGG_GEMM);
     }
-    w.gemm(GD_AGGR, 0, END_SUB, K_AGG_GEMM);
     w.op(FN_AGGR_GATHER, 0, 0, END_PHASE, K_AGG_GATHER);
     // the token blocks (reference: src/diffusion/sampler.cuh:99-134)
     const int block0 = w.n;
@@ -418,6 +459,21 @@ static void write_denoise(ProgramWriter& w, uint32_t flags) {
     w.op(FN_TOK_FINAL_LN, 0, 0, END_PHASE, K_T_OUT);
     w.gemm(GD_BROADCAST, 0, END_PHASE, K_T_OUT);
     w.op(FN_DEC_INIT, 0, 0, END_PHASE, K_DEC_GLUE);
+    if (flow) {
+        write_atom_projections(w, 1, 0);
+        w.op(FN_CTA_SYNC, 1, 0, END_PHASE, K_A_PROJ);
+        for (int b = 0; b < kAtomBlocks; b++) {
+            w.op(FN_ATOM_ATTN, 1, b, END_PHASE, K_D_ATTN);
+            write_atom_transition(w, 1, b);
+            if (b + 1 < kAtomBlocks) {
+                write_atom_projections(w, 1, b + 1);
+                w.op(FN_CTA_SYNC, 1, 0, END_PHASE, K_A_W2);
+            } else {
+                w.op(FN_ATOM_TAIL_UPDATE, 0, 0, END_PHASE, K_A_W2);
+            }
+        }
+        return;
+    }
     for (int b = 0; b < kAtomBlocks; b++) {
         if (par) { // the transition's input comes from the block input too: both adaLN passes first
             w.op(FN_ATOM_LN_QK, 1, b);
@@ -508,7 +564,7 @@ static int make_launch(Launch& L, const Template& t, const Device& dev, const vo
     p.cs = t.cs, p.nb = t.nb, p.tw1 = t.tw1, p.aw1 = t.aw1, p.nk = t.nk, p.plc = t.plc, p.plx = t.plx;
     p.ln_eps = t.flags & F_IDSCALE ? kIdScaleEps : kLnEps;
     p.flags = t.flags, p.ext = ext, p.out = out, p.out_tokens = t.Nb;
-    p.flow = g_flow && flow_allowed(t.flags), p.flow_n = t.flow_n;
+    p.flow = g_flow && flow_allowed(t.flags), p.flow_n = t.flow_n, p.flow_na = t.flow_na;
     p.attn_skew = g_attn_skew, p.wait_cycles = g_wait_cycles > 0 ? g_wait_cycles : kWaitCycles, p.barrier_extra = g_barrier_extra;
     auto F = [&](int i) { return static_cast<const float*>(in[i]); };
     auto H = [&](int i) { return static_cast<const bf16*>(in[i]); };

@@ -51,7 +51,11 @@ struct Bufs {
 // What a block writes while units of the block before may still be reading: only QKVG and VT, which the attention
 // items of a whole sample read. They alternate between two buffers: what the one of the block before last held
 // has been read when this block's rows exist, since every row went through that block's attention.
-enum FlowCnt { FC_QKVG, FC_TO, FC_TC, FC_ACT1, FC_ACT2, FC_TX, FC_TX0, kFlowCnts };
+// Between two atom attentions every atom row goes through WO -> LN -> W1 -> W2 -> LN -> projections on its own: that
+// chain runs in the same way, counted per block of 128 atom rows, with grid barriers on either side of an attention
+// only. AXT, AX: the rows of the transition's and the projections' input; AC1, ACA, AC2: the tiles of WO, W1, W2.
+enum FlowCnt { FC_QKVG, FC_TO, FC_TC, FC_ACT1, FC_ACT2, FC_TX, FC_TX0, kFlowTok, FC_AX = kFlowTok, FC_AC1, FC_AXT, FC_ACA, FC_AC2, kFlowCnts };
+constexpr int kFlowAtom = kFlowCnts - kFlowTok;
 // A counter has a 128-byte line of its own: many CTAs poll it while others add to it, and neighbours in one line
 // would share that traffic.
 constexpr int kFlowPitch = 32;
@@ -96,7 +100,7 @@ struct KP {
     unsigned long long* timing; // per phase kind [wall ns, phases], or null
     unsigned int* flow_cnt; // completion counters of the token block's dependency chains (FlowCnt), flow_n each
     int flow;     // the token block's chains run on completion counters (the program was written that way)
-    int flow_n;   // entries per counter array
+    int flow_n, flow_na; // entries per counter array of the token blocks and of the atom blocks
     long long wait_cycles; // give-up limit of every wait of this launch (kWaitCycles unless a test shortened it)
     int barrier_extra;     // test hook: arrivals that the grid barriers expect on top of the grid's (0 in production)
     int attn_skew; // test hook: cycles by which the token attention's second pipeline starts late (0 in production)

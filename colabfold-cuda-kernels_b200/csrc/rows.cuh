@@ -439,6 +439,15 @@ __device__ __forceinline__ Oct oct_load(const float* row) {
     }
     return o;
 }
+// the same from L2: rows that other CTAs have just written
+__device__ __forceinline__ Oct oct_load_cg(const float* row) {
+    Oct o;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        o.v[j] = __ldcg(reinterpret_cast<const float4*>(row + oct_col() + 32 * j));
+    }
+    return o;
+}
 __device__ __forceinline__ void oct_layernorm(Oct& x, float eps) {
     float s = 0.f;
 #pragma unroll
@@ -460,12 +469,16 @@ __device__ __forceinline__ void oct_layernorm(Oct& x, float eps) {
         v.x *= rstd, v.y *= rstd, v.z *= rstd, v.w *= rstd;
     }
 }
-// rows of a range [first, end) go four to a warp step: this lane's row of step i
+// rows of a range [first, end) go four to a warp step: this lane's row of step i, and how many steps this warp has.
+// The two warps without a role in the GEMMs come first: where there are few rows, the roles' warps get on.
+__device__ __forceinline__ int oct_rank() {
+    return (warp_id() + kWarps - kAuxWarp0) % kWarps;
+}
 __device__ __forceinline__ int oct_row(int first, int i) {
-    return first + 4 * (warp_id() + kWarps * i) + (lane_id() >> 3);
+    return first + 4 * (oct_rank() + kWarps * i) + (lane_id() >> 3);
 }
 __device__ __forceinline__ int oct_steps(int first, int end) {
-    return cdiv(end - first, 4 * kWarps);
+    return max(0, cdiv(end - first - 4 * oct_rank(), 4 * kWarps));
 }
 
 // AXQ = bf16(LN(qa)·am0 + am1), AXK = bf16(LN(qa)·am2 + am3): the inputs of the q|g and k|v
@@ -474,7 +487,7 @@ __device__ __forceinline__ void atom_ln_qk_rows(const KP& p, const AtomW& w, int
     for (int i = 0; i < oct_steps(first, end); i++) {
         const int r = min(oct_row(first, i), end - 1); // a lane past the end redoes the last row
         const float* am = atom_mods(p, w, b, r % p.A);
-        Oct x = oct_load(p.buf.qa + size_t(r) * kAtomC);
+        Oct x = oct_load_cg(p.buf.qa + size_t(r) * kAtomC);
         const Oct qs = oct_load(am + AM_Q_SCALE * kAtomC), qb = oct_load(am + AM_Q_BIAS * kAtomC);
         const Oct ks = oct_load(am + AM_K_SCALE * kAtomC), kb = oct_load(am + AM_K_BIAS * kAtomC);
         oct_layernorm(x, p.ln_eps);
@@ -502,7 +515,7 @@ __device__ __forceinline__ void atom_ln_t_rows(const KP& p, const AtomW& w, int 
     for (int i = 0; i < oct_steps(first, end); i++) {
         const int r = min(oct_row(first, i), end - 1);
         const float* am = atom_mods(p, w, b, r % p.A);
-        Oct x = oct_load(p.buf.qa + size_t(r) * kAtomC);
+        Oct x = oct_load_cg(p.buf.qa + size_t(r) * kAtomC);
         const Oct ts = oct_load(am + AM_T_SCALE * kAtomC), tb = oct_load(am + AM_T_BIAS * kAtomC);
         oct_layernorm(x, p.ln_eps);
         bf16* o = p.buf.axhl + size_t(r) * 2 * kAtomC;
@@ -521,7 +534,7 @@ __device__ __forceinline__ void atom_tail_skip_rows(const KP& p, int first, int 
     for (int i = 0; i < oct_steps(first, end); i++) {
         const int r = min(oct_row(first, i), end - 1);
         const float m = p.geo.qmask[r % p.A];
-        const Oct x = oct_load(p.buf.qa + size_t(r) * kAtomC);
+        const Oct x = oct_load_cg(p.buf.qa + size_t(r) * kAtomC);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int c = oct_col() + 32 * j;
@@ -536,7 +549,7 @@ __device__ __forceinline__ void atom_tail_update_rows(const KP& p, int first, in
     for (int i = 0; i < oct_steps(first, end); i++) {
         const int r = min(oct_row(first, i), end - 1);
         const float m = p.geo.qmask[r % p.A];
-        Oct x = oct_load(p.buf.qa + size_t(r) * kAtomC);
+        Oct x = oct_load_cg(p.buf.qa + size_t(r) * kAtomC);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             x.v[j] = make_float4(x.v[j].x * m, x.v[j].y * m, x.v[j].z * m, x.v[j].w * m);
@@ -582,30 +595,63 @@ __device__ __forceinline__ void atom_qknorm_rows(const KP& p, const AtomW& w, in
         }
     }
 }
-// the same passes over all atom rows of the launch, 32 rows (four per warp) to a CTA item
-#define CCK_ATOM_ROWS_PHASE(name, call)                                        \
-    do {                                                                       \
-        const int rows_ = p.S * p.A, items_ = cdiv(rows_, 4 * kWarps);         \
-        for (int it_ = d.first(); it_ < items_; it_ += gridDim.x) {            \
-            const int f_ = it_ * 4 * kWarps, e_ = min(rows_, f_ + 4 * kWarps); \
-            call;                                                              \
-        }                                                                      \
-        d.advance(items_);                                                     \
-    } while (0)
-__device__ CCK_PHASE_FN void atom_ln_qk(const KP& p, Deal& d, const AtomW& w, int b) {
-    CCK_ATOM_ROWS_PHASE(atom_ln_qk, atom_ln_qk_rows(p, w, b, f_, e_));
+// The same passes over all atom rows of the launch. On barriers 48 rows (four per warp) to a CTA item. On completion
+// counters every CTA takes one contiguous run, waits for the blocks of 128 rows that it touches (gemms: how
+// many times the GEMM of counter `wait` has to have gone over them) and reports its own rows to `sig` (-1: a
+// barrier follows), a warp all of its steps behind one fence.
+__device__ __forceinline__ void atom_rows_wait(const KP& p, int which, unsigned int target, int first, int end) {
+    if (lane_id() == 0) {
+        flow_wait(flow_cnt(p, which), first / kBM, (end - 1) / kBM, target, &smem_ctl()->abort);
+    }
+    __syncwarp();
 }
-__device__ CCK_PHASE_FN void atom_ln_t(const KP& p, Deal& d, const AtomW& w, int b) {
-    CCK_ATOM_ROWS_PHASE(atom_ln_t, atom_ln_t_rows(p, w, b, f_, e_));
+__device__ __forceinline__ void atom_rows_report(const KP& p, int sig, int first, int end) {
+    fence_async_global(); // for TMA reads in other CTAs
+    __syncwarp();
+    if (lane_id() == 0) {
+        unsigned int* cnt = flow_cnt(p, sig);
+        fence_acq_rel_gpu();
+        for (int i = 0; i < oct_steps(first, end); i++) {
+            const int r = first + 4 * (oct_rank() + kWarps * i);
+            red_relaxed_add(cnt + r / kBM * kFlowPitch, (unsigned int)(min(4, end - r)));
+        }
+    }
+}
+#define CCK_ATOM_ROWS_PHASE(wait, gd, gemms, sig, call)                                                                                     \
+    do {                                                                                                                                    \
+        const int rows_ = p.S * p.A, per_ = p.flow ? cdiv(cdiv(rows_, int(gridDim.x)), 4) * 4 : 4 * kWarps, items_ = cdiv(rows_, per_);     \
+        for (int it_ = p.flow ? int(blockIdx.x) : d.first(); it_ < items_; it_ += gridDim.x) {                                              \
+            const int f_ = it_ * per_, e_ = min(rows_, f_ + per_);                                                                          \
+            if (p.flow) {                                                                                                                   \
+                if (oct_steps(f_, e_) == 0) {                                                                                               \
+                    break;                                                                                                                  \
+                }                                                                                                                           \
+                atom_rows_wait(p, wait, (gemms) * (unsigned int)(gd_table()[gd].nt * kWorkWarps), f_, e_);                                  \
+            }                                                                                                                               \
+            call;                                                                                                                           \
+            if (p.flow && (sig) >= 0) {                                                                                                     \
+                atom_rows_report(p, sig, f_, e_);                                                                                           \
+            }                                                                                                                               \
+        }                                                                                                                                   \
+        if (!p.flow) {                                                                                                                      \
+            d.advance(items_);                                                                                                              \
+        }                                                                                                                                   \
+    } while (0)
+// (epoch: the atom block's running number in the launch)
+__device__ CCK_PHASE_FN void atom_ln_qk(const KP& p, Deal& d, const AtomW& w, int b, unsigned int epoch) {
+    CCK_ATOM_ROWS_PHASE(FC_AC2, GD_ENC_W2, epoch, FC_AX, atom_ln_qk_rows(p, w, b, f_, e_));
+}
+__device__ CCK_PHASE_FN void atom_ln_t(const KP& p, Deal& d, const AtomW& w, int b, unsigned int epoch) {
+    CCK_ATOM_ROWS_PHASE(FC_AC1, GD_ENC_WO, epoch + 1, FC_AXT, atom_ln_t_rows(p, w, b, f_, e_));
 }
 __device__ CCK_PHASE_FN void atom_qknorm(const KP& p, Deal& d, const AtomW& w, int b) {
-    CCK_ATOM_ROWS_PHASE(atom_qknorm, atom_qknorm_rows(p, w, b, f_, e_));
+    CCK_ATOM_ROWS_PHASE(FC_AC2, GD_ENC_W2, 0u, -1, atom_qknorm_rows(p, w, b, f_, e_));
 }
-__device__ CCK_PHASE_FN void atom_tail_skip(const KP& p, Deal& d) {
-    CCK_ATOM_ROWS_PHASE(atom_tail_skip, atom_tail_skip_rows(p, f_, e_));
+__device__ CCK_PHASE_FN void atom_tail_skip(const KP& p, Deal& d, unsigned int epoch) {
+    CCK_ATOM_ROWS_PHASE(FC_AC2, GD_ENC_W2, epoch + 1, -1, atom_tail_skip_rows(p, f_, e_));
 }
-__device__ CCK_PHASE_FN void atom_tail_update(const KP& p, Deal& d) {
-    CCK_ATOM_ROWS_PHASE(atom_tail_update, atom_tail_update_rows(p, f_, e_));
+__device__ CCK_PHASE_FN void atom_tail_update(const KP& p, Deal& d, unsigned int epoch) {
+    CCK_ATOM_ROWS_PHASE(FC_AC2, GD_ENC_W2, epoch + 1, -1, atom_tail_update_rows(p, f_, e_));
 }
 
 // qa = (skip + tb[token of a])·QMASK (reference: src/diffusion/rows.cuh:246-261)

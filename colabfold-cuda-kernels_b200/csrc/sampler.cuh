@@ -273,6 +273,11 @@ __device__ inline GemmDesc gemm_atom(const KP& p, int side, int b, int which) {
         g.gate = am + AM_T_GATE * kAtomC, g.gate_f32 = 1, g.ldg = kAtomModSlots * kAtomC, g.period = p.A;
         g.rowmask = p.geo.qmask;
     }
+    if (p.flow) {
+        const int sig = which == AG_WO ? 1 + FC_AC1 : which == AG_W1 ? 1 + FC_ACA : which == AG_W2 ? 1 + FC_AC2 : 0; // (a barrier follows the projections)
+        const int dep = which == AG_WO ? 0 : 1 + (which == AG_W1 ? FC_AXT : which == AG_W2 ? FC_ACA : FC_AX);        // (and precedes WO)
+        g.fl = GF_NFAST | sig << GF_SIG_SHIFT | dep << GF_DEP_SHIFT;
+    }
     return g;
 }
 // descriptor `id` of the table, as of block b of its stack
@@ -340,7 +345,7 @@ __device__ CCK_PHASE_FN void pair_fill_pads(const KP& p, Deal& d) {
         }
     }
     if (p.flow) { // the completion counters of the token blocks' chains
-        for (size_t i = tid; i < size_t(kFlowCnts) * p.flow_n * kFlowPitch; i += nth) {
+        for (size_t i = tid; i < (size_t(kFlowTok) * p.flow_n + size_t(kFlowAtom) * p.flow_na) * kFlowPitch; i += nth) {
             p.flow_cnt[i] = 0;
         }
     }
@@ -399,10 +404,16 @@ __device__ __forceinline__ void run_gemm(const Launch& L, Run& r, Deal& d, int i
 
 // How many token blocks of this launch came before the current one (denoiser calls so far x blocks
 // + the block): the completion counters count on through the launch and are compared with multiples of it
-__device__ __forceinline__ unsigned int flow_epoch(const KP& p, const Run& r) {
+__device__ __forceinline__ unsigned int flow_calls(const KP& p, const Run& r) { // denoiser calls before this one
     const int calls_per_step = (p.flags & F_HEUN) && !(p.flags & F_REALIGN) ? 2 : 1;
-    const int calls = p.mode == 0 ? (int(r.step) - 1) * calls_per_step + r.second : 0;
-    return (unsigned int)(calls * p.nb + r.blk);
+    return p.mode == 0 ? (unsigned int)((int(r.step) - 1) * calls_per_step + r.second) : 0u;
+}
+__device__ __forceinline__ unsigned int flow_epoch(const KP& p, const Run& r) {
+    return flow_calls(p, r) * p.nb + r.blk;
+}
+// the same for the atom blocks, encoder and decoder
+__device__ __forceinline__ unsigned int atom_epoch(const KP& p, const Run& r, int side, int b) {
+    return flow_calls(p, r) * (2 * kAtomBlocks) + side * kAtomBlocks + b;
 }
 // one operation of the program; everything it needs comes from shared memory
 __device__ __forceinline__ void run_op(const Launch& L, Run& r, const Op op) {
@@ -411,7 +422,7 @@ __device__ __forceinline__ void run_op(const Launch& L, Run& r, const Op op) {
     Deal& d = r.d;
     switch (op.fn) {
     case FN_GEMM:
-        run_gemm(L, r, d, op.a0, b, flow_epoch(p, r));
+        run_gemm(L, r, d, op.a0, b, op.a0 >= GD_ENC_QG ? atom_epoch(p, r, op.a0 >= GD_DEC_QG, b) : flow_epoch(p, r));
         break;
     case FN_POS_INIT:
         positions_init(p, d);
@@ -459,19 +470,19 @@ __device__ __forceinline__ void run_op(const Launch& L, Run& r, const Op op) {
         sc_prep(p, d);
         break;
     case FN_ATOM_LN_QK:
-        atom_ln_qk(p, d, op.a0 ? p.dec : p.enc, b);
+        atom_ln_qk(p, d, op.a0 ? p.dec : p.enc, b, atom_epoch(p, r, op.a0, b));
         break;
     case FN_ATOM_ATTN:
         atom_attention(p, d, op.a0 ? p.dec : p.enc, b);
         break;
     case FN_ATOM_LN_T:
-        atom_ln_t(p, d, op.a0 ? p.dec : p.enc, b);
+        atom_ln_t(p, d, op.a0 ? p.dec : p.enc, b, atom_epoch(p, r, op.a0, b));
         break;
     case FN_ATOM_TAIL_SKIP:
-        atom_tail_skip(p, d);
+        atom_tail_skip(p, d, atom_epoch(p, r, 0, kAtomBlocks - 1));
         break;
     case FN_ATOM_TAIL_UPDATE:
-        atom_tail_update(p, d);
+        atom_tail_update(p, d, atom_epoch(p, r, 1, kAtomBlocks - 1));
         break;
     case FN_AGGR_GATHER:
         aggr_gather(p, d);
