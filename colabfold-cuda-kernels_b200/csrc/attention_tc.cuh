@@ -154,10 +154,10 @@ __device__ __forceinline__ TcItem tc_item(int it, int S, int qblocks, bool flow)
     const KP& p = kp();
     TcItem i;
     if (flow) {
-        const uint32_t u = uint32_t(it) / kHeads, v = p.tc_div_qblocks ? __umulhi(u, p.tc_div_qblocks) : u;
+        const uint32_t u = uint32_t(it) / kHeads, v = div_prepared(u, p.tc_div_qblocks);
         i.s = int(v), i.qb = int(u) - int(v) * qblocks, i.h = it % kHeads;
     } else {
-        const uint32_t u = p.tc_div_s ? __umulhi(uint32_t(it), p.tc_div_s) : uint32_t(it);
+        const uint32_t u = div_prepared(uint32_t(it), p.tc_div_s);
         i.s = it - int(u) * S, i.h = int(u % kHeads), i.qb = int(u / kHeads);
     }
     return i;
@@ -165,7 +165,7 @@ __device__ __forceinline__ TcItem tc_item(int it, int S, int qblocks, bool flow)
 // The CTA's items of a phase are first, first + grid, ...; track t takes every second one from the
 // t-th on. How many that is:
 __device__ __forceinline__ int tc_track_items(int first, int items, int t) {
-    const int mine = items > first ? (items - first + int(gridDim.x) - 1) / int(gridDim.x) : 0;
+    const int mine = items > first ? int(div_prepared(uint32_t(items - first + int(gridDim.x) - 1), kp().div_grid)) : 0;
     return (mine - t + kTcTracks - 1) / kTcTracks;
 }
 __device__ __forceinline__ int tc_track_item(int first, int t, int j) {

@@ -123,7 +123,7 @@ constexpr int kRunOff = kCtlOff + kCtlBytes;
 constexpr int kKpOff = kRunOff + kRunSlot * kThreads;           // the CTA's copy of the parameter block
 constexpr int kKpBytes = 1280;
 constexpr int kGdOff = kKpOff + kKpBytes;                       // prepared GEMM descriptors
-constexpr int kGdBytes = 4608;
+constexpr int kGdBytes = 4800;
 constexpr int kProgOff = kGdOff + kGdBytes;                     // the phase program
 constexpr int kProgBytes = 512;
 static_assert(sizeof(Program) <= kProgBytes, "the phase program outgrew its shared-memory slot");
@@ -159,6 +159,16 @@ __device__ __forceinline__ void fail_launch(unsigned int code, unsigned int wher
     atomicOr(&c->barrier, kBarrierPoison);
 }
 
+// n / d with a prepared multiplier (div_magic; 0: d = 1). A division by a number known only at run time is some 40
+// instructions, and an operation's way in and out is run once per operation, from a cold instruction cache at 5 to 9
+// cycles an instruction.
+__host__ __device__ constexpr uint32_t div_magic(uint32_t d) {
+    return d > 1 ? 0xFFFFFFFFu / d + 1u : 0u; // exact while n·d < 2^32
+}
+__device__ __forceinline__ uint32_t div_prepared(uint32_t n, uint32_t magic) {
+    return magic ? __umulhi(n, magic) : n;
+}
+
 // per-thread pipeline positions, kept across phases for the whole launch
 struct Pipe {
     uint32_t ring = 0; // phase parity of each slot of the operand ring, as this role passes them
@@ -169,11 +179,13 @@ struct Pipe {
 // one phase continue the rotation (as the reference's Deal, src/diffusion/gemm.cuh:84-95)
 struct Deal {
     int start = 0;
-    __device__ int first() const {
-        return (int(blockIdx.x) - start + int(gridDim.x)) % int(gridDim.x);
+    __device__ __forceinline__ int first() const {
+        const int f = int(blockIdx.x) - start;
+        return f < 0 ? f + int(gridDim.x) : f;
     }
-    __device__ void advance(int items) {
-        start = (start + items) % int(gridDim.x);
+    __device__ __forceinline__ void advance(int items) {
+        const uint32_t n = uint32_t(start + items);
+        start = int(n - div_prepared(n, kp().div_grid) * gridDim.x);
     }
 };
 
@@ -521,7 +533,7 @@ __device__ __forceinline__ void resid_tile(const GemmDesc& g, const void* gate, 
     const char* gp[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const int row = min(r0 + 8 * i, m - 1), p = row % g.period;
+        const int row = min(r0 + 8 * i, m - 1), p = row - (g.div_period ? int(__umulhi((unsigned int)row, g.div_period)) : row / g.period) * g.period;
         mask[i] = g.rowmask ? g.rowmask[p] : 1.f;
         gp[i] = static_cast<const char*>(gate) + (size_t(p) * g.ldg + col0 + c0 + cl) * (GF32 ? 4 : 2);
 #pragma unroll
@@ -582,6 +594,7 @@ __host__ __device__ inline void gd_finish(GemmDesc& g) {
     if (inner == 1) {
         g.mt_magic = 0; // 2^32 does not fit
     }
+    g.div_period = (unsigned long long)(g.m) * g.period < 0x100000000ull && g.period > 1 ? div_magic(g.period) : 0u;
 }
 
 // ---- prepared GEMM descriptors: built once per launch into shared memory, so that a phase starts
@@ -668,22 +681,31 @@ __device__ __forceinline__ bool flow_wait(const unsigned int* cnt, int c0, int c
 // the attention items of every block of 128 queries (per sample of g.period rows) that the rows
 // touch, 16 heads x 4 warps each. TC: the column tiles of W1 over these rows, 8 warps each. ACA: the same of the atoms. TX,
 // TX0, AX, AXT: the rows of the block.
-__device__ __forceinline__ unsigned int flow_target(const GemmDesc& g, int which, int rb) {
-    if (which == FC_TX || which == FC_TX0 || which == FC_AX || which == FC_AXT) {
-        return (unsigned int)(min(kBM, g.m - rb * kBM));
-    }
-    if (which != FC_TO) {
-        return (unsigned int)(gd_table()[which == FC_TC ? GD_TOK_W1 : GD_ENC_W1].nt * kWorkWarps);
-    }
+__device__ __noinline__ unsigned int flow_target_to(const GemmDesc& g, int rb) {
     const int lo = rb * kBM, hi = min(lo + kBM, g.m) - 1, qblocks = cdiv(g.period, kBM);
     const int ilo = lo / g.period * qblocks + lo % g.period / kBM, ihi = hi / g.period * qblocks + hi % g.period / kBM;
     return (unsigned int)(kHeads * kAttnItemWarps * (ihi - ilo + 1));
 }
+__device__ __forceinline__ unsigned int flow_target(const GemmDesc& g, int which, int rb) {
+    if (g.dep_target) {
+        return g.dep_target;
+    }
+    return which == FC_TO ? flow_target_to(g, rb) : (unsigned int)(min(kBM, g.m - rb * kBM));
+}
+// (part of the descriptor, once all of them are there)
+__device__ inline void gd_finish_target(GemmDesc& g) {
+    const int which = int(g.fl >> GF_DEP_SHIFT & GF_CNT_MASK) - 1;
+    g.dep_target = which == FC_TC    ? (unsigned int)(gd_table()[GD_TOK_W1].nt * kWorkWarps)
+                   : which == FC_ACA ? (unsigned int)(gd_table()[GD_ENC_W1].nt * kWorkWarps)
+                   : which == FC_TO && g.period % kBM == 0 ? (unsigned int)(kHeads * kAttnItemWarps)
+                                                           : 0u;
+}
 
 // the worker warps' loop over the tiles of one GEMM, block b of its stack; every finished tile is
 // reported to the completion counter of its block of 128 rows, if the descriptor names one
-template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, const CUtensorMap* mo, int b, uint32_t tile, int tb, int te, int ts,
+template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, const CUtensorMap* mo, int b, Pipe& pipe, int tb, int te, int ts,
                                                          unsigned int epoch) {
+    uint32_t tile = pipe.tile;
     SmemCtl* ctl = smem_ctl();
     GemmDesc g = gd; // a private copy: stores through its pointers cannot alias it
     g.bias = g.bias ? g.bias + size_t(b) * g.bias_step : nullptr;
@@ -705,8 +727,10 @@ template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, con
             // the attention's adaLN rows have waited for; WO for W2, which came before W1's tiles.
             if (const int depc = gd.fl >> GF_DEP_SHIFT & GF_CNT_MASK) {
                 if (lane_id() == 0) {
-                    const int which = depc == 1 + FC_TO ? FC_TX0 : depc - 1, rb = row0 / kBM;
-                    flow_wait(flow_cnt(kp(), which), rb, rb, (epoch + 1) * flow_target(gd, which, rb), &ctl->abort);
+                    const bool wo = depc == 1 + FC_TO;
+                    const int rb = row0 / kBM;
+                    const unsigned int target = wo ? (unsigned int)(min(kBM, gd.m - row0)) : flow_target(gd, depc - 1, rb);
+                    flow_wait(flow_cnt(kp(), wo ? FC_TX0 : depc - 1), rb, rb, (epoch + 1) * target, &ctl->abort);
                 }
                 __syncwarp();
             }
@@ -739,6 +763,7 @@ template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, con
         }
         CCK_TRACE_EV(0x74, t); // stored and reported
     }
+    pipe.tile = tile;
     if constexpr (E == EPI_BF16 || E == EPI_GLU || E == EPI_MODS) {
         if (lane_id() == 0) {
             bulk_wait_done(); // this warp's TMA stores have landed before the phase ends

@@ -108,6 +108,8 @@ struct KP {
     // that divide an item number by that and by S (n / d = umulhi(n, m) while n·d < 2^32; m = 0: d = 1)
     int tc_qblocks;
     uint32_t tc_div_qblocks, tc_div_s;
+    uint32_t div_grid, div_n; // the same for the grid and for N
+    int tok_rows;             // token rows of a CTA where each takes one contiguous run: cdiv(S·N, grid)
 };
 
 // phase kinds of the per-kind timing record (mk_run's `timing`): wall ns and count per kind
@@ -222,6 +224,8 @@ struct GemmDesc {
     // what block b of a stack adds: rows of W, floats of bias, bytes of gate
     int b_step, bias_step;
     long long gate_step;
+    unsigned int dep_target; // arrivals that complete a row block of A, where that is the same for all blocks (flow_target), else 0
+    unsigned int div_period; // row / period = umulhi(row, div_period); 0: divide
 };
 
 } // namespace cck

@@ -205,7 +205,7 @@ struct AdaRow {
 };
 // the row's modulations (known since the conditioning ran: nothing to wait for)
 __device__ __forceinline__ void adaln_load_mods(AdaRow& a, const KP& p, const bf16* ms, const bf16* mo, int r) {
-    const size_t mrow = size_t(r % p.N) * kTokC + 4 * lane_id();
+    const size_t mrow = size_t(r - int(div_prepared(uint32_t(r), p.div_n)) * p.N) * kTokC + 4 * lane_id();
 #pragma unroll
     for (int j = 0; j < 6; j++) {
         a.s[j] = *reinterpret_cast<const uint2*>(ms + mrow + 128 * j);
@@ -264,7 +264,7 @@ __device__ __forceinline__ FlowRows flow_rows(const KP& p, int rows, int which, 
     // Where a warp has a row or two, the first go to the two warps without a role in the GEMMs, which are there first;
     // the roles' own warps get on with the next operation (390-1900 rows: 1.5%). With three rows and more to a warp,
     // 1024 x 5, that order took 2% longer.
-    const int per = cdiv(rows, int(gridDim.x)), rank = per <= 2 * kWarps ? (warp_id() + kWarps - kAuxWarp0) % kWarps : warp_id();
+    const int per = p.tok_rows, rank = per <= 2 * kWarps ? (warp_id() + kWarps - kAuxWarp0) % kWarps : warp_id();
     f.r0 = min(rows, int(blockIdx.x) * per) + rank, f.r1 = min(rows, (int(blockIdx.x) + 1) * per), f.ok = -1;
     f.cnt = flow_cnt(p, which);
     f.target = gemms_done * (unsigned int)(gd_table()[which == FC_ACT1 ? GD_TOK_WO : GD_TOK_W2].nt * kWorkWarps);

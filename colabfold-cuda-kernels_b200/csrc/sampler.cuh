@@ -322,6 +322,10 @@ __device__ __noinline__ void gd_build() {
         gd_table()[threadIdx.x] = g;
     }
     __syncthreads();
+    if (threadIdx.x < kNumGd) {
+        gd_finish_target(gd_table()[threadIdx.x]);
+    }
+    __syncthreads();
 }
 
 // What the pair-logit GEMM does not write but attention may read: VT's key pads (P is exactly zero
@@ -372,31 +376,29 @@ __device__ __forceinline__ void run_gemm(const Launch& L, Run& r, Deal& d, int i
     } else if (warp == 1) {
         gemm_issue(r.pipe, g, tb, tiles, ts);
     } else if (warp < kAuxWarp0) {
-        const uint32_t tile = r.pipe.tile;
         const CUtensorMap* mo = g.map_o >= 0 ? &L.tmap[g.map_o + ((g.fl & GF_ALT) ? epoch & 1 : 0)] : nullptr;
         switch (g.epi) {
         case EPI_BF16:
-            worker_tiles<EPI_BF16>(g, mo, b, tile, tb, tiles, ts, epoch);
+            worker_tiles<EPI_BF16>(g, mo, b, r.pipe, tb, tiles, ts, epoch);
             break;
         case EPI_F32:
-            worker_tiles<EPI_F32>(g, mo, b, tile, tb, tiles, ts, epoch);
+            worker_tiles<EPI_F32>(g, mo, b, r.pipe, tb, tiles, ts, epoch);
             break;
         case EPI_SCRES:
-            worker_tiles<EPI_SCRES>(g, mo, b, tile, tb, tiles, ts, epoch);
+            worker_tiles<EPI_SCRES>(g, mo, b, r.pipe, tb, tiles, ts, epoch);
             break;
         case EPI_MODS:
-            worker_tiles<EPI_MODS>(g, mo, b, tile, tb, tiles, ts, epoch);
+            worker_tiles<EPI_MODS>(g, mo, b, r.pipe, tb, tiles, ts, epoch);
             break;
         case EPI_GLU:
-            worker_tiles<EPI_GLU>(g, mo, b, tile, tb, tiles, ts, epoch);
+            worker_tiles<EPI_GLU>(g, mo, b, r.pipe, tb, tiles, ts, epoch);
             break;
         case EPI_RESID:
-            worker_tiles<EPI_RESID>(g, mo, b, tile, tb, tiles, ts, epoch);
+            worker_tiles<EPI_RESID>(g, mo, b, r.pipe, tb, tiles, ts, epoch);
             break;
         default:
-            worker_tiles<EPI_PAIR>(g, mo, b, tile, tb, tiles, ts, epoch);
+            worker_tiles<EPI_PAIR>(g, mo, b, r.pipe, tb, tiles, ts, epoch);
         }
-        r.pipe.tile = tile + (tiles > tb ? (tiles - tb + ts - 1) / ts : 0);
     }
     __syncwarp();
     d.advance(tiles);
@@ -544,8 +546,9 @@ extern "C" __global__ void __launch_bounds__(cck::kThreads, 1) cck_sampler_kerne
             }
             w.A = w.NS * kSubset, w.np = cdiv(w.N, kTcKeys) * kTcKeys, w.chunks = cdiv(w.N * kSlots, kChunk);
             w.tc_qblocks = cdiv(w.N, kTcRows);
-            w.tc_div_qblocks = w.tc_qblocks > 1 ? 0xFFFFFFFFu / uint32_t(w.tc_qblocks) + 1u : 0u;
-            w.tc_div_s = w.S > 1 ? 0xFFFFFFFFu / uint32_t(w.S) + 1u : 0u;
+            w.tc_div_qblocks = div_magic(w.tc_qblocks), w.tc_div_s = div_magic(w.S);
+            w.div_grid = div_magic(gridDim.x), w.div_n = div_magic(w.N);
+            w.tok_rows = cdiv(w.S * w.N, int(gridDim.x));
         }
         __syncthreads();
     }
