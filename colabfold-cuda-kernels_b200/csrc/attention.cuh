@@ -173,7 +173,7 @@ __device__ CCK_HOT_FN void atom_attention(const KP& p, Deal& d, const AtomW& w, 
     bf16* sm = reinterpret_cast<bf16*>(smem_base() + warp_id() * kAwBytes);
     const int lane = lane_id();
     for (int un = d.first() * kAwWarps + warp_id(); un < units && warp_id() < kAwWarps; un += gridDim.x * kAwWarps) {
-        const int s = un % p.S, h = un / p.S % kAtomHeads, u = un / (p.S * kAtomHeads);
+        const int v = int(div_prepared(uint32_t(un), p.tc_div_s)), s = un - v * p.S, h = v % kAtomHeads, u = v / kAtomHeads;
         __syncwarp(); // every lane is done with the previous window
         // the head's slice of the window's [k | v] rows: 128 rows x (64 + 64) bytes, zero where Q2K is -1.
         // Four lanes copy one 64-byte slice, so an instruction touches 8 lines rather than 32.

@@ -165,6 +165,16 @@ __device__ __forceinline__ void fail_launch(unsigned int code, unsigned int wher
 __host__ __device__ constexpr uint32_t div_magic(uint32_t d) {
     return d > 1 ? 0xFFFFFFFFu / d + 1u : 0u; // exact while n·d < 2^32
 }
+// the same for rows up to `most`; 0 where the product would not fit: divide
+__host__ __device__ constexpr uint32_t div_magic_rows(uint32_t d, unsigned long long most) {
+    return most * d < 0x100000000ull ? div_magic(d) : 0u;
+}
+__device__ __forceinline__ int div_rows(int r, int d, uint32_t magic) {
+    return magic ? int(__umulhi(uint32_t(r), magic)) : r / d;
+}
+__device__ __forceinline__ int mod_rows(int r, int d, uint32_t magic) {
+    return r - div_rows(r, d, magic) * d;
+}
 __device__ __forceinline__ uint32_t div_prepared(uint32_t n, uint32_t magic) {
     return magic ? __umulhi(n, magic) : n;
 }
@@ -329,7 +339,8 @@ __device__ __forceinline__ void pair_unit(const GemmDesc& g, int rbase, int c0, 
 __device__ __forceinline__ void vt_unit(const GemmDesc& g, int rbase, int c0, const float (&v)[32]) {
     const int row = rbase + lane_id();
     if (row < g.m) {
-        bf16* o = g.vt + (size_t(row / g.period) * kTokC + (c0 - 2 * kTokC)) * g.np + row % g.period;
+        const int s = div_rows(row, g.period, g.div_period);
+        bf16* o = g.vt + (size_t(s) * kTokC + (c0 - 2 * kTokC)) * g.np + (row - s * g.period);
 #pragma unroll
         for (int i = 0; i < 32; i++) {
             o[size_t(i) * g.np] = bf16(pack_bf2(v[i], 0.f) & 0xFFFFu);
@@ -533,7 +544,7 @@ __device__ __forceinline__ void resid_tile(const GemmDesc& g, const void* gate, 
     const char* gp[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const int row = min(r0 + 8 * i, m - 1), p = row - (g.div_period ? int(__umulhi((unsigned int)row, g.div_period)) : row / g.period) * g.period;
+        const int row = min(r0 + 8 * i, m - 1), p = mod_rows(row, g.period, g.div_period);
         mask[i] = g.rowmask ? g.rowmask[p] : 1.f;
         gp[i] = static_cast<const char*>(gate) + (size_t(p) * g.ldg + col0 + c0 + cl) * (GF32 ? 4 : 2);
 #pragma unroll
@@ -594,7 +605,7 @@ __host__ __device__ inline void gd_finish(GemmDesc& g) {
     if (inner == 1) {
         g.mt_magic = 0; // 2^32 does not fit
     }
-    g.div_period = (unsigned long long)(g.m) * g.period < 0x100000000ull && g.period > 1 ? div_magic(g.period) : 0u;
+    g.div_period = div_magic_rows(g.period, g.m);
 }
 
 // ---- prepared GEMM descriptors: built once per launch into shared memory, so that a phase starts
@@ -796,8 +807,8 @@ __device__ __forceinline__ TileRows tile_rows(const GemmDesc& gd, int b, int t) 
 // A GEMM with another column tile lays the ring out anew: what the slots hold must have been consumed.
 __device__ __forceinline__ void ring_layout(SmemCtl* ctl, uint32_t ring, int bn) {
     if (uni(ctl->ring_bn) != bn) {
-        for (int s = 0; s < kMaxSlots; s++) {
-            mbar_wait(&ctl->empty[s], (ring >> s & 1) ^ 1, &ctl->abort);
+        if (lane_id() < kMaxSlots) { // (a lane per slot: a wait that passes costs 90 cycles)
+            mbar_wait(&ctl->empty[lane_id()], (ring >> lane_id() & 1) ^ 1, &ctl->abort);
         }
         __syncwarp();
         ctl->ring_bn = bn;

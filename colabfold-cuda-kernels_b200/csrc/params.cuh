@@ -108,7 +108,8 @@ struct KP {
     // that divide an item number by that and by S (n / d = umulhi(n, m) while n·d < 2^32; m = 0: d = 1)
     int tc_qblocks;
     uint32_t tc_div_qblocks, tc_div_s;
-    uint32_t div_grid, div_n; // the same for the grid and for N
+    uint32_t div_grid;       // the same for the grid
+    uint32_t div_n, div_a;   // the same for N and A and rows of all samples; 0: divide
     int tok_rows;             // token rows of a CTA where each takes one contiguous run: cdiv(S·N, grid)
 };
 

@@ -205,7 +205,7 @@ struct AdaRow {
 };
 // the row's modulations (known since the conditioning ran: nothing to wait for)
 __device__ __forceinline__ void adaln_load_mods(AdaRow& a, const KP& p, const bf16* ms, const bf16* mo, int r) {
-    const size_t mrow = size_t(r - int(div_prepared(uint32_t(r), p.div_n)) * p.N) * kTokC + 4 * lane_id();
+    const size_t mrow = size_t(mod_rows(r, p.N, p.div_n)) * kTokC + 4 * lane_id();
 #pragma unroll
     for (int j = 0; j < 6; j++) {
         a.s[j] = *reinterpret_cast<const uint2*>(ms + mrow + 128 * j);
@@ -369,7 +369,7 @@ __device__ CCK_PHASE_FN void token_final_ln(const KP& p, Deal& d, unsigned int e
 __device__ CCK_PHASE_FN void aggr_gather(const KP& p, Deal& d) {
     const int rows = p.S * p.N;
     for (int r = row_first(d); r < rows; r += row_step()) {
-        const int s = r / p.N, n = r % p.N, lane = lane_id();
+        const int s = div_rows(r, p.N, p.div_n), n = r - s * p.N, lane = lane_id();
         // the token's slots, one per lane; then its atoms' rows two at a time, in slot order (a slot per step, each
         // waiting for its index and then for its row, was 24 trips to L2: 24 -> 20 us at 512 x 5, 10 -> 7.7 at 32 x 1)
         const float wl = lane < kSlots ? p.geo.tam[n * kSlots + lane] : 0.f;
@@ -486,7 +486,7 @@ __device__ __forceinline__ int oct_steps(int first, int end) {
 __device__ __forceinline__ void atom_ln_qk_rows(const KP& p, const AtomW& w, int b, int first, int end) {
     for (int i = 0; i < oct_steps(first, end); i++) {
         const int r = min(oct_row(first, i), end - 1); // a lane past the end redoes the last row
-        const float* am = atom_mods(p, w, b, r % p.A);
+        const float* am = atom_mods(p, w, b, mod_rows(r, p.A, p.div_a));
         Oct x = oct_load_cg(p.buf.qa + size_t(r) * kAtomC);
         const Oct qs = oct_load(am + AM_Q_SCALE * kAtomC), qb = oct_load(am + AM_Q_BIAS * kAtomC);
         const Oct ks = oct_load(am + AM_K_SCALE * kAtomC), kb = oct_load(am + AM_K_BIAS * kAtomC);
@@ -514,7 +514,7 @@ __device__ __forceinline__ void atom_ln_qk_rows(const KP& p, const AtomW& w, int
 __device__ __forceinline__ void atom_ln_t_rows(const KP& p, const AtomW& w, int b, int first, int end) {
     for (int i = 0; i < oct_steps(first, end); i++) {
         const int r = min(oct_row(first, i), end - 1);
-        const float* am = atom_mods(p, w, b, r % p.A);
+        const float* am = atom_mods(p, w, b, mod_rows(r, p.A, p.div_a));
         Oct x = oct_load_cg(p.buf.qa + size_t(r) * kAtomC);
         const Oct ts = oct_load(am + AM_T_SCALE * kAtomC), tb = oct_load(am + AM_T_BIAS * kAtomC);
         oct_layernorm(x, p.ln_eps);
@@ -533,7 +533,7 @@ __device__ __forceinline__ void atom_ln_t_rows(const KP& p, const AtomW& w, int 
 __device__ __forceinline__ void atom_tail_skip_rows(const KP& p, int first, int end) {
     for (int i = 0; i < oct_steps(first, end); i++) {
         const int r = min(oct_row(first, i), end - 1);
-        const float m = p.geo.qmask[r % p.A];
+        const float m = p.geo.qmask[mod_rows(r, p.A, p.div_a)];
         const Oct x = oct_load_cg(p.buf.qa + size_t(r) * kAtomC);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -548,7 +548,7 @@ __device__ __forceinline__ void atom_tail_skip_rows(const KP& p, int first, int 
 __device__ __forceinline__ void atom_tail_update_rows(const KP& p, int first, int end) {
     for (int i = 0; i < oct_steps(first, end); i++) {
         const int r = min(oct_row(first, i), end - 1);
-        const float m = p.geo.qmask[r % p.A];
+        const float m = p.geo.qmask[mod_rows(r, p.A, p.div_a)];
         Oct x = oct_load_cg(p.buf.qa + size_t(r) * kAtomC);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -659,7 +659,7 @@ __device__ CCK_PHASE_FN void decoder_init(const KP& p, Deal& d) {
     const int rows = p.S * p.A;
     const int c = 4 * lane_id();
     for (int r = row_first(d); r < rows; r += row_step()) {
-        const int s = r / p.A, a = r % p.A;
+        const int s = div_rows(r, p.A, p.div_a), a = r - s * p.A;
         const int slot = p.geo.tok2q[a];
         const float m = p.geo.qmask[a];
         float4 x = ld4(p.buf.skip + size_t(r) * kAtomC + c);

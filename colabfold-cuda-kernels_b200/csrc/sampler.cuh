@@ -547,7 +547,8 @@ extern "C" __global__ void __launch_bounds__(cck::kThreads, 1) cck_sampler_kerne
             w.A = w.NS * kSubset, w.np = cdiv(w.N, kTcKeys) * kTcKeys, w.chunks = cdiv(w.N * kSlots, kChunk);
             w.tc_qblocks = cdiv(w.N, kTcRows);
             w.tc_div_qblocks = div_magic(w.tc_qblocks), w.tc_div_s = div_magic(w.S);
-            w.div_grid = div_magic(gridDim.x), w.div_n = div_magic(w.N);
+            w.div_grid = div_magic(gridDim.x);
+            w.div_n = div_magic_rows(w.N, w.S * w.N), w.div_a = div_magic_rows(w.A, (unsigned long long)(w.S) * w.A);
             w.tok_rows = cdiv(w.S * w.N, int(gridDim.x));
         }
         __syncthreads();
