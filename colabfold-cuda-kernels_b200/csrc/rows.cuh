@@ -255,16 +255,21 @@ __device__ CCK_PHASE_FN void token_adaln2(const KP& p, Deal& d, int b) {
 // wrote ACT over the row's block are complete (cnt counts on through the launch: target is the
 // count after the GEMM of the current token block). Returns false when the wait gave up.
 struct FlowRows {
-    int r0, r1, ok;
+    int r0, r1, ok, step;
     const unsigned int* cnt;
     unsigned int target;
 };
 __device__ __forceinline__ FlowRows flow_rows(const KP& p, int rows, int which, unsigned int gemms_done) {
     FlowRows f;
-    // Where a warp has a row or two, the first go to the two warps without a role in the GEMMs, which are there first;
-    // the roles' own warps get on with the next operation (390-1900 rows: 1.5%). With three rows and more to a warp,
-    // 1024 x 5, that order took 2% longer.
-    const int per = p.tok_rows, rank = per <= 2 * kWarps ? (warp_id() + kWarps - kAuxWarp0) % kWarps : warp_id();
+    // The warps that hold the GEMM roles take rows only where that saves the workers a second or a further one: they
+    // get on with the next operation, whose weights they fetch meanwhile (256 x 5: 1.601 -> 1.571 ms per step, 512 x 5:
+    // 2.457 -> 2.430). The two warps without a role come first, the workers, which still have W2's or WO's epilogue to
+    // finish, after them; up to kWarps + 2 rows those two alone have a second row.
+    const int per = p.tok_rows, w = warp_id();
+    const bool roles = (per > kWarps - 2 && per <= kWarps + 2) || cdiv(per, kWarps - 2) > cdiv(per, kWarps);
+    f.step = roles ? kWarps : kWarps - 2;
+    const int aux_first = (w + kWarps - kAuxWarp0) % kWarps; // idle, roles, workers
+    const int rank = roles ? (per <= 2 * kWarps ? aux_first : w) : w >= kAuxWarp0 ? w - kAuxWarp0 : w >= kWorkWarp0 ? w : per;
     f.r0 = min(rows, int(blockIdx.x) * per) + rank, f.r1 = min(rows, (int(blockIdx.x) + 1) * per), f.ok = -1;
     f.cnt = flow_cnt(p, which);
     f.target = gemms_done * (unsigned int)(gd_table()[which == FC_ACT1 ? GD_TOK_WO : GD_TOK_W2].nt * kWorkWarps);
@@ -288,7 +293,7 @@ __device__ CCK_HOT_FN void token_adaln(const KP& p, Deal& d, int b, int slot, un
         // the attention's input follows W2 of the block before, the transition's input WO of this block
         FlowRows f = flow_rows(p, rows, slot == TM_ATTN_SCALE ? FC_ACT2 : FC_ACT1, epoch + (slot != TM_ATTN_SCALE));
         unsigned int* tx_done = flow_cnt(p, slot == TM_ATTN_SCALE ? FC_TX0 : FC_TX);
-        for (int r = f.r0; r < f.r1; r += kWarps) {
+        for (int r = f.r0; r < f.r1; r += f.step) {
             AdaRow a0;
             adaln_load_mods(a0, p, ms, mo, r); // (nothing to wait for: they travel while the counter is awaited)
             flow_row_wait(f, r);
@@ -348,7 +353,7 @@ __device__ CCK_PHASE_FN void token_final_ln(const KP& p, Deal& d, unsigned int e
     const int rows = p.S * p.N;
     if (p.flow) { // after W2 of the last token block
         FlowRows f = flow_rows(p, rows, FC_ACT2, epoch);
-        for (int r = f.r0; r < f.r1; r += kWarps) {
+        for (int r = f.r0; r < f.r1; r += f.step) {
             flow_row_wait(f, r);
             RowV<6> x = load_f32_cg<6>(p.buf.act + size_t(r) * kTokC);
             layernorm<6>(x, kLnEps);
