@@ -747,11 +747,17 @@ template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, con
             }
             const char* gate = static_cast<const char*>(gd.gate) + (long long)(b)*gd.gate_step;
             if (gd.gate_f32) {
-                resid_tile<true, 2>(gd, gate, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);
+                if (gd.bn == 64) {
+                    resid_tile<true, 2>(gd, gate, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);
+                } else {
+                    resid_tile<true, 1>(gd, gate, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);
+                }
             } else if (gd.bn == 128) {
                 resid_tile<false, 4>(gd, gate, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);
-            } else {
+            } else if (gd.bn == 64) {
                 resid_tile<false, 2>(gd, gate, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);
+            } else {
+                resid_tile<false, 1>(gd, gate, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);
             }
         } else {
             epilogue_tile<E>(g, mo, acc, row0, col0, &ctl->tfull[buf], tpar, &ctl->abort);

@@ -283,20 +283,26 @@ static int encode_rows_store_map(CUtensorMap* m, const void* base, size_t rows, 
     return E_OK;
 }
 
-// The column tile of a GEMM with m rows, n columns and kblocks k-blocks: 256, 128 or 64 (GLU GEMMs whose units have
-// 96 rows: 192 or 96), the one with the least estimated time of the CTA that has most tiles. Measured: with the
+// The column tile of a GEMM with m rows, n columns and kblocks k-blocks: 256, 128, 64 or 32 (GLU GEMMs, whose units have
+// 64 or 96 rows: 256, 128 or 64; 192 or 96), the one with the least estimated time of the CTA that has most tiles. Measured: with the
 // whole grid loading, a k-block arrives at 83 bytes per cycle; an epilogue takes about 18 cycles a column and
 // overlaps the next tile's main loop, except the last one; going from one tile to the next costs some 1500.
 // (Choosing by rounds and width alone gave 256 columns where 13 row tiles x 12 column tiles need two rounds
 // of the grid for 8 tiles, 320 x 5: 2.46 -> 2.28 ms per step, and 128 where that is bound by the loads, 1024 x 5: 5.32 -> 5.04.)
-inline int choose_bn(size_t m, int n, int kblocks, int grid, int max_bn = kMaxBN, int unit = 64) {
-    int best = unit;
+// 32 columns only while half of the grid has no tile even then: a row block waits for twice the arrivals of a GEMM with
+// 64, and its rows are read twice as often (32 x 1: 0.973 -> 0.951 ms per step with this limit, 0.987 without; 256 x 1 with two
+// calls per step 2.311 -> 2.254).
+inline int choose_bn(size_t m, int n, int kblocks, int grid, int max_bn = kMaxBN, int unit = 32) {
+    int best = unit < 64 ? 64 : unit;
     double best_cost = 1e300;
-    for (int bn = 4 * unit; bn >= unit; bn /= 2) {
+    for (int bn = 8 * unit; bn >= unit; bn /= 2) {
         if (n % bn || bn > max_bn) {
             continue;
         }
         const size_t tiles = (m + kBM - 1) / kBM * size_t(n / bn);
+        if (bn < 64 && 2 * tiles > size_t(grid)) {
+            continue;
+        }
         const double kblock = (kStageA + bn * kBK * 2) / 83.0, epi = 18.0 * bn;
         const double cost = double((tiles + grid - 1) / grid) * (std::max(kblocks * kblock, epi) + 1500) + epi;
         if (cost < best_cost) {
@@ -651,9 +657,9 @@ static int make_launch(Launch& L, const Template& t, const Device& dev, const vo
         size_t rows, cols, m; // m: rows of the GEMM's A, for the tile choice
         int n;                // the GEMM's n (per block)
         int max_bn = kMaxBN;  // gated-residual epilogues hold a whole tile's inputs in registers
-        int unit = 64;        // GLU GEMMs: rows of W1 per unit
+        int unit = 32;        // the narrowest tile; GLU GEMMs: rows of W1 per unit
     } bmaps[] = {
-        {TM_B_ST0_W1, IN_ST0_W1, 4 * cs, cs, size_t(N), int(4 * cs)}, {TM_B_ST1_W1, IN_ST1_W1, 4 * cs, cs, size_t(N), int(4 * cs)},
+        {TM_B_ST0_W1, IN_ST0_W1, 4 * cs, cs, size_t(N), int(4 * cs), kMaxBN, 2 * kGluHalf}, {TM_B_ST1_W1, IN_ST1_W1, 4 * cs, cs, size_t(N), int(4 * cs), kMaxBN, 2 * kGluHalf},
         {TM_B_ST0_W2, IN_ST0_W2, cs, 2 * cs, size_t(N), int(cs)}, {TM_B_ST1_W2, IN_ST1_W2, cs, 2 * cs, size_t(N), int(cs)},
         {TM_B_WM1, IN_WM1, nb * kTokMods1 * kTokC, cs, size_t(N), int(nb * kTokMods1 * kTokC)},
         {TM_B_WM2, IN_WM2, nb * 2 * kTokC, cs, size_t(N), int(nb * 2 * kTokC)},
