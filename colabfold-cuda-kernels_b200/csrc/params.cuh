@@ -110,6 +110,7 @@ struct KP {
     uint32_t tc_div_qblocks, tc_div_s;
     uint32_t div_grid;       // the same for the grid
     uint32_t div_n, div_a;   // the same for N and A and rows of all samples; 0: divide
+    int atom_rows, atom_roles; // the same of the atoms, whole groups of four rows; whether the GEMM roles' warps take some
     int tok_rows;             // token rows of a CTA where each takes one contiguous run: cdiv(S·N, grid)
 };
 

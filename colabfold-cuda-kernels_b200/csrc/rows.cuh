@@ -259,6 +259,9 @@ struct FlowRows {
     const unsigned int* cnt;
     unsigned int target;
 };
+__device__ __forceinline__ bool rows_for_roles(int per) {
+    return (per > kWarps - 2 && per <= kWarps + 2) || cdiv(per, kWarps - 2) > cdiv(per, kWarps);
+}
 __device__ __forceinline__ FlowRows flow_rows(const KP& p, int rows, int which, unsigned int gemms_done) {
     FlowRows f;
     // The warps that hold the GEMM roles take rows only where that saves the workers a second or a further one: they
@@ -266,7 +269,7 @@ __device__ __forceinline__ FlowRows flow_rows(const KP& p, int rows, int which, 
     // 2.457 -> 2.430). The two warps without a role come first, the workers, which still have W2's or WO's epilogue to
     // finish, after them; up to kWarps + 2 rows those two alone have a second row.
     const int per = p.tok_rows, w = warp_id();
-    const bool roles = (per > kWarps - 2 && per <= kWarps + 2) || cdiv(per, kWarps - 2) > cdiv(per, kWarps);
+    const bool roles = rows_for_roles(per);
     f.step = roles ? kWarps : kWarps - 2;
     const int aux_first = (w + kWarps - kAuxWarp0) % kWarps; // idle, roles, workers
     const int rank = roles ? (per <= 2 * kWarps ? aux_first : w) : w >= kAuxWarp0 ? w - kAuxWarp0 : w >= kWorkWarp0 ? w : per;
@@ -474,23 +477,31 @@ __device__ __forceinline__ void oct_layernorm(Oct& x, float eps) {
         v.x *= rstd, v.y *= rstd, v.z *= rstd, v.w *= rstd;
     }
 }
-// rows of a range [first, end) go four to a warp step: this lane's row of step i, and how many steps this warp has.
-// The two warps without a role in the GEMMs come first: where there are few rows, the roles' warps get on.
-__device__ __forceinline__ int oct_rank() {
-    return (warp_id() + kWarps - kAuxWarp0) % kWarps;
-}
-__device__ __forceinline__ int oct_row(int first, int i) {
-    return first + 4 * (oct_rank() + kWarps * i) + (lane_id() >> 3);
-}
-__device__ __forceinline__ int oct_steps(int first, int end) {
-    return max(0, cdiv(end - first - 4 * oct_rank(), 4 * kWarps));
+// Rows [first, end) of a CTA go four to a warp step. The two warps without a role in the GEMMs come first: where there
+// are few rows, the roles' warps get on. `roles`: whether those take steps at all (flow_rows, the same rule).
+struct OctRows {
+    int first, end, rank, warps, steps; // this warp's steps: rank, rank + warps, ...
+    __device__ __forceinline__ int row(int i) const { // this lane's row of step i; a lane past the end redoes the last row
+        return min(first + 4 * (rank + warps * i) + (lane_id() >> 3), end - 1);
+    }
+};
+__device__ __forceinline__ OctRows oct_rows(int first, int end, bool roles) {
+    OctRows o;
+    const int w = warp_id(), n = cdiv(end - first, 4);
+    o.first = first, o.end = end, o.warps = roles ? kWarps : kWarps - 2;
+    o.rank = roles ? (w + kWarps - kAuxWarp0) % kWarps : w >= kAuxWarp0 ? w - kAuxWarp0 : w >= kWorkWarp0 ? w : n;
+    o.steps = 0;
+    for (int i = o.rank; i < n; i += o.warps) {
+        o.steps++;
+    }
+    return o;
 }
 
 // AXQ = bf16(LN(qa)·am0 + am1), AXK = bf16(LN(qa)·am2 + am3): the inputs of the q|g and k|v
 // projections (reference: src/diffusion/atom_mlp.cuh:339-364), rows [first, end) by this CTA
-__device__ __forceinline__ void atom_ln_qk_rows(const KP& p, const AtomW& w, int b, int first, int end) {
-    for (int i = 0; i < oct_steps(first, end); i++) {
-        const int r = min(oct_row(first, i), end - 1); // a lane past the end redoes the last row
+__device__ __forceinline__ void atom_ln_qk_rows(const KP& p, const AtomW& w, int b, const OctRows& o) {
+    for (int i = 0; i < o.steps; i++) {
+        const int r = o.row(i);
         const float* am = atom_mods(p, w, b, mod_rows(r, p.A, p.div_a));
         Oct x = oct_load_cg(p.buf.qa + size_t(r) * kAtomC);
         const Oct qs = oct_load(am + AM_Q_SCALE * kAtomC), qb = oct_load(am + AM_Q_BIAS * kAtomC);
@@ -516,9 +527,9 @@ __device__ __forceinline__ void atom_ln_qk_rows(const KP& p, const AtomW& w, int
 // AXHL = [hi | lo] of x = LN(qa)·am4 + am5 with hi = bf16(x), lo = bf16(x - hi): the transition
 // input carried to ~16 mantissa bits (reference: src/diffusion/atom_mlp.cuh:510-517,
 // src/diffusion/frag.cuh:396-406)
-__device__ __forceinline__ void atom_ln_t_rows(const KP& p, const AtomW& w, int b, int first, int end) {
-    for (int i = 0; i < oct_steps(first, end); i++) {
-        const int r = min(oct_row(first, i), end - 1);
+__device__ __forceinline__ void atom_ln_t_rows(const KP& p, const AtomW& w, int b, const OctRows& o) {
+    for (int i = 0; i < o.steps; i++) {
+        const int r = o.row(i);
         const float* am = atom_mods(p, w, b, mod_rows(r, p.A, p.div_a));
         Oct x = oct_load_cg(p.buf.qa + size_t(r) * kAtomC);
         const Oct ts = oct_load(am + AM_T_SCALE * kAtomC), tb = oct_load(am + AM_T_BIAS * kAtomC);
@@ -535,9 +546,9 @@ __device__ __forceinline__ void atom_ln_t_rows(const KP& p, const AtomW& w, int 
     }
 }
 // the encoder's tail: SKIP = qa·QMASK (f32), ABF = bf16(SKIP) (reference: src/diffusion/atom_mlp.cuh:576-591)
-__device__ __forceinline__ void atom_tail_skip_rows(const KP& p, int first, int end) {
-    for (int i = 0; i < oct_steps(first, end); i++) {
-        const int r = min(oct_row(first, i), end - 1);
+__device__ __forceinline__ void atom_tail_skip_rows(const KP& p, const OctRows& o) {
+    for (int i = 0; i < o.steps; i++) {
+        const int r = o.row(i);
         const float m = p.geo.qmask[mod_rows(r, p.A, p.div_a)];
         const Oct x = oct_load_cg(p.buf.qa + size_t(r) * kAtomC);
 #pragma unroll
@@ -550,9 +561,9 @@ __device__ __forceinline__ void atom_tail_skip_rows(const KP& p, int first, int 
     }
 }
 // the decoder's tail: upd = LN(qa·QMASK) @ WUPDᵀ + UPD_B (reference: src/diffusion/atom_mlp.cuh:592-611)
-__device__ __forceinline__ void atom_tail_update_rows(const KP& p, int first, int end) {
-    for (int i = 0; i < oct_steps(first, end); i++) {
-        const int r = min(oct_row(first, i), end - 1);
+__device__ __forceinline__ void atom_tail_update_rows(const KP& p, const OctRows& o) {
+    for (int i = 0; i < o.steps; i++) {
+        const int r = o.row(i);
         const float m = p.geo.qmask[mod_rows(r, p.A, p.div_a)];
         Oct x = oct_load_cg(p.buf.qa + size_t(r) * kAtomC);
 #pragma unroll
@@ -579,10 +590,10 @@ __device__ __forceinline__ void atom_tail_update_rows(const KP& p, int first, in
 // over the 128 channels with the block's scale and offset rows. The reference normalises the f32
 // accumulators inside its fused projection (src/diffusion/atom_mlp.cuh:306-313, :366-392); here the
 // projections are GEMMs with a bf16 epilogue, so this pass reads the rounded q and k.
-__device__ __forceinline__ void atom_qknorm_rows(const KP& p, const AtomW& w, int b, int first, int end) {
+__device__ __forceinline__ void atom_qknorm_rows(const KP& p, const AtomW& w, int b, const OctRows& o) {
     const float* qkn = w.qkn + size_t(b) * kQkNormRows * kAtomC;
-    for (int i = 0; i < oct_steps(first, end); i++) {
-        const int r = min(oct_row(first, i), end - 1);
+    for (int i = 0; i < o.steps; i++) {
+        const int r = o.row(i);
 #pragma unroll
         for (int k = 0; k < 2; k++) {
             bf16* row = (k ? p.buf.akv : p.buf.aqg) + size_t(r) * 2 * kAtomC;
@@ -610,53 +621,54 @@ __device__ __forceinline__ void atom_rows_wait(const KP& p, int which, unsigned 
     }
     __syncwarp();
 }
-__device__ __forceinline__ void atom_rows_report(const KP& p, int sig, int first, int end) {
+__device__ __forceinline__ void atom_rows_report(const KP& p, int sig, const OctRows& o) {
     fence_async_global(); // for TMA reads in other CTAs
     __syncwarp();
     if (lane_id() == 0) {
         unsigned int* cnt = flow_cnt(p, sig);
         fence_acq_rel_gpu();
-        for (int i = 0; i < oct_steps(first, end); i++) {
-            const int r = first + 4 * (oct_rank() + kWarps * i);
-            red_relaxed_add(cnt + r / kBM * kFlowPitch, (unsigned int)(min(4, end - r)));
+        for (int i = 0; i < o.steps; i++) {
+            const int r = o.first + 4 * (o.rank + o.warps * i);
+            red_relaxed_add(cnt + r / kBM * kFlowPitch, (unsigned int)(min(4, o.end - r)));
         }
     }
 }
 #define CCK_ATOM_ROWS_PHASE(wait, gd, gemms, sig, call)                                                                                     \
     do {                                                                                                                                    \
-        const int rows_ = p.S * p.A, per_ = p.flow ? cdiv(cdiv(rows_, int(gridDim.x)), 4) * 4 : 4 * kWarps, items_ = cdiv(rows_, per_);     \
-        for (int it_ = p.flow ? int(blockIdx.x) : d.first(); it_ < items_; it_ += gridDim.x) {                                              \
-            const int f_ = it_ * per_, e_ = min(rows_, f_ + per_);                                                                          \
+        const int rows_ = p.S * p.A, per_ = p.flow ? p.atom_rows : 4 * kWarps;                                                              \
+        const bool roles_ = !p.flow || p.atom_roles;                                                                                        \
+        for (int f_ = (p.flow ? int(blockIdx.x) : d.first()) * per_; f_ < rows_; f_ += int(gridDim.x) * per_) {                             \
+            const OctRows o_ = oct_rows(f_, min(rows_, f_ + per_), roles_);                                                                 \
             if (p.flow) {                                                                                                                   \
-                if (oct_steps(f_, e_) == 0) {                                                                                               \
+                if (o_.steps == 0) {                                                                                                        \
                     break;                                                                                                                  \
                 }                                                                                                                           \
-                atom_rows_wait(p, wait, (gemms) * (unsigned int)(gd_table()[gd].nt * kWorkWarps), f_, e_);                                  \
+                atom_rows_wait(p, wait, (gemms) * (unsigned int)(gd_table()[gd].nt * kWorkWarps), f_, o_.end);                              \
             }                                                                                                                               \
             call;                                                                                                                           \
             if (p.flow && (sig) >= 0) {                                                                                                     \
-                atom_rows_report(p, sig, f_, e_);                                                                                           \
+                atom_rows_report(p, sig, o_);                                                                                               \
             }                                                                                                                               \
         }                                                                                                                                   \
         if (!p.flow) {                                                                                                                      \
-            d.advance(items_);                                                                                                              \
+            d.advance(cdiv(rows_, 4 * kWarps));                                                                                             \
         }                                                                                                                                   \
     } while (0)
 // (epoch: the atom block's running number in the launch)
 __device__ CCK_PHASE_FN void atom_ln_qk(const KP& p, Deal& d, const AtomW& w, int b, unsigned int epoch) {
-    CCK_ATOM_ROWS_PHASE(FC_AC2, GD_ENC_W2, epoch, FC_AX, atom_ln_qk_rows(p, w, b, f_, e_));
+    CCK_ATOM_ROWS_PHASE(FC_AC2, GD_ENC_W2, epoch, FC_AX, atom_ln_qk_rows(p, w, b, o_));
 }
 __device__ CCK_PHASE_FN void atom_ln_t(const KP& p, Deal& d, const AtomW& w, int b, unsigned int epoch) {
-    CCK_ATOM_ROWS_PHASE(FC_AC1, GD_ENC_WO, epoch + 1, FC_AXT, atom_ln_t_rows(p, w, b, f_, e_));
+    CCK_ATOM_ROWS_PHASE(FC_AC1, GD_ENC_WO, epoch + 1, FC_AXT, atom_ln_t_rows(p, w, b, o_));
 }
 __device__ CCK_PHASE_FN void atom_qknorm(const KP& p, Deal& d, const AtomW& w, int b) {
-    CCK_ATOM_ROWS_PHASE(FC_AC2, GD_ENC_W2, 0u, -1, atom_qknorm_rows(p, w, b, f_, e_));
+    CCK_ATOM_ROWS_PHASE(FC_AC2, GD_ENC_W2, 0u, -1, atom_qknorm_rows(p, w, b, o_));
 }
 __device__ CCK_PHASE_FN void atom_tail_skip(const KP& p, Deal& d, unsigned int epoch) {
-    CCK_ATOM_ROWS_PHASE(FC_AC2, GD_ENC_W2, epoch + 1, -1, atom_tail_skip_rows(p, f_, e_));
+    CCK_ATOM_ROWS_PHASE(FC_AC2, GD_ENC_W2, epoch + 1, -1, atom_tail_skip_rows(p, o_));
 }
 __device__ CCK_PHASE_FN void atom_tail_update(const KP& p, Deal& d, unsigned int epoch) {
-    CCK_ATOM_ROWS_PHASE(FC_AC2, GD_ENC_W2, epoch + 1, -1, atom_tail_update_rows(p, f_, e_));
+    CCK_ATOM_ROWS_PHASE(FC_AC2, GD_ENC_W2, epoch + 1, -1, atom_tail_update_rows(p, o_));
 }
 
 // qa = (skip + tb[token of a])·QMASK (reference: src/diffusion/rows.cuh:246-261)

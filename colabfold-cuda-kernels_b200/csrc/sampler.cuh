@@ -550,6 +550,7 @@ extern "C" __global__ void __launch_bounds__(cck::kThreads, 1) cck_sampler_kerne
             w.div_grid = div_magic(gridDim.x);
             w.div_n = div_magic_rows(w.N, w.S * w.N), w.div_a = div_magic_rows(w.A, (unsigned long long)(w.S) * w.A);
             w.tok_rows = cdiv(w.S * w.N, int(gridDim.x));
+            w.atom_rows = cdiv(cdiv(w.S * w.A, int(gridDim.x)), 4) * 4, w.atom_roles = rows_for_roles(w.atom_rows / 4);
         }
         __syncthreads();
     }

@@ -479,6 +479,33 @@ def test_masked_bucket(lib, oracle_lib):
     assert driver.max_rel_err(lib.read("POS"), pos) > 1e-4
 
 
+@pytest.mark.parametrize("n_tok,samples", [(24, 1), (300, 5), (416, 5), (592, 2)])
+def test_row_dealing_matches_barriers(lib, make_case, n_tok, samples):
+    """On completion counters a CTA takes one run of token rows and one of atom rows, and whether the warps of
+    the GEMM roles take some depends on how many there are: 1, 11, 15 and 8 token rows per CTA of 148, 4 to
+    116 atom rows, and a last block of rows that some lane quarters of the GEMM epilogues have no part in. On
+    barriers rows are dealt in another way; positions are bit-identical."""
+    x, meta = make_case(n_tok, samples, 8, False)
+    lib.setup(x, meta)
+    xn = synth.noisy_positions(meta, mg.T_ONCE)
+    got = {}
+    try:
+        for on in (True, False):
+            lib.set_flow(on)
+            lib.run(mode=1, xn=xn, t=mg.T_ONCE)
+            got[on] = lib.read("OUT").copy()
+    finally:
+        lib.set_flow(True)
+    assert np.isfinite(got[True]).all()
+    assert np.array_equal(got[True], got[False])
+
+
+@pytest.mark.parametrize("shape", [(32, 768, 768, 0), (77, 64, 128, 0), (384, 768, 1536, 0), (385, 768, 768, 0)])
+def test_gemm_door_of_few_tiles(lib, oracle_lib, shape):
+    """Column tiles of 32 while half of the grid has no tile (the last shape is just past that), with a partial row tile."""
+    test_gemm_door(lib, oracle_lib, shape)
+
+
 def test_pipelines_of_the_token_attention_do_not_depend_on_their_skew(lib, make_case):
     """The token attention keeps two items in flight per CTA as independent pipelines; whatever their
     relative timing, a fold's result is the same bit for bit. The test hook delays the second pipeline
