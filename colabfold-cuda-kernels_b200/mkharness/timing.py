@@ -3,8 +3,9 @@ barrier to grid barrier, sampled by CTA 0, summed per kind of phase.
 
     python -m mkharness.timing [--tokens 512] [--samples 5] [--nsteps 200] [--barriers]
 
---barriers: every operation of a token block ends at a grid barrier (the reference's schedule), which
-splits the block's time by operation; the default runs the blocks on completion counters.
+--barriers: every operation ends at a grid barrier (the reference's schedule), which splits the time by
+operation; the default runs on completion counters: T_OUT's first phase holds all token blocks, A_W2 an atom
+block's chain from WO to the next projections.
 Run from colabfold-cuda-kernels_b200/ (or with it on PYTHONPATH).
 """
 import argparse

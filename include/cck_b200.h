@@ -91,8 +91,8 @@ int mk_set_extent(int N, int NS);
  * flags (not an operator flag) asks for the form on completion counters that mk_set_flow(1) runs.
  * No counterpart in the reference's debug API. */
 int mk_program(int mode, int nsteps, int flags, unsigned char* ops, int max_ops);
-/* 1 (default): a token block runs as one phase (QKVG -> attention -> WO -> adaLN -> W1 -> W2 -> the next
- * block's adaLN), a unit waiting for completion counters of the units it reads; 0: every operation
+/* 1 (default): the token blocks run as one phase, an atom block's chain from its attention to the next
+ * projections as another, a unit waiting for completion counters of the units it reads; 0: every operation
  * ends at a grid barrier as in the reference's schedule (src/diffusion/sampler.cuh:99-134), which the
  * per-kind timing record and dbg_stop count (mk_run with dbg_stop > 0 always runs on barriers). Same
  * results either way. Returns the previous setting. No counterpart in the reference's debug API. */
