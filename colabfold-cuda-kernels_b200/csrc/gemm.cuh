@@ -826,7 +826,7 @@ __device__ __forceinline__ void ring_layout(SmemCtl* ctl, uint32_t ring, int bn)
 // then come from HBM. Where few row tiles share a weight tile, within microseconds, the weights are marked as
 // the first to leave: 1.20 -> 1.11 ms per step at 32 x 1, 1.37 -> 1.34 at 61 x 5. With many row tiles that
 // loses the weights between two of them (5.37 -> 5.51 ms at 1024 x 5; with 24 for the limit, 16 to 20 row tiles
-// read 0.3 GB per step more from HBM than with 8: 512 x 5 2.440 -> 2.417, 391 x 5 2.230 -> 2.200). 2, 4, 8 and 12 are alike.
+// read 0.5 GB per step more from HBM than with 8: 512 x 5 2.440 -> 2.417, 391 x 5 2.230 -> 2.200). 2, 4, 8 and 12 are alike.
 constexpr int kOnceRowTiles = 8;
 __device__ __forceinline__ uint64_t weights_policy(const GemmDesc& gd) {
     return l2_policy(uni(gd.mt) <= kOnceRowTiles);
