@@ -62,14 +62,16 @@ struct Template {
     int S, Nb, NSb, nsteps;
     uint32_t flags;
     int steps, cs, nb, tw1, aw1, nk, plc, plx, np, flow_n, flow_na;
+    bool flow; // the layout has room for completion counters and what runs on them
     size_t off[kNumBufs], bytes[kNumBufs];
     size_t total;
 };
 
-// widths from byte sizes (reference: src/diffusion/host.cuh:74-89), then every size is checked
-static int make_template(Template& t, int S, int Nb, int NSb, int nsteps, uint32_t flags, const size_t* in) {
+// widths from byte sizes (reference: src/diffusion/host.cuh:74-89), then every size is checked. flow = false: the layout of a
+// run on grid barriers, which needs less (no second QKVG and VT, no counters) and gives the same results
+static int make_template(Template& t, int S, int Nb, int NSb, int nsteps, uint32_t flags, const size_t* in, bool flow = true) {
     t = Template{};
-    t.S = S, t.Nb = Nb, t.NSb = NSb, t.nsteps = nsteps, t.flags = flags;
+    t.S = S, t.Nb = Nb, t.NSb = NSb, t.nsteps = nsteps, t.flags = flags, t.flow = flow && flow_allowed(flags);
     if (flags & ~(kReferenceFlagBits | kExtensionFlagBits)) {
         return fail(E_FLAGS, "MkSample: flags " + std::to_string(flags) + " set bits that no variant uses");
     }
@@ -177,8 +179,8 @@ static int make_template(Template& t, int S, int Nb, int NSb, int nsteps, uint32
     want[B_VT] = size_t(S) * kTokC * t.np * h;
     t.flow_n = int(cdiv(int(rt), kBM)) + 1;
     t.flow_na = int(cdiv(int(ra), kBM));
-    want[B_FLOW] = (size_t(kFlowTok) * t.flow_n + size_t(kFlowAtom) * t.flow_na) * kFlowPitch * sizeof(unsigned int);
-    if (flow_allowed(flags)) { // the second buffers of the token blocks' chains
+    if (t.flow) { // the counters, and the second buffers of the token blocks' chains
+        want[B_FLOW] = (size_t(kFlowTok) * t.flow_n + size_t(kFlowAtom) * t.flow_na) * kFlowPitch * sizeof(unsigned int);
         want[B_QKVG2] = want[B_QKVG], want[B_VT2] = want[B_VT];
     }
     size_t off = align_up(sizeof(Control), kAlign);
@@ -570,7 +572,7 @@ static int make_launch(Launch& L, const Template& t, const Device& dev, const vo
     p.cs = t.cs, p.nb = t.nb, p.tw1 = t.tw1, p.aw1 = t.aw1, p.nk = t.nk, p.plc = t.plc, p.plx = t.plx;
     p.ln_eps = t.flags & F_IDSCALE ? kIdScaleEps : kLnEps;
     p.flags = t.flags, p.ext = ext, p.out = out, p.out_tokens = t.Nb;
-    p.flow = g_flow && flow_allowed(t.flags), p.flow_n = t.flow_n, p.flow_na = t.flow_na;
+    p.flow = g_flow && t.flow, p.flow_n = t.flow_n, p.flow_na = t.flow_na;
     p.attn_skew = g_attn_skew, p.wait_cycles = g_wait_cycles > 0 ? g_wait_cycles : kWaitCycles, p.barrier_extra = g_barrier_extra;
     auto F = [&](int i) { return static_cast<const float*>(in[i]); };
     auto H = [&](int i) { return static_cast<const bf16*>(in[i]); };
@@ -698,6 +700,19 @@ static int enqueue(const Launch& L, const Device& dev, cudaStream_t st) {
         return fail(E_LAUNCH, std::string("MkSample: ") + cudaGetErrorString(err));
     }
     return E_OK;
+}
+// a whole sampling run on buffers of the caller's: ws holds t.total bytes
+static int enqueue_sample(const Template& t, const void* const* in, float* out, const int* ext, void* ws, void* stream) {
+    Device dev;
+    if (int e = device_state(dev)) {
+        return e;
+    }
+    Launch L;
+    if (int e = make_launch(L, t, dev, in, static_cast<char*>(ws), out, ext)) {
+        return e;
+    }
+    L.kp.mode = 0;
+    return enqueue(L, dev, static_cast<cudaStream_t>(stream));
 }
 
 } // namespace cck

@@ -56,8 +56,10 @@ const char* cck_last_error(void);
  * cudaMalloc is refused there, so such a caller has no way to make scratch. This variant uses a
  * fixed 32 MiB scratch array that the library keeps in device memory on every GPU that loads it.
  * Arguments and result are those of cck_mk_sample without ws / ws_bytes. It allocates nothing.
- *  - A fold whose scratch exceeds cck_static_workspace_bytes() is refused with CCK_E_WORKSPACE
- *    (the message names both sizes): small folds only, e.g. 32 tokens x 1 sample.
+ *  - Small folds only. One whose mk_workspace_bytes exceeds cck_static_workspace_bytes() runs on grid
+ *    barriers, which takes less scratch and gives the same results (mk_set_flow); one that does not
+ *    fit in that way either is refused with CCK_E_WORKSPACE (the message names the sizes). At 8 atoms a
+ *    token the largest are 68 tokens x 1 sample, 48 x 5 and 20 x 16 (on counters 65, 45 and 16).
  *  - The first call on a device looks up the array's device address; make it outside any capture.
  *  - All calls on a device share the array. Calls ordered on a stream are independent (the control
  *    words are cleared at the start of each call, everything else is written before it is read);

@@ -3,6 +3,8 @@ error paths that are decided before any device call."""
 import ctypes
 import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -152,3 +154,33 @@ def test_operator_errors_before_any_device_work(lib, tiny_sizes):
     bad = (ctypes.c_size_t * 74)(*sizes)
     bad[synth.IN["ENC_W2"]] += 2
     assert lib.cck_mk_sample(None, None, ptrs, bad, 74, None, meta["N"], None, 1 << 40, 1, 20, 0) == 3
+
+
+@pytest.mark.parametrize("tokens,samples", [(68, 1), (48, 5), (20, 16), (12, 24)])
+@pytest.mark.parametrize("flags", [0, synth.F_HEUN, synth.F_PARALLEL, synth.F_QKNORM])
+def test_static_scratch_takes_what_fits_on_barriers(product_lib_path, make_case, tokens, samples, flags):
+    """The operator without a workspace runs a fold whose full layout (with completion counters) does not fit its
+    built-in scratch on grid barriers: it is not refused for its size. Asked in a process that sees no
+    device, so that nothing can be launched: the answer is then CCK_E_DEVICE (6), not CCK_E_WORKSPACE (2). Twice the
+    samples are refused, with the sizes in the message. PARALLEL and QKNORM folds, which never run on
+    counters, have room for none."""
+    x, meta = synth.pad_to_bucket(*make_case(8 if tokens < 32 else 32, 1, 20, True), tokens, tokens // 4)
+    sizes = [a.nbytes for a in x]
+    code = """
+import ctypes
+lib = ctypes.CDLL(%r)
+lib.mk_workspace_bytes.restype = lib.cck_static_workspace_bytes.restype = ctypes.c_size_t
+lib.cck_last_error.restype = ctypes.c_char_p
+sizes = (ctypes.c_size_t * 74)(*%r)
+for s in (%d, %d):
+    rc = lib.cck_mk_sample_static(None, None, (ctypes.c_void_p * 74)(), sizes, 74, None, %d, s, 20, %d)
+    print(rc, lib.mk_workspace_bytes(s, %d, %d, 20, %d, sizes), lib.cck_static_workspace_bytes(), lib.cck_last_error().decode(), sep="|")
+""" % (product_lib_path, sizes, samples, 2 * samples, tokens, flags, tokens, tokens // 4, flags)
+    env = dict(os.environ, CUDA_VISIBLE_DEVICES="")
+    run = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env=env, timeout=300)
+    assert run.returncode == 0, run.stderr
+    fits, twice = [line.split("|", 3) for line in run.stdout.splitlines()]
+    if flags in (0, synth.F_HEUN):
+        assert int(fits[1]) > int(fits[2]), "a fold that fits with its counters does not show this"
+    assert int(fits[0]) == 6, fits
+    assert int(twice[0]) == 2 and twice[1] in twice[3] and twice[2] in twice[3], twice

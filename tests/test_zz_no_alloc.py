@@ -81,3 +81,34 @@ def test_static_workspace_entry_point_matches_the_ordinary_one(product_lib_path,
     assert "built-in scratch holds %d" % (32 << 20) in msg and str(big) in msg
     torch.cuda.synchronize()
     assert float(out64.abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("tokens,samples", [(68, 1), (48, 5), (20, 16)])
+def test_static_workspace_of_a_fold_that_fits_on_barriers_only(product_lib_path, make_case, tokens, samples):
+    """Folds whose full layout (with completion counters) exceeds the built-in scratch run in it on grid barriers: the
+    positions of the ordinary entry point, bit for bit, whatever an earlier call left in the array."""
+    import torch
+
+    lib = ctypes.CDLL(product_lib_path)
+    lib.cck_last_error.restype = ctypes.c_char_p
+    lib.mk_workspace_bytes.argtypes = [ctypes.c_int] * 5 + [ctypes.c_void_p]
+    lib.mk_workspace_bytes.restype = lib.cck_static_workspace_bytes.restype = ctypes.c_size_t
+    lib.cck_mk_sample.argtypes = ARGS + [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_int, ctypes.c_int]
+    lib.cck_mk_sample_static.argtypes = ARGS + [ctypes.c_int, ctypes.c_int, ctypes.c_int]
+    x, meta = make_case(tokens, 1, 8, False)
+    dev = [torch.from_numpy(a.view(np.uint8).reshape(-1).copy()).cuda() for a in x]
+    ptrs = (ctypes.c_void_p * 74)(*[t.data_ptr() for t in dev])
+    sizes = (ctypes.c_size_t * 74)(*[a.nbytes for a in x])
+    ext = torch.tensor([tokens, meta["NS"], 1, 21, 0], dtype=torch.int32, device="cuda")
+    stream, steps = torch.cuda.current_stream().cuda_stream, 3
+    need = lib.mk_workspace_bytes(samples, tokens, meta["NS"], steps, 0, sizes)
+    assert need > lib.cck_static_workspace_bytes()
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    want, got = (torch.zeros((samples, tokens, 24, 3), dtype=torch.float32, device="cuda") for _ in range(2))
+    assert lib.cck_mk_sample(stream, ext.data_ptr(), ptrs, sizes, 74, want.data_ptr(), tokens, ws.data_ptr(), need, samples, steps, 0) == 0
+    for _ in range(2):
+        rc = lib.cck_mk_sample_static(stream, ext.data_ptr(), ptrs, sizes, 74, got.data_ptr(), tokens, samples, steps, 0)
+        assert rc == 0, lib.cck_last_error()
+        torch.cuda.synchronize()
+        assert torch.isfinite(want).all() and torch.equal(got, want)
+        got.zero_()
