@@ -579,3 +579,93 @@ def test_waits_give_up_and_the_launch_ends(lib, make_case):
         wt(0, 0)
     lib.run(mode=0, nsteps=2, seed=3)
     assert np.array_equal(lib.read("POS"), want)
+
+
+def outgrown_reference_logits(n, rng):
+    """PLX rows by class of query row: flat; one later chunk of 64 keys far above the others; a ramp up, every chunk far
+    above the one before; a ramp down; a step of 4.5 (the maximum grows by 2^6.5, but the chunk adds up to more than 2^8).
+    Every fourth group of 32 rows (a softmax warp) is flat throughout."""
+    chunk, chunks = np.arange(n) // 64, (n + 63) // 64
+    x = rng.standard_normal((n, n)).astype(np.float32)
+    for q in range(n):
+        if q // 32 % 4 == 3:
+            continue
+        at = 1 + q // 5 % (chunks - 1)
+        x[q] += [0 * chunk, 60 * (chunk == at), 25 * chunk, -25 * chunk, 4.5 * (chunk >= at)][q % 5]
+    return synth.to_bf16(x)
+
+
+def check_token_attention(lib, n, samples, min_repeats):
+    """TO of the first token block against softmax(q·k + pair logits)·v ⊙ g in 64 bits on the kernel's own q, k, v, gates
+    and pair logits. Per element: P is rounded to bf16 (2^-8 of each summand of P·V) and so is the result (2^-8); f32
+    sums, the exponential's approximation and the rounding of scores of up to 2^8 in f32 stay below 2^-13."""
+    np_ = (n + 63) // 64 * 64
+    qkvg = lib.read("QKVG").astype(np.float64).reshape(samples, n, 4, 16, 48)
+    plg = lib.read("PLG").reshape(-1, np_, np_)[:16, :n, :n].astype(np.float64)
+    got = lib.read("TO").reshape(samples, n, 16, 48)
+    repeats = 0
+    for s in range(samples):
+        for h in range(16):
+            q, k, v, g = (qkvg[s, :, i, h] for i in range(4))
+            x = q @ k.T * (np.log2(np.e) / np.sqrt(48)) + plg[h]
+            p = np.exp2(x - x.max(1, keepdims=True))
+            p /= p.sum(1, keepdims=True)
+            want = p @ v * g
+            bound = (2.0 ** -8 + 2.0 ** -13) * (p @ np.abs(v) * g + np.abs(want)) + 1e-30
+            err = np.abs(got[s, :, h] - want) / bound
+            assert np.isfinite(got[s, :, h]).all() and err.max() <= 1.0, (s, h, np.unravel_index(err.argmax(), err.shape), err.max())
+            ref = np.full(n, -np.inf)  # how often the kernel's rule sends a warp through a chunk again
+            for c in range(0, np_, 64):
+                for w in range(0, n, 32):
+                    rows, keys = slice(w, min(w + 32, n)), slice(c, min(c + 64, n))
+                    with np.errstate(over="ignore"):
+                        over = c and (np.exp2(x[rows, keys] - ref[rows, None]).sum(1) > 256).any()
+                    repeats += bool(over)
+                    if over or not c:
+                        ref[rows] = np.maximum(ref[rows], x[rows, keys].max(1))
+    share = repeats / (samples * 16 * ((n + 31) // 32) * (np_ // 64 - 1))
+    assert share >= min_repeats, share
+
+
+@pytest.mark.parametrize("n_tok,samples,masked", [(192, 1, 0), (200, 2, 0), (512, 1, 0), (192, 1, 64), (192, 2, 100)])
+def test_token_attention_when_later_chunks_outgrow_the_first(lib, oracle_lib, make_case, n_tok, samples, masked):
+    """The token attention takes a row's exponentials against a reference value from the row's first chunk of keys, and
+    repeats a chunk's pass, with O and the row sum rescaled, where that has been outgrown. Here that is the rule:
+    by extra pair logits (in one chunk for some rows, in all for others, in none for a whole warp here and there), or
+    because the first keys of a 256-token bucket are masked, all 64 of the first chunk or more, and no real key is in
+    it. Each row against 64 bits within a derived bound, TO and the denoiser's output against the oracle, and the
+    output on completion counters bit for bit that on barriers."""
+    x, meta = make_case(n_tok, samples, 8, False)
+    x = [a.copy() for a in x]
+    # no pair representation: the pair logits are sums of given numbers, rounded alike by kernel and oracle (a logit of
+    # 64 is rounded to 0.5, and a tie decided differently is no error of the attention's)
+    x[synth.IN["PC"]][:] = 0
+    x[synth.IN["PCS"]][..., 0] = 0
+    if masked:
+        x, meta = synth.pad_to_bucket(x, meta, 256, 64)
+        x[synth.IN["TMASK"]][:masked] = 0
+    else:
+        x[synth.IN["PLX"]] = outgrown_reference_logits(n_tok, np.random.default_rng(n_tok))
+    lib.setup(x, meta)
+    oracle_lib.setup(x, meta)
+    xn = synth.noisy_positions(meta, mg.T_ONCE)
+    stop, _ = mg.STOPS["tok0_attn"]
+    oracle_lib.clear_snapshots()
+    oracle_lib.snapshot(stop, "TO")
+    oracle_lib.run(mode=1, xn=xn, t=mg.T_ONCE)
+    lib.run(mode=1, dbg_stop=stop, xn=xn, t=mg.T_ONCE)
+    check_token_attention(lib, meta["N"], samples, 1 / 3 if masked else 0.6)
+    err = driver.max_rel_err(lib.read("TO"), oracle_lib.read("TO@%d" % stop))
+    oracle_lib.clear_snapshots()
+    out = {}
+    try:
+        for on in (True, False):
+            lib.set_flow(on)
+            lib.run(mode=1, xn=xn, t=mg.T_ONCE)
+            out[on] = lib.read("OUT").copy()
+    finally:
+        lib.set_flow(True)
+    assert np.array_equal(out[True], out[False])
+    err_out = driver.max_rel_err(out[True], oracle_lib.read("OUT"))
+    print("N=%d S=%d masked=%d: TO vs oracle %.2e, OUT vs oracle %.2e" % (n_tok, samples, masked, err, err_out))
+    assert err <= BF16_TOL and err_out < GATE
