@@ -194,11 +194,9 @@ __device__ CCK_PHASE_FN void sc_prep(const KP& p, Deal& d) {
 __device__ __forceinline__ const bf16* tok_mods(const KP& p, int b, int slot) {
     return p.buf.mods + (size_t(b) * kTokModSlots + slot) * p.N * kTokC;
 }
-// TX = bf16(LN(act)·mods[slot] + mods[slot+1]) (reference: src/diffusion/rows.cuh:270-285).
-// A warp keeps two rows in flight: all loads of both rows are issued before the first reduction.
-#ifndef CCK_ADALN_ROWS
-#define CCK_ADALN_ROWS 1
-#endif
+// TX = bf16(LN(act)·mods[slot] + mods[slot+1]) (reference: src/diffusion/rows.cuh:270-285). A warp takes one row at a
+// time, all of its loads issued before the first reduction: a second row in flight costs registers that the
+// kernel does not have.
 struct AdaRow {
     RowV<6> x;
     uint2 s[6], o[6];
@@ -306,26 +304,11 @@ __device__ CCK_HOT_FN void token_adaln(const KP& p, Deal& d, int b, int slot, un
         }
         return;
     }
-#if CCK_ADALN_ROWS == 1
     for (int r = row_first(d); r < rows; r += step) {
         AdaRow a0;
         adaln_load(a0, p, ms, mo, r);
         adaln_finish(a0, p, r);
     }
-#else
-    for (int r = row_first(d); r < rows; r += 2 * step) {
-        AdaRow a0, a1;
-        const bool two = r + step < rows;
-        adaln_load(a0, p, ms, mo, r);
-        if (two) {
-            adaln_load(a1, p, ms, mo, r + step);
-        }
-        adaln_finish(a0, p, r);
-        if (two) {
-            adaln_finish(a1, p, r + step);
-        }
-    }
-#endif
     rows_done(d, rows);
 }
 // QKNORM: LayerNorm of q and of k over their 768 flattened channels with the block's scale and
