@@ -2,7 +2,7 @@
 // tensor cores. Per CTA: one warp feeds a shared-memory ring with TMA tile loads, one warp issues
 // tcgen05.mma into a double-buffered TMEM accumulator (2 x 256 columns), and eight warps drain finished
 // accumulators with tcgen05.ld and apply the fused epilogue, so the epilogue of tile i overlaps the main
-// loop of tile i+1. Tiles are 128 x bn (bn = 64..256) x 64.
+// loop of tile i+1. Tiles are 128 x bn (bn = 32..256) x 64.
 // A main loop runs at the rate of its MMAs when both roles issue from warp-uniform code (ptx.cuh): measured
 // inside the kernel, a k-block went from some 590 cycles at any width to 265 (bn = 128) and 525 (bn = 256).
 //

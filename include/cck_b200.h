@@ -127,9 +127,10 @@ int mk_set_wait_test(long long cycles, int extra);
 int mk_wait_test(long long cycles, float* ms);
 int mk_philox_test(uint32_t idx, uint32_t step, uint32_t sample, uint32_t stream, uint64_t seed, uint32_t* words, float* z);
 
-/* Status word of the last mk_run: 0 ok, 1 grid barrier gave up, 2 a pipeline wait gave up,
- * 3 unsupported extent; and how many grid barriers the run passed. No counterpart in the reference,
- * whose barriers are unbounded. */
+/* Status word of the last mk_run: 0 ok, 1 a grid barrier gave up, 2 a wait inside a phase gave up; where it
+ * stood (grid barriers passed); and the arrivals at the grid's barrier word per CTA: its barriers, and on completion
+ * counters also the ends of operations that are only counted there. No counterpart in the reference, whose
+ * barriers are unbounded. */
 void cck_last_status(unsigned int* status, unsigned int* where, unsigned int* barriers);
 
 #ifdef __cplusplus

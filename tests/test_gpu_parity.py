@@ -117,7 +117,7 @@ def test_status_words_after_a_clean_run(case, lib):
     lib.run(mode=1, xn=xn, t=mg.T_ONCE)
     st, where, bars = ctypes.c_uint(9), ctypes.c_uint(9), ctypes.c_uint(0)
     lib.lib.cck_last_status(ctypes.byref(st), ctypes.byref(where), ctypes.byref(bars))
-    assert st.value == 0 and bars.value > 60  # one denoiser call: 2 barriers per token block on completion counters (7 without), ~25 around them
+    assert st.value == 0 and bars.value > 60  # one denoiser call on completion counters: 23 barriers, and 54 ends of operations that are only counted
 
 
 def test_operator_entry_point_matches_debug_api(lib, make_case):
@@ -299,7 +299,7 @@ def test_real_extents_inside_a_larger_bucket(lib, make_case):
 
 @pytest.mark.parametrize("n_tok,samples", [(160, 3), (256, 2)])
 def test_completion_counters_match_barriers(lib, make_case, n_tok, samples):
-    """Inside a token block QKVG -> attention -> WO and W1 -> W2 run without grid barriers, a unit
+    """The token blocks, and an atom block from its attention to the next projections, run without grid barriers, a unit
     waiting for the completion counters of the rows it reads (mk_set_flow, on by default). The same
     units compute the same values in another order: positions are bit-identical to the run on
     barriers. 160 tokens: samples do not start on a 128-row block, so blocks of rows and blocks of

@@ -78,7 +78,7 @@ def test_unsupported_flags_are_refused(lib, tiny_sizes):
     assert heun >= plain + meta["S"] * meta["N"] * 24 * 3 * 4
 
 
-END_NONE, END_SUB, END_PHASE = 0, 1, 2
+END_NONE, END_SUB, END_PHASE, END_ARRIVE = 0, 1, 2, 3
 
 
 def program(lib, mode, nsteps, flags):
@@ -115,11 +115,11 @@ def test_phase_program(lib):
 
 
 def test_flow_program(lib):
-    """With the program writer's flow bit the token block has one barrier instead of seven, after the
-    adaLN pass that opens it: QKVG, attention, WO, the transition's adaLN, W1, W2 and the next block's
-    adaLN share a phase (units and rows wait for completion counters). The attention is bracketed by
-    CTA-level syncs because it restages shared memory, and one more stands before W1, whose tiles
-    fill the ring slots that WO's epilogue borrows. PARALLEL and QKNORM blocks stay on barriers."""
+    """With the program writer's flow bit the token block has no barrier instead of seven: all blocks share
+    a phase (units and rows wait for completion counters), and the end of the adaLN pass that opens a block is only
+    counted at the barrier word. The attention is bracketed by CTA-level syncs because it restages shared memory;
+    the third operation of that kind, before W1, marks a place where the roles need not rejoin. PARALLEL and QKNORM
+    blocks stay on barriers."""
     PROG_FLOW = 1 << 30
     base = program(lib, 0, 5, 0)
     flow = program(lib, 0, 5, PROG_FLOW)
@@ -132,6 +132,7 @@ def test_flow_program(lib):
         return sub[int(sub[loop_at, 1]) - (end + 1):loop_at]
     b0, b1 = body(base), body(flow)
     assert int(((b0[:, 3] & 3) != 0).sum()) == 7 and int(((b1[:, 3] & 3) != 0).sum()) == 1
+    assert int((b1[:, 3] & 3).max()) == END_ARRIVE and all((b0[:, 3] & 3) == END_PHASE)
     assert int((b1[:, 0] == fn_cta_sync).sum()) == 3
     work = lambda b: [tuple(int(v) for v in o[:3]) for o in b if int(o[0]) != fn_cta_sync]
     assert work(b0) == work(b1), "the same operations in the same order"
