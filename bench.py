@@ -52,7 +52,7 @@ def measured_peaks():
     if os.path.isfile(path):
         p = json.load(open(path))
         return float(p["bf16_tflops_sustained"]), float(p["hbm_gbs"]), "measured (MEASURED_PEAKS.json, sustained cuBLAS bf16)"
-    return 1400.0, 6650.0, "fallback (earlier measurement on this pool, sustained)"
+    return 1400.0, 6650.0, "fallback (an earlier measurement, sustained)"
 
 
 class ClockSampler:

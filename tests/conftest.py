@@ -12,7 +12,7 @@ for p in (PKG, ROOT):
 
 
 def pytest_configure(config):
-    config.addinivalue_line("markers", "gpu: needs a B200; run with -m gpu on the GPU box")
+    config.addinivalue_line("markers", "gpu: needs a B200; run with -m gpu where there is one")
 
 
 @pytest.fixture(scope="session")

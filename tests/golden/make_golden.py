@@ -1,6 +1,6 @@
 """Generates the golden fixtures of the sampler from the reference's own CUDA kernel.
 
-Run on a GPU box (the reference kernel needs a GPU):
+Run where there is a GPU (the reference kernel needs one):
     python tests/golden/make_golden.py <output dir> [case ...]
 It loads oracle/_ref/libref_sm100.so (the reference's diffusion.cu compiled unmodified for sm_100 by
 oracle/Makefile), drives it through its ctypes API on seeded synthetic inputs, and stores the buffers

@@ -61,7 +61,7 @@ def test_denoiser_checkpoints(case, oracle_lib):
     assert worst["atom_init.QA"] <= EXACT_TOL and worst["atom_init.NTV"] <= EXACT_TOL, worst
     bad = {k: v for k, v in worst.items() if v > BF16_TOL}
     assert not bad, bad
-    # the gate of the north star: one denoiser evaluation within 2e-2
+    # the stated gate: one denoiser evaluation within 2e-2
     assert worst["final.OUT"] < 2e-2
 
 
