@@ -1,7 +1,7 @@
 """Per-phase-kind timing of one fold from the library's own record (no profiler): wall time from grid
 barrier to grid barrier, sampled by CTA 0, summed per kind of phase.
 
-    python -m mkharness.timing [--tokens 512] [--samples 5] [--nsteps 200] [--barriers]
+    python -m mkharness.timing [--tokens 512] [--samples 5] [--nsteps 200] [--flags 0] [--barriers]
 
 --barriers: every operation ends at a grid barrier (the reference's schedule), which splits the time by
 operation; the default runs on completion counters: T_OUT's first phase holds all token blocks, A_W2 an atom
@@ -18,10 +18,11 @@ def main():
     ap.add_argument("--tokens", type=int, default=512)
     ap.add_argument("--samples", type=int, default=5)
     ap.add_argument("--nsteps", type=int, default=200)
+    ap.add_argument("--flags", type=int, default=0, help="variant bits")
     ap.add_argument("--barriers", action="store_true")
     ap.add_argument("--lib", default=driver.PRODUCT_LIB)
     a = ap.parse_args()
-    x, meta = synth.make_inputs(a.tokens, samples=a.samples, steps=max(a.nsteps, 1), seed=0)
+    x, meta = synth.make_inputs(a.tokens, samples=a.samples, steps=max(a.nsteps, 1), seed=0, flags=a.flags)
     lib = driver.MkLib(a.lib)
     lib.setup(x, meta)
     lib.set_flow(not a.barriers)
