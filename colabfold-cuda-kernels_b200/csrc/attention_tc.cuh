@@ -424,6 +424,8 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                 // The chunk's P buffer held P of chunk g - 2. That chunk's P·V was issued before this chunk's
                 // Q·Kᵀ, by the same warp, and the commit behind s_full covers everything issued before it:
                 // having seen S, the buffer is free.
+                // (rounded once, as the pass rounds score - m: where all logits are masked ones, -1.4e9 with a step of 128, a
+                // product rounded by itself could go to the other neighbour and leave an exponential of 2^128)
                 auto row_max = [&]() {
                     float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll 1
@@ -437,7 +439,8 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
                             const uint32_t w[4] = {bw.x, bw.y, bw.z, bw.w};
 #pragma unroll
                             for (int k = 0; k < 4; k++) {
-                                const float2 x = add_bf2(w[k], __fmul2_rn(make_float2(__uint_as_float(sr[8 * jj + 2 * k]), __uint_as_float(sr[8 * jj + 2 * k + 1])), scale2));
+                                const float2 x = __ffma2_rn(make_float2(__uint_as_float(sr[8 * jj + 2 * k]), __uint_as_float(sr[8 * jj + 2 * k + 1])), scale2,
+                                                            make_float2(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xFFFF0000u)));
                                 mx[k & 1] = max3(mx[k & 1], x.x, x.y);
                             }
                         }

@@ -669,3 +669,31 @@ def test_token_attention_when_later_chunks_outgrow_the_first(lib, oracle_lib, ma
     err_out = driver.max_rel_err(out[True], oracle_lib.read("OUT"))
     print("N=%d S=%d masked=%d: TO vs oracle %.2e, OUT vs oracle %.2e" % (n_tok, samples, masked, err, err_out))
     assert err <= BF16_TOL and err_out < GATE
+
+
+def test_masked_first_chunk_with_a_score_on_a_rounding_tie(lib, oracle_lib, make_case):
+    """A row whose first 64 keys are all masked takes its reference value from logits of -1.4e9, where f32 has a step of
+    128. Scores a hair above an odd multiple of 64 lie on a tie there: if the maximum and the pass rounded them to
+    different neighbours, an exponential would be 2^128 and the row NaN. q and k are given by QKNORM's offsets (scale
+    0), so that every q·k is 1536.7246, which scales to 320 + 2.6e-6 in base 2."""
+    flags = synth.F_QKNORM
+    x, meta = make_case(192, 1, 8, False, flags=flags)
+    x = [a.copy() for a in x]
+    x[synth.IN["PC"]][:] = 0
+    x[synth.IN["PCS"]][..., 0] = 0
+    x[synth.IN["TMASK"]][:64] = 0
+    tqkn = x[synth.IN["TQKN"]].reshape(-1, 4, 16, 48)
+    tqkn[:] = 0
+    steps = round((float(np.float32(1536.7246)) - 1536) * 2 ** 13)
+    tqkn[:, 1, :, :3] = 1
+    tqkn[:, 3, :, :3] = 1536, (steps & ~63) / 2.0 ** 13, (steps & 63) / 2.0 ** 13
+    lib.setup(x, meta)
+    xn = synth.noisy_positions(meta, mg.T_ONCE)
+    lib.run(mode=1, dbg_stop=mg.STOPS["tok0_attn"][0] + 1, xn=xn, t=mg.T_ONCE)  # QKNORM has a phase of its own before it
+    qk = lib.read("QKVG").astype(np.float64).reshape(192, 4, 16, 48)
+    assert np.unique(np.einsum("nhd,mhd->hnm", qk[:, 0], qk[:, 1])).tolist() == [float(np.float32(1536.7246))]
+    check_token_attention(lib, 192, 1, 1 / 2)
+    oracle_lib.setup(x, meta)
+    oracle_lib.run(mode=1, xn=xn, t=mg.T_ONCE)
+    lib.run(mode=1, xn=xn, t=mg.T_ONCE)
+    assert driver.max_rel_err(lib.read("OUT"), oracle_lib.read("OUT")) < GATE
