@@ -388,6 +388,11 @@ __device__ __forceinline__ void red_release_add(unsigned int* p, unsigned int v)
 __device__ __forceinline__ void red_relaxed_add(unsigned int* p, unsigned int v) {
     asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+__device__ __forceinline__ unsigned int atom_add_cta(unsigned int* p, unsigned int v) { // shared memory
+    unsigned int old;
+    asm volatile("atom.acq_rel.cta.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(smem_u32(p)), "r"(v) : "memory");
+    return old;
+}
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
     unsigned int v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -605,7 +605,6 @@ __device__ __forceinline__ void atom_rows_wait(const KP& p, int which, unsigned 
     __syncwarp();
 }
 __device__ __forceinline__ void atom_rows_report(const KP& p, int sig, const OctRows& o) {
-    fence_async_global(); // for TMA reads in other CTAs
     __syncwarp();
     if (lane_id() == 0) {
         unsigned int* cnt = flow_cnt(p, sig);
