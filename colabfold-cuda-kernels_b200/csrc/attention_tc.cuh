@@ -177,7 +177,7 @@ __device__ __forceinline__ int tc_track_item(int first, int t, int j) {
     return first + (t + kTcTracks * j) * int(gridDim.x);
 }
 // one phase: all items of this CTA
-__device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, int b, unsigned int epoch) {
+__device__ CCK_PHASE_FN void token_attention_tc(const Launch& L, Deal& d, int b, unsigned int epoch) {
     const KP& p = kp();
     char* sm = smem_base();
     SmemCtl* ctl = smem_ctl();
@@ -185,6 +185,7 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
     const int N = p.N, np = p.np, npb = p.npb, S = p.S;
     const int qblocks = cdiv(N, kTcRows), items = kHeads * qblocks * S, chunks = np / kTcKeys;
     const int warp = warp_id(), lane = lane_id(), first = d.first();
+    d.advance(items);
     const uint32_t tmem = ctl->tmem_base;
     const bool flow = p.flow;
     const int alt = flow ? int(epoch & 1) : 0; // which of the two buffers holds this block's q, k, v and gates
@@ -578,7 +579,6 @@ __device__ CCK_PHASE_FN int token_attention_tc(const Launch& L, const Deal d, in
             bars->items[t] = j0 + uint32_t(n), bars->chunks[t] = g;
         }
     }
-    return items;
 }
 
 } // namespace cck

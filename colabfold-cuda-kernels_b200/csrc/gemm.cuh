@@ -59,6 +59,7 @@ struct SmemCtl {
     volatile int quit;                      // the launch has failed somewhere: leave the schedule
     unsigned long long t0;                  // end of the previous phase, ns (timing record, CTA 0)
     int ring_bn;                            // the column tile that the ring's slots are laid out for (TMA thread)
+    const Launch* launch;                   // the kernel's parameter block
     unsigned int parts[4];                  // worker warps' parts of tiles counted so far, tile t in slot t % 4 (flow_signal_tile)
 };
 
@@ -138,6 +139,13 @@ __device__ __forceinline__ char* smem_base() {
     extern __shared__ char smem_raw[];
     const uint32_t a = smem_u32(smem_raw);
     return smem_raw + ((1024u - (a & 1023u)) & 1023u);
+}
+// the same, worked out anew where it is asked for: nothing of it is held in registers from an earlier place
+__device__ __forceinline__ char* smem_base_anew() {
+    extern __shared__ char smem_raw[];
+    uint32_t a;
+    asm volatile("mov.u32 %0, %1;" : "=r"(a) : "r"(smem_u32(smem_raw)));
+    return static_cast<char*>(__cvta_shared_to_generic((a + 1023u) & ~1023u));
 }
 // The parameter block with the call's real extents filled in (the kernel parameter holds the
 // bucket's): every CTA keeps a copy in shared memory

@@ -59,9 +59,18 @@ __device__ __forceinline__ Op flow_next(const Program& prog, const KP& p, Flow& 
 }
 
 // ---- grid barrier
-// The schedule state of the calling thread (shared memory)
+// The schedule state of the calling thread (shared memory). Its address is worked out anew each time, so that the
+// compiler does not hold it in a register over an operation, and so is the parameter's (SmemCtl::launch): a called
+// function that needs all registers saves what its caller holds to local memory and loads it back when it is
+// through, from L2, since every look at a completion counter empties L1. The token attention saved eight registers
+// (ms per step with none: 61 x 5 1.099 -> 1.081, 256 x 5 1.547 -> 1.531, 512 x 5 2.382 -> 2.363, 384 x 1 on barriers 1.367 -> 1.339).
 __device__ __forceinline__ Run& run_state() {
-    return *reinterpret_cast<Run*>(smem_base() + kRunOff + threadIdx.x * kRunSlot);
+    uint32_t t;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    return *reinterpret_cast<Run*>(smem_base_anew() + kRunOff + t * kRunSlot);
+}
+__device__ __forceinline__ const Program& program() {
+    return *reinterpret_cast<const Program*>(smem_base_anew() + kProgOff);
 }
 // Ends a phase (end_kind: OpEnd in the low two bits, the timing kind above). Returns true when a debug
 // run has reached its last phase. Takes and returns next to nothing, so that the caller holds no
@@ -371,6 +380,7 @@ __device__ __forceinline__ void run_gemm(const Launch& L, Run& r, Deal& d, int i
     const GemmDesc& g = gd_table()[id];
     const int tiles = g.tiles, tb = d.first(), ts = gridDim.x;
     const int warp = warp_id();
+    d.advance(tiles);
     if (warp == 0) {
         gemm_produce(L, r.pipe, g, b, tb, tiles, ts, false, 0, epoch);
     } else if (warp == 1) {
@@ -401,7 +411,6 @@ __device__ __forceinline__ void run_gemm(const Launch& L, Run& r, Deal& d, int i
         }
     }
     __syncwarp();
-    d.advance(tiles);
 }
 
 // How many token blocks of this launch came before the current one (denoiser calls so far x blocks
@@ -496,7 +505,7 @@ __device__ __forceinline__ void run_op(const Launch& L, Run& r, const Op op) {
         token_adaln2(p, d, b);
         break;
     case FN_TOK_ATTN:
-        d.advance(token_attention_tc(L, d, b, flow_epoch(p, r)));
+        token_attention_tc(L, d, b, flow_epoch(p, r));
         break;
     case FN_TOK_FINAL_LN:
         token_final_ln(p, d, flow_epoch(p, r) + p.nb); // (the loop has set the block back to 0)
@@ -514,9 +523,6 @@ __device__ __forceinline__ void run_op(const Launch& L, Run& r, const Op op) {
         if (op.a0 == 0) {
             __syncthreads();
         }
-    }
-    if (op.fn != FN_GEMM && op.fn != FN_CTA_SYNC) {
-        fence_async_smem(); // what this thread did in the scratch area, before TMA loads fill the ring there
     }
 }
 
@@ -557,6 +563,9 @@ extern "C" __global__ void __launch_bounds__(cck::kThreads, 1) cck_sampler_kerne
     if (threadIdx.x < 2 * kKinds) {
         reinterpret_cast<unsigned long long*>(smem_base() + kCtlOff + kTimingOff)[threadIdx.x] = 0;
     }
+    if (threadIdx.x == 0) {
+        smem_ctl()->launch = &L; // (read after the barriers that follow)
+    }
     gd_build();
     gemm_init();
     attn_tc_init();
@@ -565,22 +574,28 @@ extern "C" __global__ void __launch_bounds__(cck::kThreads, 1) cck_sampler_kerne
     // every grid barrier empties L1, and state kept in local memory would then cost an L2 round
     // trip per touch right at the start of every phase.
     static_assert(sizeof(Run) <= kRunSlot, "Run outgrew its shared-memory slot");
-    Run& r = *new (&run_state()) Run();
-    // The interpreter: all of its state lives in r (shared memory), so nothing but addresses is
-    // held in registers across the calls of the phase functions.
-    const Program& prog = *reinterpret_cast<const Program*>(smem_base() + kProgOff);
-    r.step = kp().mode == 0 ? 1 : 0;
+    (new (&run_state()) Run())->step = kp().mode == 0 ? 1 : 0;
+    // The interpreter: all of its state lives in shared memory, so nothing is held in registers across the calls of
+    // the phase functions.
     for (;;) {
-        Flow f{r.pc, r.blk, r.step, r.ret, r.second};
-        const Op op = flow_next(prog, kp(), f);
-        r.pc = f.pc, r.blk = f.blk, r.step = f.step, r.ret = f.ret, r.second = f.second;
-        if (op.fn == FN_END) {
-            break;
+        {
+            Run& r = run_state();
+            Flow f{r.pc, r.blk, r.step, r.ret, r.second};
+            const Op op = flow_next(program(), kp(), f);
+            r.pc = f.pc, r.blk = f.blk, r.step = f.step, r.ret = f.ret, r.second = f.second;
+            if (op.fn == FN_END) {
+                break;
+            }
+            if (threadIdx.x == 0) {
+                CCK_TRACE_ONE(6, 0x80, op.fn);
+            }
+            run_op(*smem_ctl()->launch, r, op);
         }
-        if (threadIdx.x == 0) {
-            CCK_TRACE_ONE(6, 0x80, op.fn);
+        Run& r = run_state(); // (looked up again rather than kept: run_state)
+        const Op op = program().ops[r.pc];
+        if (op.fn != FN_GEMM && op.fn != FN_CTA_SYNC) {
+            fence_async_smem(); // what this thread did in the scratch area, before TMA loads fill the ring there
         }
-        run_op(L, r, op);
         if (threadIdx.x == 0) {
             CCK_TRACE_ONE(6, 0x82, op.fn);
         }
@@ -591,7 +606,7 @@ extern "C" __global__ void __launch_bounds__(cck::kThreads, 1) cck_sampler_kerne
                 atomicAdd(&kp().ctl->barrier, 1u);
             }
             r.syncs++;
-        } else if ((op.end_kind & 3) != END_NONE && grid_barrier(L, op.end_kind)) {
+        } else if ((op.end_kind & 3) != END_NONE && grid_barrier(*smem_ctl()->launch, op.end_kind)) {
             break;
         }
     }
