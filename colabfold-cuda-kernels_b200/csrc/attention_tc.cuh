@@ -220,7 +220,7 @@ __device__ CCK_PHASE_FN void token_attention_tc(const Launch& L, Deal& d, int b,
                 if (flow && is != ready) {
                     // every column tile of QKVG over the sample's rows (q, k, v and the gate), and over the
                     // next sample's rows that the last chunk of keys reaches into (masked, but read)
-                    flow_wait(flow_cnt(p, FC_QKVG), is * N / kBM, (min(is * N + np, S * N) - 1) / kBM, qkvg_done, &ctl->abort);
+                    flow_wait_warp(flow_cnt(p, FC_QKVG), is * N / kBM, (min(is * N + np, S * N) - 1) / kBM, qkvg_done, &ctl->abort);
                     __syncwarp();
                     ready = is;
                 }
