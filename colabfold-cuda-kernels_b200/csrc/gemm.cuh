@@ -402,22 +402,21 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
             float* bs = reinterpret_cast<float*>(smem_base() + kBiasOff) + (warp_id() - kWorkWarp0) * 32;
             const bool has_bias = E != EPI_GLU && g.bias != nullptr;
             float bnext = 0.f;
-            if (has_bias && gp < units) {
-                const int c = oc0 + 32 * gp + lane_id();
-                bnext = c < g.bias_cols ? g.bias[c] : 0.f;
+            if (has_bias && gp < units && oc0 + 32 * gp < g.bias_cols) {
+                bnext = g.bias[oc0 + 32 * gp + lane_id()];
             }
             mbar_wait(tfull, tpar, abort);
             tc_fence_after();
 #pragma unroll 1
             for (int u = gp; u < units; u += 2) {
                 const int oc = oc0 + 32 * u;
-                if (has_bias) {
+                const bool biased = has_bias && oc < g.bias_cols; // (a unit has a bias or has none: bias_cols is a multiple of 32)
+                if (biased) {
                     __syncwarp();
                     bs[lane_id()] = bnext;
                     __syncwarp();
-                    if (u + 2 < units) {
-                        const int c = oc + 64 + lane_id();
-                        bnext = c < g.bias_cols ? g.bias[c] : 0.f;
+                    if (u + 2 < units && oc + 64 < g.bias_cols) {
+                        bnext = g.bias[oc + 64 + lane_id()];
                     }
                 }
                 float v[32];
@@ -428,8 +427,10 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
                     tmem_ld_wait(ga);
                     tmem_ld_wait(pr);
 #pragma unroll
-                    for (int i = 0; i < 32; i++) {
-                        v[i] = silu_fast(__uint_as_float(ga[i])) * __uint_as_float(pr[i]);
+                    for (int i = 0; i < 32; i += 2) {
+                        const float2 y = __fmul2_rn(silu_fast2(make_float2(__uint_as_float(ga[i]), __uint_as_float(ga[i + 1]))),
+                                                    make_float2(__uint_as_float(pr[i]), __uint_as_float(pr[i + 1])));
+                        v[i] = y.x, v[i + 1] = y.y;
                     }
                     if (kIn > 2 * kGluHalf) { // [gate | proj | a_to_b]: the third part multiplies
                         float ab[32];
@@ -442,7 +443,7 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
                 } else {
                     tmem_ld32(taddr + u * kIn, v);
                 }
-                if (has_bias) {
+                if (biased) {
 #pragma unroll
                     for (int i = 0; i < 8; i++) {
                         const float4 bb = reinterpret_cast<const float4*>(bs)[i];
@@ -465,8 +466,9 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
                 }
                 if (sig) {
 #pragma unroll
-                    for (int i = 0; i < 32; i++) {
-                        v[i] = sigmoid_fast(v[i]);
+                    for (int i = 0; i < 32; i += 2) {
+                        const float2 y = sigmoid_fast2(make_float2(v[i], v[i + 1]));
+                        v[i] = y.x, v[i + 1] = y.y;
                     }
                 }
                 store_unit_tma(mo, st, x, y, v);

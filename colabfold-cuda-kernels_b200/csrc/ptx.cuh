@@ -421,6 +421,21 @@ __device__ __forceinline__ float silu_fast(float x) {
     const float h = 0.5f * x;
     return fmaf(h, tanh_approx(h), h);
 }
+// two at a time: a packed instruction costs the pipe what two scalar ones do, but it is one to fetch and to issue. A GEMM's
+// epilogue is run from instructions that are mostly fetched anew (past 32 KB of code 6.5 cycles an instruction, within it
+// 1.5 to 4, measured with straight-line code): with these, and without the addition of a bias that is zero, ms per step
+// 61 x 5 1.102 -> 1.083, 256 x 5 1.528 -> 1.517, 512 x 1 1.333 -> 1.325, 512 x 5 2.340 -> 2.321.
+__device__ __forceinline__ float2 tanh2(float2 x) {
+    return make_float2(tanh_approx(x.x), tanh_approx(x.y));
+}
+__device__ __forceinline__ float2 sigmoid_fast2(float2 x) {
+    const float2 half = make_float2(0.5f, 0.5f);
+    return __ffma2_rn(half, tanh2(__fmul2_rn(x, half)), half);
+}
+__device__ __forceinline__ float2 silu_fast2(float2 x) {
+    const float2 h = __fmul2_rn(x, make_float2(0.5f, 0.5f));
+    return __ffma2_rn(h, tanh2(h), h);
+}
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
