@@ -52,7 +52,7 @@ __device__ __forceinline__ float quad_sum(float v) {
 }
 
 // ---- atom attention
-// Work unit = (subset, head, sample), one warp each with its own staging area, no CTA-wide
+// Work unit = (subset, head, sample), or half of one in small folds, one warp each with its own staging area, no CTA-wide
 // synchronisation: the ten warps of a CTA sit at different points of load -> scores -> softmax ->
 // P·V, which is what hides the latency of the gathered key rows. Samples run fastest so that the
 // units that share a subset's pair logits run at the same time and meet in L2.
@@ -168,12 +168,18 @@ __device__ __forceinline__ void atom_half_compute(AtomHalf& a, const KP& p, int 
 }
 
 // AO = softmax(q·kᵀ/√32 + 1e9(QMASK-1)(KMASK-1) + APL)·v ⊙ g (reference: src/diffusion/attention.cuh:313-434)
-__device__ CCK_HOT_FN void atom_attention(const KP& p, Deal& d, const AtomW& w, int b) {
-    const int units = p.NS * kAtomHeads * p.S;
+__device__ CCK_PHASE_FN void atom_attention(const KP& p, Deal& d, const AtomW& w, int b) {
+    // Where even the halves (16 queries) of the units find a warp each, a half is a unit: the window is gathered twice, but
+    // a warp is through with it in some three quarters of the time, and one unit per warp is all these folds have (ms
+    // per step 32 x 1 0.953 -> 0.931, 512 x 1 1.324 -> 1.298). With more units than that, three rounds of halves would take longer than
+    // two of units. Both kinds go through the same code, out of line: 61 x 5 1.047 -> 1.042 against inlined and unrolled.
+    const int full = p.NS * kAtomHeads * p.S;
+    const int halves = 2 * full <= int(gridDim.x) * kAwWarps ? 2 : 1, units = halves * full;
     bf16* sm = reinterpret_cast<bf16*>(smem_base() + warp_id() * kAwBytes);
     const int lane = lane_id();
     for (int un = d.first() * kAwWarps + warp_id(); un < units && warp_id() < kAwWarps; un += gridDim.x * kAwWarps) {
-        const int v = int(div_prepared(uint32_t(un), p.tc_div_s)), s = un - v * p.S, h = v % kAtomHeads, u = v / kAtomHeads;
+        const int whole = halves == 2 ? un >> 1 : un, v = int(div_prepared(uint32_t(whole), p.tc_div_s)), s = whole - v * p.S, h = v % kAtomHeads, u = v / kAtomHeads;
+        int qt = halves == 2 ? un & 1 : 0; // which half
         __syncwarp(); // every lane is done with the previous window
         // the head's slice of the window's [k | v] rows: 128 rows x (64 + 64) bytes, zero where Q2K is -1.
         // Four lanes copy one 64-byte slice, so an instruction touches 8 lines rather than 32.
@@ -196,12 +202,17 @@ __device__ CCK_HOT_FN void atom_attention(const KP& p, Deal& d, const AtomW& w, 
         cp_async16(kmask + 4 * lane, p.geo.kmask + u * kSubsetKeys + 4 * lane, true);
         cp_async_commit();
         AtomHalf a;
-        atom_half_load(a, p, w, b, u, s, h, 0); // under way while the window lands
+        atom_half_load(a, p, w, b, u, s, h, qt); // under way while the window lands
         cp_async_wait<0>();
         __syncwarp();
-        atom_half_compute(a, p, h, sm, kmask);
-        atom_half_load(a, p, w, b, u, s, h, 1);
-        atom_half_compute(a, p, h, sm, kmask);
+#pragma unroll 1
+        for (;;) {
+            atom_half_compute(a, p, h, sm, kmask);
+            if (halves == 2 || qt) {
+                break;
+            }
+            atom_half_load(a, p, w, b, u, s, h, ++qt);
+        }
     }
     d.advance(cdiv(units, kAwWarps));
 }

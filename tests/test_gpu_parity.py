@@ -697,3 +697,25 @@ def test_masked_first_chunk_with_a_score_on_a_rounding_tie(lib, oracle_lib, make
     oracle_lib.run(mode=1, xn=xn, t=mg.T_ONCE)
     lib.run(mode=1, xn=xn, t=mg.T_ONCE)
     assert driver.max_rel_err(lib.read("OUT"), oracle_lib.read("OUT")) < GATE
+
+
+@pytest.mark.parametrize("n_tok,samples", [(184, 4), (188, 4)])
+def test_atom_attention_by_halves_and_whole(lib, oracle_lib, make_case, n_tok, samples):
+    """The last size at which the halves of the atom attention's units find a warp each (46 subsets x 4 heads x 4 samples, twice 736
+    for 1480 warps on 148 SMs) and the next, where a unit is whole: the attention's output of the first encoder block and
+    the denoiser's output against the oracle."""
+    x, meta = make_case(n_tok, samples, 8, False)
+    lib.setup(x, meta)
+    oracle_lib.setup(x, meta)
+    xn = synth.noisy_positions(meta, mg.T_ONCE)
+    stop, _ = mg.STOPS["enc0_attn"]
+    oracle_lib.clear_snapshots()
+    oracle_lib.snapshot(stop, "AO")
+    oracle_lib.run(mode=1, xn=xn, t=mg.T_ONCE)
+    want = oracle_lib.read("AO@%d" % stop).copy()
+    oracle_lib.clear_snapshots()
+    lib.run(mode=1, dbg_stop=stop, xn=xn, t=mg.T_ONCE)
+    ao = lib.read("AO").copy()
+    lib.run(mode=1, xn=xn, t=mg.T_ONCE)
+    assert driver.max_rel_err(ao, want) <= BF16_TOL and driver.rms_rel_err(ao, want) <= RMS_TOL
+    assert driver.max_rel_err(lib.read("OUT"), oracle_lib.read("OUT")) < GATE
