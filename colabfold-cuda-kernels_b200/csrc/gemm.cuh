@@ -219,6 +219,7 @@ __host__ __device__ inline int cdiv(int a, int b) {
 // conflict-free both ways), after which lane l holds the four columns 4(l % 4).. of rows l / 4 + 8i,
 // i < 4: every warp access covers eight full 64-byte row segments.
 constexpr int kPiece = 16;
+static_assert(kTokMods1 == 4 && kTokModSlots - kTokMods1 == 2 && kTokC % kMaxBN == 0, "EPI_MODS finds block and slot by shifts, once per tile");
 __device__ __forceinline__ float* epi_stage() {
     return reinterpret_cast<float*>(smem_base() + kEpiOff + (warp_id() - kWorkWarp0) * kEpiStageBytes);
 }
@@ -405,6 +406,12 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
             if (has_bias && gp < units && oc0 + 32 * gp < g.bias_cols) {
                 bnext = g.bias[oc0 + 32 * gp + lane_id()];
             }
+            int mx = 0, my = 0; // MODS: a tile lies in one slot of one block (768 is a multiple of every width): column c is slot slot0 + (c / 768) % slots of block c / (slots·768)
+            bool msig = false;
+            if constexpr (E == EPI_MODS) {
+                const int s = oc0 / kTokC, blk = g.slots == 4 ? s >> 2 : s >> 1, slot = g.slot0 + (s & (g.slots - 1));
+                msig = g.sig_slots >> slot & 1, mx = oc0 - s * kTokC, my = (blk * kTokModSlots + slot) * g.period + rbase;
+            }
             mbar_wait(tfull, tpar, abort);
             tc_fence_after();
 #pragma unroll 1
@@ -459,10 +466,7 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
                     }
                 }
                 if constexpr (E == EPI_MODS) {
-                    // column c is slot slot0 + (c / 768) % slots of block c / (slots·768): one slot per unit
-                    const int blk = oc / (g.slots * kTokC), slot = g.slot0 + (oc / kTokC) % g.slots;
-                    sig = g.sig_slots >> slot & 1;
-                    x = oc % kTokC, y = (blk * kTokModSlots + slot) * g.period + rbase;
+                    x = mx + 32 * u, y = my, sig = msig;
                 }
                 if (sig) {
 #pragma unroll
