@@ -323,24 +323,35 @@ template <int E> __device__ __forceinline__ void epi_store(const GemmDesc& g, co
 }
 
 // The pair logits of one unit: a tile's rows are 128 consecutive keys k of one query q (rbase
-// encodes q·ktiles·128 + k0), the column is the table (block·16 + head); base-2 logits. Lanes are
-// consecutive k of one table row already: stored without the turn. Keys past the real tokens are
-// masked, keys past the padded extent are not stored.
-__device__ __forceinline__ void pair_unit(const GemmDesc& g, int rbase, int c0, const float (&v)[32]) {
-    const int q = rbase / (g.ktiles * kBM), k = rbase % (g.ktiles * kBM) + lane_id();
-    if (q < g.nreal && k < g.npreal) {
+// encodes q·ktiles·128 + k0), the column is the table (block·16 + head); base-2 logits. Keys past the real tokens
+// are masked, keys past the padded extent (a multiple of 64: a warp's 32 are in or out together) are not stored. The
+// 32 tables x 32 keys leave the warp's stage as one block of the tables' planes; stored by the lanes themselves, 2 bytes to
+// a lane and 32 addresses to a unit, a tile took 22,000 cycles (2048 tokens: the whole build 4.4 ms).
+__device__ __forceinline__ void pair_unit(const GemmDesc& g, const CUtensorMap* mo, float* st, int rbase, int c0, const float (&v)[32]) {
+    const int q = rbase / (g.ktiles * kBM), k0 = rbase % (g.ktiles * kBM), l = lane_id(), k = k0 + l;
+    if (q < g.nreal && k0 < g.npreal) {
         const TokenW& tw = kp().tw;
         const bool masked = k >= g.nreal || tw.tmask[k] == 0.f;
         const size_t pq = size_t(q) * g.ldn + (masked ? 0 : k);
         const float mean = tw.pcs[2 * pq], rstd = tw.pcs[2 * pq + 1];
         const float extra = kp().plx ? bf_to_f32(tw.plx[pq]) : 0.f;
-        bf16* o = static_cast<bf16*>(g.out) + size_t(q) * g.np + k;
-        const size_t plane = size_t(g.np) * g.np;
+        const float ws = tw.plws[c0 + l], wb = tw.plb[c0 + l]; // (lane l: of table c0 + l)
+        if (l == 0) {
+            bulk_wait_read(); // the previous store has read the stage
+        }
+        __syncwarp();
+        bf16* out = reinterpret_cast<bf16*>(st) + l;
 #pragma unroll
         for (int i = 0; i < 32; i++) {
-            const int col = c0 + i;
-            const float y = kLog2e * (masked ? -kMaskBias : rstd * (v[i] - mean * tw.plws[col]) + tw.plb[col] + extra);
-            o[col * plane] = bf16(pack_bf2(y, 0.f) & 0xFFFFu);
+            const float wi = __shfl_sync(0xffffffffu, ws, i), bi = __shfl_sync(0xffffffffu, wb, i); // (by all lanes, masked or not)
+            const float y = kLog2e * (masked ? -kMaskBias : rstd * (v[i] - mean * wi) + bi + extra);
+            out[32 * i] = bf16(pack_bf2(y, 0.f) & 0xFFFFu);
+        }
+        fence_async_smem();
+        __syncwarp();
+        if (l == 0) {
+            tma_store_3d(mo, k0, q, c0, st);
+            bulk_commit();
         }
     }
 }
@@ -520,7 +531,7 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
             tmem_ld32(taddr + u * kIn, v);
         }
         if constexpr (E == EPI_PAIR) {
-            pair_unit(g, rbase, oc, v);
+            pair_unit(g, mo, st, rbase, oc, v);
         } else {
             if constexpr (E == EPI_BF16) {
                 if (g.vt && oc >= 2 * kTokC && oc < 3 * kTokC) {
@@ -836,7 +847,7 @@ template <int E> __device__ CCK_HOT_FN void worker_tiles(const GemmDesc& gd, con
         CCK_TRACE_EV(0x74, t); // stored and reported
     }
     pipe.tile = tile;
-    if constexpr (E == EPI_BF16 || E == EPI_GLU || E == EPI_MODS) {
+    if constexpr (E == EPI_BF16 || E == EPI_GLU || E == EPI_MODS || E == EPI_PAIR) {
         if (lane_id() == 0) {
             bulk_wait_done(); // this warp's TMA stores have landed before the phase ends
         }

@@ -270,6 +270,21 @@ static int encode_store_map(CUtensorMap* m, const void* base, size_t rows, size_
     return E_OK;
 }
 
+// the planes [tables][np][np] of the pair logits, stored in blocks of 32 tables x 32 keys of one query (dense 64-byte rows)
+static int encode_planes_map(CUtensorMap* m, const void* base, size_t tables, size_t np) {
+    const cuuint64_t dims[3] = {np, np, tables};
+    const cuuint64_t strides[2] = {np * sizeof(bf16), np * np * sizeof(bf16)};
+    const cuuint32_t box[3] = {32, 1, 32};
+    const cuuint32_t elem[3] = {1, 1, 1};
+    const CUresult r = g_encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem,
+                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        return fail(E_LAUNCH, "MkSample: cuTensorMapEncodeTiled failed for the pair logits (" + std::to_string(int(r)) + ")");
+    }
+    return E_OK;
+}
+
 // a bf16 output [rows][cols] stored in boxes of box_rows x box_cols from dense rows in shared memory
 static int encode_rows_store_map(CUtensorMap* m, const void* base, size_t rows, size_t cols, int box_rows, int box_cols) {
     const cuuint64_t dims[2] = {cols, rows};
@@ -633,6 +648,9 @@ static int make_launch(Launch& L, const Template& t, const Device& dev, const vo
         }
     }
     if (int e = encode_map(&L.tmap[TM_T_PLG], b.plg, size_t(t.nb) * kPairHeads * t.np, size_t(t.np), size_t(t.np), 128)) {
+        return e;
+    }
+    if (int e = encode_planes_map(&L.tmap[TM_O_PLG], b.plg, size_t(t.nb) * kPairHeads, size_t(t.np))) {
         return e;
     }
     // the attention's output: a softmax warp's 32 rows of one head

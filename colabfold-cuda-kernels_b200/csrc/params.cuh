@@ -19,7 +19,7 @@ namespace cck {
     X(B_ENC_WQG) X(B_ENC_WKV) X(B_ENC_WO) X(B_ENC_W1) X(B_ENC_W2)                                  \
     X(B_DEC_WQG) X(B_DEC_WKV) X(B_DEC_WO) X(B_DEC_W1) X(B_DEC_W2)                                  \
     X(T_QK) X(T_QK2) X(T_VT) X(T_VT2) X(T_PLG) X(T_TO)                                                                    \
-    X(O_QKVG) X(O_QKVG2) X(O_AQG) X(O_AKV) X(O_TC) X(O_ACA) X(O_SCH) X(O_MODS)
+    X(O_QKVG) X(O_QKVG2) X(O_AQG) X(O_AKV) X(O_TC) X(O_ACA) X(O_SCH) X(O_MODS) X(O_PLG)
 #define CCK_ENUM(name) TM_##name,
 enum TMap { CCK_TMAPS(CCK_ENUM) kNumTMaps };
 #undef CCK_ENUM

@@ -719,3 +719,37 @@ def test_atom_attention_by_halves_and_whole(lib, oracle_lib, make_case, n_tok, s
     lib.run(mode=1, xn=xn, t=mg.T_ONCE)
     assert driver.max_rel_err(ao, want) <= BF16_TOL and driver.rms_rel_err(ao, want) <= RMS_TOL
     assert driver.max_rel_err(lib.read("OUT"), oracle_lib.read("OUT")) < GATE
+
+
+@pytest.mark.parametrize("n_tok,bucket,masked", [(32, 0, 0), (100, 0, 7), (132, 192, 3)])
+def test_pair_logits(lib, make_case, n_tok, bucket, masked):
+    """The pair logits of all blocks, whose tiles leave as blocks of 32 tables x 32 keys: less than one tile of 128 keys, ragged, and
+    past a tile inside a bucket, with masked tokens. Each against 64 bits: the logit is a bf16 (2^-8 of itself), its
+    dot product and the two terms of its folded LayerNorm sums of f32 (2^-16 of the terms' sizes is far above them)."""
+    x, meta = make_case(n_tok, 1, 8, False)
+    x = [a.copy() for a in x]
+    if bucket:
+        x, meta = synth.pad_to_bucket(x, meta, bucket, bucket // 4)
+    x[synth.IN["TMASK"]][:masked] = 0
+    lib.setup(x, meta)
+    n, nb = n_tok, meta["N"]
+    if bucket:
+        lib.set_extent(n_tok, n_tok // 4)
+    lib.run(mode=1, dbg_stop=1, xn=np.zeros(meta["S"] * nb * 24 * 3, np.float32), t=mg.T_ONCE)
+    if bucket:
+        lib.set_extent(0, 0)
+    np_ = (nb + 63) // 64 * 64
+    got = lib.read("PLG").reshape(-1, np_, np_)[:, :n, :(n + 63) // 64 * 64].astype(np.float64)
+    f = lambda name: synth.from_bf16(x[synth.IN[name]]).astype(np.float64)
+    z = f("PC").reshape(nb, nb, -1)[:n, :n]
+    w = f("PLW").reshape(-1, z.shape[-1])
+    stats = x[synth.IN["PCS"]].reshape(nb, nb, 2)[:n, :n].astype(np.float64)
+    dot, ws, wb = np.einsum("qkc,tc->tqk", z, w), x[synth.IN["PLWS"]].astype(np.float64), x[synth.IN["PLB"]].astype(np.float64)
+    terms = stats[..., 1] * np.abs(dot), np.abs(stats[..., 1] * stats[..., 0]) * np.abs(ws)[:, None, None], np.abs(wb)[:, None, None]
+    want = np.log2(np.e) * (stats[..., 1] * (dot - stats[..., 0] * ws[:, None, None]) + wb[:, None, None])
+    bound = 2.0 ** -8 * np.abs(want) + 2.0 ** -16 * (1 + sum(terms)) * np.log2(np.e)
+    real = np.ones(n, bool)
+    real[:masked] = False
+    assert (np.abs(got[:, :, :n] - want)[:, :, real] <= bound[:, :, real]).all()
+    off = got[:, :, ~np.concatenate([real, np.zeros(got.shape[2] - n, bool)])]
+    assert off.size == 0 or np.abs(off / (-1e9 * np.log2(np.e)) - 1).max() < 2.0 ** -8
