@@ -240,27 +240,21 @@ __device__ __forceinline__ void epi_turn(float* st, const float* v, float4 (&t)[
     }
     __syncwarp();
 }
-__device__ __forceinline__ uint2 pack_bf4(float4 x) {
-    return make_uint2(pack_bf2(x.x, x.y), pack_bf2(x.z, x.w));
-}
 __device__ __forceinline__ float4 unpack_bf4(uint2 u) {
     return make_float4(bf_to_f32(u.x & 0xFFFFu), bf_to_f32(u.x >> 16), bf_to_f32(u.y & 0xFFFFu), bf_to_f32(u.y >> 16));
 }
 __device__ __forceinline__ float4 add4(float4 a, float4 b) {
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
-__device__ __forceinline__ float4 sigmoid4(float4 x) {
-    return make_float4(sigmoid_fast(x.x), sigmoid_fast(x.y), sigmoid_fast(x.z), sigmoid_fast(x.w));
-}
 
-// What a unit of 32 columns needs from global memory besides the accumulator: the bias of its two
-// pieces, fetched one unit ahead (the first unit's before the accumulator is complete), because
-// after a grid barrier every such load is an L2 round trip
+// f32 outputs, one piece after the turn: rows r0 + 8i, columns c..c+3 at o (of row 0). The bias of a unit's two pieces is
+// fetched one unit ahead (the first unit's before the accumulator is complete), because after a grid barrier every
+// such load is an L2 round trip.
 struct EpiPre {
     float4 b[2];
 };
 template <int E> __device__ __forceinline__ void epi_prefetch(const GemmDesc& g, int c0, EpiPre& pre) {
-    if constexpr (E == EPI_BF16 || E == EPI_F32 || E == EPI_MODS) {
+    if constexpr (E == EPI_F32) {
         const int col = c0 + 4 * (lane_id() & 3);
 #pragma unroll
         for (int pc = 0; pc < 2; pc++) {
@@ -269,55 +263,22 @@ template <int E> __device__ __forceinline__ void epi_prefetch(const GemmDesc& g,
         }
     }
 }
-// per unit: where its rows go (row r of the GEMM at o + r·ld, in elements of the output type) and
-// whether the sigmoid applies
-struct EpiUnit {
-    void* o;
-    int ld;
-    bool sig;
-};
-template <int E> __device__ __forceinline__ EpiUnit epi_unit(const GemmDesc& g, int oc) {
-    EpiUnit u;
-    u.ld = g.ldo, u.sig = false;
-    if constexpr (E == EPI_MODS) {
-        // column c is slot slot0 + (c / 768) % slots of block c / (slots·768): one slot per unit
-        const int blk = oc / (g.slots * kTokC), slot = g.slot0 + (oc / kTokC) % g.slots;
-        u.sig = g.sig_slots >> slot & 1;
-        u.o = static_cast<bf16*>(g.out) + (size_t(blk) * kTokModSlots + slot) * g.period * kTokC + oc % kTokC;
-        u.ld = kTokC;
-    } else if constexpr (E == EPI_BF16 || E == EPI_GLU) {
-        u.sig = oc >= g.sig_from;
-        u.o = static_cast<bf16*>(g.out) + oc;
-    } else {
-        u.o = static_cast<float*>(g.out) + oc;
-    }
-    return u;
-}
-
-// one piece after the turn: rows r0 + 8i, columns c..c+3 of the unit
-template <int E> __device__ __forceinline__ void epi_store(const GemmDesc& g, const EpiUnit& u, int r0, int c, const float4 (&t)[4],
-                                                           const float4& b) {
+template <int E> __device__ __forceinline__ void epi_store(const GemmDesc& g, float* o, int r0, const float4 (&t)[4], const float4& b) {
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int row = r0 + 8 * i;
         if (row >= g.m) {
             continue;
         }
-        if constexpr (E == EPI_BF16 || E == EPI_MODS || E == EPI_GLU) {
-            float4 x = E == EPI_GLU ? t[i] : add4(t[i], b);
-            if (E != EPI_GLU && u.sig) {
-                x = sigmoid4(x);
-            }
-            *reinterpret_cast<uint2*>(static_cast<bf16*>(u.o) + size_t(row) * u.ld + c) = pack_bf4(x);
-        } else if constexpr (E == EPI_F32) {
+        float4* p = reinterpret_cast<float4*>(o + size_t(row) * g.ldo);
+        if constexpr (E == EPI_F32) {
             float4 x = add4(t[i], b);
             if (g.relu) {
                 x = make_float4(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f), fmaxf(x.z, 0.f), fmaxf(x.w, 0.f));
             }
-            *reinterpret_cast<float4*>(static_cast<float*>(u.o) + size_t(row) * u.ld + c) = x;
-        } else if constexpr (E == EPI_SCRES) {
-            float4* o = reinterpret_cast<float4*>(static_cast<float*>(u.o) + size_t(row) * u.ld + c);
-            *o = add4(*o, t[i]);
+            *p = x;
+        } else { // EPI_SCRES
+            *p = add4(*p, t[i]);
         }
     }
 }
@@ -369,12 +330,28 @@ __device__ __forceinline__ void vt_unit(const GemmDesc& g, int rbase, int c0, co
     }
 }
 
-// A unit of bf16 output through TMA: the warp's 32 rows x 32 columns go row-per-lane (as they
-// leave TMEM) into the warp's stage in the 64-byte-swizzled layout of the store map, and one lane
-// issues the store. No turn, no per-row address arithmetic; rows past the tensor's end are clipped
-// by the copy, so the caller takes this path only when all 32 rows belong to the GEMM.
-__device__ __forceinline__ void store_unit_tma(const CUtensorMap* mo, float* st, int x, int y, const float (&v)[32]) {
+// A unit of bf16 output: the warp's 32 rows x 32 columns go row-per-lane (as they leave TMEM) into the
+// warp's stage in the 64-byte-swizzled layout of the store map, and one lane issues the store. No turn, no per-row
+// address arithmetic. In the last row tile, where what the store would write past the GEMM's rows is somebody else's, the lanes
+// store their rows themselves. (A second epilogue for that, with the turn, was half of the code of these kinds: ms per
+// step with it gone: 32 x 1 0.920 -> 0.903, 256 x 5 1.511 -> 1.489, 512 x 5 2.317 -> 2.287, 391 x 5 2.103 -> 2.048.)
+__device__ __forceinline__ void store_unit(const CUtensorMap* mo, float* st, int x, int y, bool whole, bf16* own, const float (&v)[32]) {
     const int l = lane_id();
+    uint4 w[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        w[c] = make_uint4(pack_bf2(v[8 * c], v[8 * c + 1]), pack_bf2(v[8 * c + 2], v[8 * c + 3]), pack_bf2(v[8 * c + 4], v[8 * c + 5]),
+                          pack_bf2(v[8 * c + 6], v[8 * c + 7]));
+    }
+    if (!whole) {
+        if (own) {
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                reinterpret_cast<uint4*>(own)[c] = w[c];
+            }
+        }
+        return;
+    }
     if (l == 0) {
         bulk_wait_read(); // the previous store has read the stage
     }
@@ -382,8 +359,7 @@ __device__ __forceinline__ void store_unit_tma(const CUtensorMap* mo, float* st,
     uint4* row = reinterpret_cast<uint4*>(reinterpret_cast<char*>(st) + 64 * l);
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-        row[c ^ ((l >> 1) & 3)] = make_uint4(pack_bf2(v[8 * c], v[8 * c + 1]), pack_bf2(v[8 * c + 2], v[8 * c + 3]),
-                                            pack_bf2(v[8 * c + 4], v[8 * c + 5]), pack_bf2(v[8 * c + 6], v[8 * c + 7]));
+        row[c ^ ((l >> 1) & 3)] = w[c];
     }
     fence_async_smem();
     __syncwarp();
@@ -398,154 +374,119 @@ __device__ __forceinline__ void store_unit_tma(const CUtensorMap* mo, float* st,
 // accumulator itself, after the first unit's global loads are under way.
 template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g, const CUtensorMap* mo, uint32_t acc, int row0, int col0,
                                                                uint64_t* tfull, uint32_t tpar, volatile int* abort) {
-    const int q = work_quarter(), gp = work_group();
-    const int rbase = row0 + q * 32, r0 = rbase + (lane_id() >> 2), cl = 4 * (lane_id() & 3);
+    const int q = work_quarter(), gp = work_group(), rbase = row0 + q * 32;
     const uint32_t taddr = acc + (uint32_t(q * 32) << 16);
     float* st = epi_stage();
-    const int kIn = E == EPI_GLU ? g.glu_unit : 32; // accumulator columns per unit
-    constexpr bool kTma = E == EPI_BF16 || E == EPI_GLU || E == EPI_MODS;
-    const int units = g.bn / kIn;
-    // output column of unit u: a GLU unit of 64 (or 96) columns gives 32
-    const int oc0 = E == EPI_GLU ? col0 / kIn * kGluHalf : col0;
-    if constexpr (kTma) {
-        if (mo && rbase + 32 <= g.m) {
-            // ---- all 32 rows are real: TMA stores. The unit's bias (one value per lane) waits in the
-            // warp's shared-memory slot, fetched a unit ahead.
-            float* bs = reinterpret_cast<float*>(smem_base() + kBiasOff) + (warp_id() - kWorkWarp0) * 32;
-            const bool has_bias = E != EPI_GLU && g.bias != nullptr;
-            float bnext = 0.f;
-            if (has_bias && gp < units && oc0 + 32 * gp < g.bias_cols) {
-                bnext = g.bias[oc0 + 32 * gp + lane_id()];
-            }
-            int mx = 0, my = 0; // MODS: a tile lies in one slot of one block (768 is a multiple of every width): column c is slot slot0 + (c / 768) % slots of block c / (slots·768)
-            bool msig = false;
-            if constexpr (E == EPI_MODS) {
-                const int s = oc0 / kTokC, blk = g.slots == 4 ? s >> 2 : s >> 1, slot = g.slot0 + (s & (g.slots - 1));
-                msig = g.sig_slots >> slot & 1, mx = oc0 - s * kTokC, my = (blk * kTokModSlots + slot) * g.period + rbase;
-            }
-            mbar_wait(tfull, tpar, abort);
-            tc_fence_after();
+    if constexpr (E == EPI_BF16 || E == EPI_GLU || E == EPI_MODS) {
+        const int kIn = E == EPI_GLU ? g.glu_unit : 32; // accumulator columns per unit
+        const int units = g.bn / kIn;
+        // output column of unit u: a GLU unit of 64 (or 96) columns gives 32
+        const int oc0 = E == EPI_GLU ? col0 / kIn * kGluHalf : col0;
+        const bool whole = rbase + 32 <= g.m;
+        // the unit's bias (one value per lane) waits in the warp's shared-memory slot, fetched a unit ahead
+        float* bs = reinterpret_cast<float*>(smem_base() + kBiasOff) + (warp_id() - kWorkWarp0) * 32;
+        const bool has_bias = E != EPI_GLU && g.bias != nullptr;
+        float bnext = 0.f;
+        if (has_bias && gp < units && oc0 + 32 * gp < g.bias_cols) {
+            bnext = g.bias[oc0 + 32 * gp + lane_id()];
+        }
+        // MODS: a tile lies in one slot of one block (768 is a multiple of every width): column c is slot slot0 + (c / 768) % slots of block c / (slots·768)
+        int x0 = oc0, y = rbase;
+        bool msig = false;
+        if constexpr (E == EPI_MODS) {
+            const int s = oc0 / kTokC, blk = g.slots == 4 ? s >> 2 : s >> 1, slot = g.slot0 + (s & (g.slots - 1));
+            msig = g.sig_slots >> slot & 1, x0 = oc0 - s * kTokC, y = (blk * kTokModSlots + slot) * g.period + rbase;
+        }
+        mbar_wait(tfull, tpar, abort);
+        tc_fence_after();
 #pragma unroll 1
-            for (int u = gp; u < units; u += 2) {
-                const int oc = oc0 + 32 * u;
-                const bool biased = has_bias && oc < g.bias_cols; // (a unit has a bias or has none: bias_cols is a multiple of 32)
-                if (biased) {
-                    __syncwarp();
-                    bs[lane_id()] = bnext;
-                    __syncwarp();
-                    if (u + 2 < units && oc + 64 < g.bias_cols) {
-                        bnext = g.bias[oc + 64 + lane_id()];
-                    }
-                }
-                float v[32];
-                if constexpr (E == EPI_GLU) {
-                    uint32_t ga[32], pr[32];
-                    tmem_ld32_issue(taddr + u * kIn, ga);
-                    tmem_ld32_issue(taddr + u * kIn + kGluHalf, pr);
-                    tmem_ld_wait(ga);
-                    tmem_ld_wait(pr);
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float2 y = __fmul2_rn(silu_fast2(make_float2(__uint_as_float(ga[i]), __uint_as_float(ga[i + 1]))),
-                                                    make_float2(__uint_as_float(pr[i]), __uint_as_float(pr[i + 1])));
-                        v[i] = y.x, v[i + 1] = y.y;
-                    }
-                    if (kIn > 2 * kGluHalf) { // [gate | proj | a_to_b]: the third part multiplies
-                        float ab[32];
-                        tmem_ld32(taddr + u * kIn + 2 * kGluHalf, ab);
-#pragma unroll
-                        for (int i = 0; i < 32; i++) {
-                            v[i] *= ab[i];
-                        }
-                    }
-                } else {
-                    tmem_ld32(taddr + u * kIn, v);
-                }
-                if (biased) {
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const float4 bb = reinterpret_cast<const float4*>(bs)[i];
-                        v[4 * i] += bb.x, v[4 * i + 1] += bb.y, v[4 * i + 2] += bb.z, v[4 * i + 3] += bb.w;
-                    }
-                }
-                int x = oc, y = rbase;
-                bool sig = false;
-                if constexpr (E == EPI_BF16) {
-                    sig = oc >= g.sig_from;
-                    if (g.vt && oc >= 2 * kTokC && oc < 3 * kTokC) {
-                        vt_unit(g, rbase, oc, v);
-                    }
-                }
-                if constexpr (E == EPI_MODS) {
-                    x = mx + 32 * u, y = my, sig = msig;
-                }
-                if (sig) {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float2 y = sigmoid_fast2(make_float2(v[i], v[i + 1]));
-                        v[i] = y.x, v[i + 1] = y.y;
-                    }
-                }
-                store_unit_tma(mo, st, x, y, v);
-            }
-            return;
-        }
-        if (lane_id() == 0) {
-            bulk_wait_read(); // a store of an earlier tile may still be reading the stage
-        }
-        __syncwarp();
-    }
-    EpiPre cur, nxt;
-    if (gp < units) {
-        epi_prefetch<E>(g, oc0 + 32 * gp, cur);
-    }
-    mbar_wait(tfull, tpar, abort);
-    tc_fence_after();
-#pragma unroll 1
-    for (int u = gp; u < units; u += 2) {
-        const int oc = oc0 + 32 * u;
-        if (u + 2 < units) {
-            epi_prefetch<E>(g, oc + 64, nxt);
-        }
-        float v[32];
-        if constexpr (E == EPI_GLU) {
-            // [gate 32 | proj 32] per unit of 64 accumulator columns -> 32 outputs
-            uint32_t ga[32], pr[32];
-            tmem_ld32_issue(taddr + u * kIn, ga);
-            tmem_ld32_issue(taddr + u * kIn + kGluHalf, pr);
-            tmem_ld_wait(ga);
-            tmem_ld_wait(pr);
-#pragma unroll
-            for (int i = 0; i < 32; i++) {
-                v[i] = silu_fast(__uint_as_float(ga[i])) * __uint_as_float(pr[i]);
-            }
-            if (kIn > 2 * kGluHalf) {
-                float ab[32];
-                tmem_ld32(taddr + u * kIn + 2 * kGluHalf, ab);
-#pragma unroll
-                for (int i = 0; i < 32; i++) {
-                    v[i] *= ab[i];
+        for (int u = gp; u < units; u += 2) {
+            const int oc = oc0 + 32 * u, x = x0 + 32 * u;
+            const bool biased = has_bias && oc < g.bias_cols; // (a unit has a bias or has none: bias_cols is a multiple of 32)
+            if (biased) {
+                __syncwarp();
+                bs[lane_id()] = bnext;
+                __syncwarp();
+                if (u + 2 < units && oc + 64 < g.bias_cols) {
+                    bnext = g.bias[oc + 64 + lane_id()];
                 }
             }
-        } else {
-            tmem_ld32(taddr + u * kIn, v);
-        }
-        if constexpr (E == EPI_PAIR) {
-            pair_unit(g, mo, st, rbase, oc, v);
-        } else {
+            float v[32];
+            if constexpr (E == EPI_GLU) {
+                uint32_t ga[32], pr[32];
+                tmem_ld32_issue(taddr + u * kIn, ga);
+                tmem_ld32_issue(taddr + u * kIn + kGluHalf, pr);
+                tmem_ld_wait(ga);
+                tmem_ld_wait(pr);
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                    const float2 z = __fmul2_rn(silu_fast2(make_float2(__uint_as_float(ga[i]), __uint_as_float(ga[i + 1]))),
+                                                make_float2(__uint_as_float(pr[i]), __uint_as_float(pr[i + 1])));
+                    v[i] = z.x, v[i + 1] = z.y;
+                }
+                if (kIn > 2 * kGluHalf) { // [gate | proj | a_to_b]: the third part multiplies
+                    float ab[32];
+                    tmem_ld32(taddr + u * kIn + 2 * kGluHalf, ab);
+#pragma unroll
+                    for (int i = 0; i < 32; i++) {
+                        v[i] *= ab[i];
+                    }
+                }
+            } else {
+                tmem_ld32(taddr + u * kIn, v);
+            }
+            if (biased) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const float4 bb = reinterpret_cast<const float4*>(bs)[i];
+                    v[4 * i] += bb.x, v[4 * i + 1] += bb.y, v[4 * i + 2] += bb.z, v[4 * i + 3] += bb.w;
+                }
+            }
+            bool sig = msig;
             if constexpr (E == EPI_BF16) {
+                sig = oc >= g.sig_from;
                 if (g.vt && oc >= 2 * kTokC && oc < 3 * kTokC) {
                     vt_unit(g, rbase, oc, v);
                 }
             }
-            const EpiUnit eu = epi_unit<E>(g, oc);
-            float4 t[4];
-            epi_turn(st, v, t);
-            epi_store<E>(g, eu, r0, cl, t, cur.b[0]);
-            epi_turn(st, v + kPiece, t);
-            epi_store<E>(g, eu, r0, kPiece + cl, t, cur.b[1]);
+            if (sig) {
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                    const float2 z = sigmoid_fast2(make_float2(v[i], v[i + 1]));
+                    v[i] = z.x, v[i + 1] = z.y;
+                }
+            }
+            bf16* own = rbase + lane_id() < g.m ? static_cast<bf16*>(g.out) + size_t(y + lane_id()) * (E == EPI_MODS ? kTokC : g.ldo) + x : nullptr;
+            store_unit(mo, st, x, y, whole, own, v);
         }
-        cur = nxt;
+    } else {
+        const int r0 = rbase + (lane_id() >> 2), cl = 4 * (lane_id() & 3), units = g.bn / 32;
+        EpiPre cur, nxt;
+        if (gp < units) {
+            epi_prefetch<E>(g, col0 + 32 * gp, cur);
+        }
+        mbar_wait(tfull, tpar, abort);
+        tc_fence_after();
+#pragma unroll 1
+        for (int u = gp; u < units; u += 2) {
+            const int oc = col0 + 32 * u;
+            if (u + 2 < units) {
+                epi_prefetch<E>(g, oc + 64, nxt);
+            }
+            float v[32];
+            tmem_ld32(taddr + u * 32, v);
+            if constexpr (E == EPI_PAIR) {
+                pair_unit(g, mo, st, rbase, oc, v);
+            } else {
+                float* o = static_cast<float*>(g.out) + oc + cl;
+                float4 t[4];
+                epi_turn(st, v, t);
+                epi_store<E>(g, o, r0, t, cur.b[0]);
+                epi_turn(st, v + kPiece, t);
+                epi_store<E>(g, o + kPiece, r0, t, cur.b[1]);
+            }
+            cur = nxt;
+        }
     }
 }
 

@@ -420,13 +420,6 @@ __device__ __forceinline__ float tanh_approx(float x) {
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float sigmoid_fast(float x) {
-    return fmaf(0.5f, tanh_approx(0.5f * x), 0.5f);
-}
-__device__ __forceinline__ float silu_fast(float x) {
-    const float h = 0.5f * x;
-    return fmaf(h, tanh_approx(h), h);
-}
 // two at a time: a packed instruction costs the pipe what two scalar ones do, but it is one to fetch and to issue. A GEMM's
 // epilogue is run from instructions that are mostly fetched anew (past 32 KB of code 6.5 cycles an instruction, within it
 // 1.5 to 4, measured with straight-line code): with these, and without the addition of a bias that is zero, ms per step
