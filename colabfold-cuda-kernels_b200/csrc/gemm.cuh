@@ -247,23 +247,10 @@ __device__ __forceinline__ float4 add4(float4 a, float4 b) {
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
 
-// f32 outputs, one piece after the turn: rows r0 + 8i, columns c..c+3 at o (of row 0). The bias of a unit's two pieces is
-// fetched one unit ahead (the first unit's before the accumulator is complete), because after a grid barrier every
-// such load is an L2 round trip.
-struct EpiPre {
-    float4 b[2];
-};
-template <int E> __device__ __forceinline__ void epi_prefetch(const GemmDesc& g, int c0, EpiPre& pre) {
-    if constexpr (E == EPI_F32) {
-        const int col = c0 + 4 * (lane_id() & 3);
-#pragma unroll
-        for (int pc = 0; pc < 2; pc++) {
-            pre.b[pc] = g.bias && col + kPiece * pc < g.bias_cols ? *reinterpret_cast<const float4*>(g.bias + col + kPiece * pc)
-                                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    }
-}
-template <int E> __device__ __forceinline__ void epi_store(const GemmDesc& g, float* o, int r0, const float4 (&t)[4], const float4& b) {
+// f32 outputs, one piece after the turn: rows r0 + 8i, columns c..c+3 (of the GEMM). The few of these with a bias fetch it here.
+template <int E> __device__ __forceinline__ void epi_store(const GemmDesc& g, int r0, int c, const float4 (&t)[4]) {
+    float* const o = static_cast<float*>(g.out) + c;
+    const float4 b = E == EPI_F32 && g.bias && c < g.bias_cols ? *reinterpret_cast<const float4*>(g.bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int row = r0 + 8 * i;
@@ -461,31 +448,25 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
         }
     } else {
         const int r0 = rbase + (lane_id() >> 2), cl = 4 * (lane_id() & 3), units = g.bn / 32;
-        EpiPre cur, nxt;
-        if (gp < units) {
-            epi_prefetch<E>(g, col0 + 32 * gp, cur);
-        }
         mbar_wait(tfull, tpar, abort);
         tc_fence_after();
 #pragma unroll 1
         for (int u = gp; u < units; u += 2) {
             const int oc = col0 + 32 * u;
-            if (u + 2 < units) {
-                epi_prefetch<E>(g, oc + 64, nxt);
-            }
-            float v[32];
-            tmem_ld32(taddr + u * 32, v);
             if constexpr (E == EPI_PAIR) {
+                float v[32];
+                tmem_ld32(taddr + u * 32, v);
                 pair_unit(g, mo, st, rbase, oc, v);
             } else {
-                float* o = static_cast<float*>(g.out) + oc + cl;
-                float4 t[4];
-                epi_turn(st, v, t);
-                epi_store<E>(g, o, r0, t, cur.b[0]);
-                epi_turn(st, v + kPiece, t);
-                epi_store<E>(g, o + kPiece, r0, t, cur.b[1]);
+#pragma unroll 1
+                for (int k = 0; k < 32; k += kPiece) {
+                    float v[16];
+                    tmem_ld16(taddr + u * 32 + k, v);
+                    float4 t[4];
+                    epi_turn(st, v, t);
+                    epi_store<E>(g, r0, oc + k + cl, t);
+                }
             }
-            cur = nxt;
         }
     }
 }
