@@ -273,7 +273,7 @@ template <int E> __device__ __forceinline__ void epi_store(const GemmDesc& g, in
 // The pair logits of one unit: a tile's rows are 128 consecutive keys k of one query q (rbase
 // encodes q·ktiles·128 + k0), the column is the table (block·16 + head); base-2 logits. Keys past the real tokens
 // are masked, keys past the padded extent (a multiple of 64: a warp's 32 are in or out together) are not stored. The
-// 32 tables x 32 keys leave the warp's stage as one block of the tables' planes; stored by the lanes themselves, 2 bytes to
+// 32 tables x 32 keys leave the warp's stage as one block of the tables' planes, clipped at the last table; stored by the lanes themselves, 2 bytes to
 // a lane and 32 addresses to a unit, a tile took 22,000 cycles (2048 tokens: the whole build 4.4 ms).
 __device__ __forceinline__ void pair_unit(const GemmDesc& g, const CUtensorMap* mo, float* st, int rbase, int c0, const float (&v)[32]) {
     const int q = rbase / (g.ktiles * kBM), k0 = rbase % (g.ktiles * kBM), l = lane_id(), k = k0 + l;
@@ -283,7 +283,8 @@ __device__ __forceinline__ void pair_unit(const GemmDesc& g, const CUtensorMap* 
         const size_t pq = size_t(q) * g.ldn + (masked ? 0 : k);
         const float mean = tw.pcs[2 * pq], rstd = tw.pcs[2 * pq + 1];
         const float extra = kp().plx ? bf_to_f32(tw.plx[pq]) : 0.f;
-        const float ws = tw.plws[c0 + l], wb = tw.plb[c0 + l]; // (lane l: of table c0 + l)
+        const bool table = c0 + l < kp().nb * kPairHeads; // (with an odd number of blocks the last unit has 16)
+        const float ws = table ? tw.plws[c0 + l] : 0.f, wb = table ? tw.plb[c0 + l] : 0.f; // (lane l: of table c0 + l)
         if (l == 0) {
             bulk_wait_read(); // the previous store has read the stage
         }

@@ -308,16 +308,16 @@ static int encode_rows_store_map(CUtensorMap* m, const void* base, size_t rows, 
 // of the grid for 8 tiles, 320 x 5: 2.46 -> 2.28 ms per step, and 128 where that is bound by the loads, 1024 x 5: 5.32 -> 5.04.)
 // 32 columns only while half of the grid has no tile even then: a row block waits for twice the arrivals of a GEMM with
 // 64, and its rows are read twice as often (32 x 1: 0.973 -> 0.951 ms per step with this limit, 0.987 without; 256 x 1 with two
-// calls per step 2.311 -> 2.254).
+// calls per step 2.311 -> 2.254), or where nothing wider divides n (the pair logits of 6 blocks, say). 0: no width does.
 inline int choose_bn(size_t m, int n, int kblocks, int grid, int max_bn = kMaxBN, int unit = 32) {
-    int best = unit < 64 ? 64 : unit;
+    int best = 0;
     double best_cost = 1e300;
     for (int bn = 8 * unit; bn >= unit; bn /= 2) {
         if (n % bn || bn > max_bn) {
             continue;
         }
         const size_t tiles = (m + kBM - 1) / kBM * size_t(n / bn);
-        if (bn < 64 && 2 * tiles > size_t(grid)) {
+        if (bn < 64 && best && 2 * tiles > size_t(grid)) {
             continue;
         }
         const double kblock = (kStageA + bn * kBK * 2) / 83.0, epi = 18.0 * bn;
@@ -687,7 +687,7 @@ static int make_launch(Launch& L, const Template& t, const Device& dev, const vo
         {TM_B_WQKVG, IN_WQKVG, nb * kQKVG, kTokC, rt, kQKVG}, {TM_B_WO, IN_WO, nb * kTokC, kTokC, rt, kTokC, kResidMaxBnBf},
         {TM_B_W1, IN_W1, nb * t.tw1, kTokC, rt, t.tw1, kMaxBN, t.tw1 / (kTokHidden / kGluHalf)}, {TM_B_W2, IN_W2, nb * kTokC, kTokHidden, rt, kTokC, kResidMaxBnBf},
         {TM_B_WTB, IN_WTB, kAtomC, kTokC, rt, kAtomC}, {TM_B_WAGGR, IN_WAGGR, kTokC, kAtomC, ra, kTokC},
-        {TM_B_PLW, IN_PLW, nb * kPairHeads, size_t(t.plc), size_t(N) * N, int(nb * kPairHeads)},
+        {TM_B_PLW, IN_PLW, nb * kPairHeads, size_t(t.plc), size_t(N) * N, pair_columns(t.nb)},
         {TM_B_ENC_WQG, IN_ENC_WQG, 3 * 2 * kAtomC, kAtomC, ra, 2 * kAtomC}, {TM_B_ENC_WKV, IN_ENC_WKV, 3 * 2 * kAtomC, kAtomC, ra, 2 * kAtomC},
         {TM_B_ENC_WO, IN_ENC_WO, 3 * kAtomC, kAtomC, ra, kAtomC, kResidMaxBnF32}, {TM_B_ENC_W1, IN_ENC_W1, size_t(3 * t.aw1), kAtomC, ra, t.aw1, kMaxBN, t.aw1 / (kAtomHidden / kGluHalf)},
         {TM_B_ENC_W2, IN_ENC_W2, 3 * kAtomC, kAtomHidden, ra, kAtomC, kResidMaxBnF32},
@@ -698,6 +698,9 @@ static int make_launch(Launch& L, const Template& t, const Device& dev, const vo
     for (const BMap& m : bmaps) {
         const int kb = int(m.cols / kBK) * (m.id == TM_B_ENC_W1 || m.id == TM_B_DEC_W1 ? 2 : 1); // (hi | lo inputs: W1 of the atoms twice)
         const int bn = choose_bn(m.m, m.n, kb, dev.sms, m.max_bn, m.unit);
+        if (bn == 0) { // (no model that make_template takes)
+            return fail(E_SHAPE, "MkSample: no column tile divides the " + std::to_string(m.n) + " columns of a GEMM");
+        }
         p.bn[m.id] = bn;
         if (int e = encode_map(&L.tmap[m.id], in[m.in], m.rows, m.cols, m.cols, bn)) {
             return e;

@@ -178,6 +178,12 @@ struct alignas(64) Launch {
     Program prog;
 };
 
+// Columns of the pair-logit GEMM: its epilogue takes units of 32, and an odd number of blocks ends with half of one. The
+// rows of PLW that are missing there arrive as zeros, and the store of the planes is clipped.
+__host__ __device__ constexpr int pair_columns(int blocks) {
+    return (blocks * kPairHeads + 31) / 32 * 32;
+}
+
 // ---- GEMM work descriptor: C[m][n] = A[m][k] · W[n][k]ᵀ then a fused epilogue
 enum Epi : int {
     EPI_BF16,  // bf16(C + bias on the first bias_cols, sigmoid from sig_from on)

@@ -248,10 +248,10 @@ __device__ inline GemmDesc gemm_tok(const KP& p, int b, int which) {
     return g;
 }
 // one-time pair logits of all blocks: row tiles are (query q, 128 keys) read straight out of PC
-// (row q·Nb + k), columns the nb·16 tables
+// (row q·Nb + k), columns the nb·16 tables (pair_columns)
 __device__ inline GemmDesc gemm_pair(const KP& p) {
     const int ktiles = cdiv(p.N, kBM);
-    GemmDesc g = make_gemm(p, TM_A_PC, TM_B_PLW, 0, p.N * ktiles * kBM, p.nb * kPairHeads, p.plc, EPI_PAIR, p.buf.plg, 0);
+    GemmDesc g = make_gemm(p, TM_A_PC, TM_B_PLW, 0, p.N * ktiles * kBM, pair_columns(p.nb), p.plc, EPI_PAIR, p.buf.plg, 0);
     g.map_o = TM_O_PLG, g.fl = GF_NFAST; // (the column tiles of a row tile together: PC, the largest input, is read from HBM once)
     g.np = p.npb, g.ldn = p.Nb, g.ktiles = ktiles, g.nreal = p.N, g.npreal = p.np;
     return g;

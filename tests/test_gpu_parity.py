@@ -731,12 +731,17 @@ def test_pair_logits(lib, make_case, n_tok, bucket, masked):
     if bucket:
         x, meta = synth.pad_to_bucket(x, meta, bucket, bucket // 4)
     x[synth.IN["TMASK"]][:masked] = 0
+    check_pair_logits(lib, x, meta, n_tok, masked)
+
+
+def check_pair_logits(lib, x, meta, n, masked):
+    """PLG of the first n tokens of meta's bucket, the first `masked` of them masked."""
+    nb = meta["N"]
     lib.setup(x, meta)
-    n, nb = n_tok, meta["N"]
-    if bucket:
-        lib.set_extent(n_tok, n_tok // 4)
+    if n < nb:
+        lib.set_extent(n, n // 4)
     lib.run(mode=1, dbg_stop=1, xn=np.zeros(meta["S"] * nb * 24 * 3, np.float32), t=mg.T_ONCE)
-    if bucket:
+    if n < nb:
         lib.set_extent(0, 0)
     np_ = (nb + 63) // 64 * 64
     got = lib.read("PLG").reshape(-1, np_, np_)[:, :n, :(n + 63) // 64 * 64].astype(np.float64)
@@ -753,3 +758,26 @@ def test_pair_logits(lib, make_case, n_tok, bucket, masked):
     assert (np.abs(got[:, :, :n] - want)[:, :, real] <= bound[:, :, real]).all()
     off = got[:, :, ~np.concatenate([real, np.zeros(got.shape[2] - n, bool)])]
     assert off.size == 0 or np.abs(off / (-1e9 * np.log2(np.e)) - 1).max() < 2.0 ** -8
+
+
+@pytest.mark.parametrize("blocks,n_tok,samples", [(1, 40, 1), (1, 132, 2), (2, 104, 1), (3, 132, 1), (5, 72, 2), (6, 132, 1), (22, 100, 1), (23, 72, 1)])
+def test_pair_logits_of_any_number_of_blocks(lib, oracle_lib, blocks, n_tok, samples):
+    """Models of 1 to 24 token blocks are taken: 16 tables a block, so their number need not be a multiple of any column tile.
+    All of the tables (as test_pair_logits), where a tile of 32 is chosen for the small number of tiles and where it is the
+    only one that divides them, half of the last one past the tables or not; the denoiser's output against the oracle, and
+    on completion counters bit for bit that on barriers."""
+    x, meta = synth.make_inputs(n_tok, samples=samples, steps=8, nb=blocks)
+    check_pair_logits(lib, x, meta, n_tok, 0)
+    oracle_lib.setup(x, meta)
+    xn = synth.noisy_positions(meta, mg.T_ONCE)
+    oracle_lib.run(mode=1, xn=xn, t=mg.T_ONCE)
+    out = {}
+    try:
+        for on in (True, False):
+            lib.set_flow(on)
+            lib.run(mode=1, xn=xn, t=mg.T_ONCE)
+            out[on] = lib.read("OUT").copy()
+    finally:
+        lib.set_flow(True)
+    assert driver.max_rel_err(out[True], oracle_lib.read("OUT")) < GATE
+    assert np.array_equal(out[True], out[False])
