@@ -59,6 +59,30 @@ __global__ void wait_test_kernel(Control* ctl, long long limit) {
         }
     }
 }
+// One warp waiting for completion counters in one of the kernel's three ways: 1 flow_wait by one lane, one counter after the
+// other; 2 flow_wait_warp, a lane to each counter; 3 FlowWait in single looks, as a GEMM's TMA warp polls.
+__global__ void counter_wait_test_kernel(Control* ctl, const unsigned int* cnt, int counters, unsigned int target, int form, long long limit) {
+    KP* p = reinterpret_cast<KP*>(smem_base() + kKpOff);
+    SmemCtl* sc = smem_ctl();
+    if (threadIdx.x == 0) {
+        p->ctl = ctl, p->wait_cycles = limit;
+        sc->abort = 0;
+    }
+    __syncthreads();
+    if (form == 2) {
+        flow_wait_warp(cnt, 0, counters - 1, target, &sc->abort);
+    } else if (form == 3) {
+        for (int c = 0; c < counters; c++) {
+            FlowWait w(cnt + c * kFlowPitch, target, &sc->abort);
+            while (!uni(int(w.ready()))) {
+            }
+            w.acquire();
+        }
+    } else if (threadIdx.x == 0) {
+        flow_wait(cnt, 0, counters - 1, target, &sc->abort);
+    }
+    __syncwarp();
+}
 // the sampler's Philox words and normals for one counter
 __global__ void philox_test_kernel(uint32_t idx, uint32_t step, uint32_t sample, uint32_t stream, uint32_t k0, uint32_t k1,
                                    uint32_t* words, float* z) {
@@ -279,6 +303,46 @@ int mk_wait_test(long long cycles, float* ms) {
     cudaMemcpy(&c, ctl, sizeof c, cudaMemcpyDeviceToHost);
     cudaEventDestroy(e0), cudaEventDestroy(e1);
     cudaFree(ctl);
+    return err == cudaSuccess ? int(c.status) : -1;
+}
+// One warp waits in way `form` (counter_wait_test_kernel) for `counters` completion counters, all of them complete but, with
+// missing >= 0, that one, for at most `cycles` SM cycles. Returns the status word the kernel left (0: it saw all of
+// them complete; 2: the wait gave up), or -1 on a CUDA error or bad arguments; *ms gets the launch time.
+int mk_counter_wait_test(int form, int counters, int missing, long long cycles, float* ms) {
+    constexpr int kMost = 64;
+    constexpr unsigned int kTarget = 96;
+    if (form < 1 || form > 3 || counters < 1 || counters > kMost || missing >= counters || cycles < 1) {
+        return -1;
+    }
+    std::vector<unsigned int> words(kMost * kFlowPitch, 0);
+    for (int c = 0; c < counters; c++) {
+        words[c * kFlowPitch] = c == missing ? kTarget - 1 : kTarget;
+    }
+    const size_t bytes = words.size() * sizeof(unsigned int);
+    Device dev;
+    Control* ctl = nullptr;
+    unsigned int* cnt = nullptr;
+    if (device_state(dev) || cudaMalloc(&ctl, sizeof(Control)) != cudaSuccess || cudaMemset(ctl, 0, sizeof(Control)) != cudaSuccess ||
+        cudaMalloc(&cnt, bytes) != cudaSuccess || cudaMemcpy(cnt, words.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaFree(ctl), cudaFree(cnt);
+        return -1;
+    }
+    cudaFuncSetAttribute(reinterpret_cast<const void*>(counter_wait_test_kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlloc);
+    cudaEvent_t e0, e1;
+    cudaEventCreate(&e0), cudaEventCreate(&e1);
+    cudaEventRecord(e0);
+    counter_wait_test_kernel<<<1, 32, kSmemAlloc>>>(ctl, cnt, counters, kTarget, form, cycles);
+    cudaEventRecord(e1);
+    const cudaError_t err = cudaDeviceSynchronize();
+    float el = 0.f;
+    cudaEventElapsedTime(&el, e0, e1);
+    if (ms) {
+        *ms = el;
+    }
+    Control c{};
+    cudaMemcpy(&c, ctl, sizeof c, cudaMemcpyDeviceToHost);
+    cudaEventDestroy(e0), cudaEventDestroy(e1);
+    cudaFree(ctl), cudaFree(cnt);
     return err == cudaSuccess ? int(c.status) : -1;
 }
 // The sampler's Philox4x32-10 words and Box-Muller normals for counter (idx, step, sample, stream) and

@@ -119,12 +119,17 @@ int mk_gemm_test(const uint16_t* A, const uint16_t* W, float* C, int M, int N, i
  *                     OUT is NaN. (0, 0) restores production.
  *  mk_wait_test       one thread waits `cycles` SM cycles on an mbarrier that nothing arrives at;
  *                     returns the status the kernel left (2, as it must) or -1 on a CUDA error.
+ *  mk_counter_wait_test  one warp waits for `counters` (1 to 64) completion counters in one of the kernel's
+ *                     ways (form 1: one lane, one after the other; 2: a lane to each; 3: single looks);
+ *                     with missing >= 0 that one never completes and the wait lasts `cycles` SM cycles.
+ *                     Returns the status the kernel left (0, or 2 with one missing) or -1 on an error.
  *  mk_philox_test     the sampler's Philox4x32-10 words (4) and Box-Muller normals (4) for counter
  *                     (idx, step, sample, stream) and key seed, computed on the device
  *                     (src/diffusion/rng.cuh:14-46). */
 int mk_set_attn_skew(int cycles);
 int mk_set_wait_test(long long cycles, int extra);
 int mk_wait_test(long long cycles, float* ms);
+int mk_counter_wait_test(int form, int counters, int missing, long long cycles, float* ms);
 int mk_philox_test(uint32_t idx, uint32_t step, uint32_t sample, uint32_t stream, uint64_t seed, uint32_t* words, float* z);
 
 /* Status word of the last mk_run: 0 ok, 1 a grid barrier gave up, 2 a wait inside a phase gave up; where it

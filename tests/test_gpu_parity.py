@@ -581,6 +581,21 @@ def test_waits_give_up_and_the_launch_ends(lib, make_case):
     assert np.array_equal(lib.read("POS"), want)
 
 
+@pytest.mark.parametrize("form", [1, 2, 3])
+@pytest.mark.parametrize("counters", [1, 5, 32, 33, 40])
+def test_waits_for_completion_counters_give_up(lib, form, counters):
+    """The kernel's three ways to wait for completion counters (one lane, counter by counter; a warp with a lane to each, 32 at
+    a time; single looks by a warp) return at once when every counter is there, and give up with status 2 within the
+    limit, here about a millisecond, where one of them, the first or the last, stays one short."""
+    f = lib.lib.mk_counter_wait_test
+    f.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.POINTER(ctypes.c_float)]
+    ms = ctypes.c_float(0)
+    assert f(form, counters, -1, 1 << 21, ctypes.byref(ms)) == 0
+    for missing in {0, counters - 1}:
+        assert f(form, counters, missing, 1 << 21, ctypes.byref(ms)) == 2  # ST_PIPE_TIMEOUT
+        assert 0.9 < ms.value < 100.0  # 2^21 cycles at 2 GHz or less
+
+
 def outgrown_reference_logits(n, rng):
     """PLX rows by class of query row: flat; one later chunk of 64 keys far above the others; a ramp up, every chunk far
     above the one before; a ramp down; a step of 4.5 (the maximum grows by 2^6.5, but the chunk adds up to more than 2^8).
