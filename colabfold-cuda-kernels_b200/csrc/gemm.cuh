@@ -630,7 +630,7 @@ struct FlowWait {
 };
 // One thread waits until the counters [c0, c1] have reached target, one after the other; what it then reads is what
 // the signalling warps wrote.
-__device__ __forceinline__ bool flow_wait(const unsigned int* cnt, int c0, int c1, unsigned int target, volatile int* abort) {
+__device__ __forceinline__ void flow_wait(const unsigned int* cnt, int c0, int c1, unsigned int target, volatile int* abort) {
     const long long t0 = clock64();
     unsigned int looks = 0;
     if (*abort) { // a wait inside this CTA gave up earlier: tell the grid, which would otherwise wait for this CTA's units
@@ -639,18 +639,17 @@ __device__ __forceinline__ bool flow_wait(const unsigned int* cnt, int c0, int c
     for (int c = c0; c <= c1; c++) {
         while (ld_acquire(cnt + c * kFlowPitch) < target) {
             if (*abort) {
-                return false;
+                return;
             }
             // another CTA gave up (its units will not come), or this wait ran out: the launch drains
             if (++looks % 32 == 0 && (ld_relaxed(&kp().ctl->status) != ST_OK || clock64() - t0 > wait_limit())) {
                 fail_launch(ST_PIPE_TIMEOUT, 0);
                 *abort = 1;
-                return false;
+                return;
             }
         }
     }
     fence_async_global();
-    return true;
 }
 // The same by a whole warp, a lane to a counter: the counters of a sample of the token attention (5 at 512 tokens, 16 at
 // 2048) then cost one trip to L2 when the last of them is complete, not one each (ms per step 512 x 1 1.349 -> 1.333, 512 x 5 2.358

@@ -50,10 +50,6 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -187,6 +183,7 @@ __device__ __forceinline__ void umma_bf16_ts_k64_el(uint32_t el, uint32_t tmem_d
         : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc), "r"(el)
         : "memory");
 }
+// the mbarrier gets one arrival when every MMA issued so far by this lane has completed
 __device__ __forceinline__ void umma_commit_el(uint32_t el, uint32_t bar) {
     asm volatile(
         "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
@@ -225,22 +222,13 @@ __device__ __forceinline__ void fence_mbar_init() {
 __device__ __forceinline__ void fence_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
-__device__ __forceinline__ void fence_async_all() {
-    asm volatile("fence.proxy.async;" ::: "memory");
-}
-// the same for global memory only: what the grid barrier needs on either side
+// generic-proxy accesses of global memory ordered with those of the async proxy: what the grid barrier needs on either side, and
+// what the reader of a completion counter needs behind its acquire
 __device__ __forceinline__ void fence_async_global() {
     asm volatile("fence.proxy.async.global;" ::: "memory");
 }
 
-// ---- TMA: one 2D tile, 128-byte swizzle decided by the tensor map
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        :
-        : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
-        : "memory");
-}
+// ---- TMA stores (the loads are with the roles' instructions above)
 // one 2D tile from shared memory to global memory (rows and columns past the tensor's extent are
 // clipped), as part of this thread's bulk async-group
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, const void* smem_src) {
@@ -264,9 +252,6 @@ __device__ __forceinline__ void bulk_wait_read() {
 }
 __device__ __forceinline__ void bulk_wait_done() {
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-}
-__device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
 // ---- tcgen05
@@ -304,22 +289,6 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
 // and [10,13) = 1), both K-major (bits 15, 16 = 0), N >> 3 in [17,23), M >> 4 in [24,29).
 __device__ __forceinline__ uint32_t umma_idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24);
-}
-// D[tmem] (+)= A[smem] · B[smem]ᵀ; issued by one thread
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                          uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        :
-        : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// the mbarrier gets one arrival when every UMMA issued so far by this thread has completed
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
 }
 // 32 lanes x 32 consecutive f32 columns: thread l of the warp gets lane (base lane + l)
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
