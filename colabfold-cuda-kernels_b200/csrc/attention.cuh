@@ -170,9 +170,13 @@ __device__ __forceinline__ void atom_half_compute(AtomHalf& a, const KP& p, int 
 // AO = softmax(q·kᵀ/√32 + 1e9(QMASK-1)(KMASK-1) + APL)·v ⊙ g (reference: src/diffusion/attention.cuh:313-434)
 __device__ CCK_PHASE_FN void atom_attention(const KP& p, Deal& d, const AtomW& w, int b) {
     // Where even the halves (16 queries) of the units find a warp each, a half is a unit: the window is gathered twice, but
-    // a warp is through with it in some three quarters of the time, and one unit per warp is all these folds have (ms
-    // per step 32 x 1 0.953 -> 0.931, 512 x 1 1.324 -> 1.298). With more units than that, three rounds of halves would take longer than
-    // two of units. Both kinds go through the same code, out of line: 61 x 5 1.047 -> 1.042 against inlined and unrolled.
+    // a warp is through with it in three quarters of the time, and one unit per warp is all these folds have. Past that the
+    // halves need a second round of the grid where the units still need one. us of a decoder phase on 148 SMs, halves and
+    // whole: 32 units 9.0 and 12.7, 320 10.3 and 14.0, 736 (1472 halves for 1480 warps, the last of the first kind) 10.8
+    // and 14.5; 752 16.7 and 14.5, 1024 17.2 and 14.6, 1456 17.4 and 15.0. (Further on three rounds of halves are a little
+    // shorter than two of units, 1600 units 23.3 and 24.4, 1920 24.5 and 25.6, which is 0.3 % of a step, and four longer,
+    // 2560 31.7 and 25.8: not told apart.)
+    // Both kinds go through the same code, out of line: 61 x 5 1.047 -> 1.042 ms per step against inlined and unrolled.
     const int full = p.NS * kAtomHeads * p.S;
     const int halves = 2 * full <= int(gridDim.x) * kAwWarps ? 2 : 1, units = halves * full;
     bf16* sm = reinterpret_cast<bf16*>(smem_base() + warp_id() * kAwBytes);

@@ -274,7 +274,7 @@ template <int E> __device__ __forceinline__ void epi_store(const GemmDesc& g, in
 // encodes q·ktiles·128 + k0), the column is the table (block·16 + head); base-2 logits. Keys past the real tokens
 // are masked, keys past the padded extent (a multiple of 64: a warp's 32 are in or out together) are not stored. The
 // 32 tables x 32 keys leave the warp's stage as one block of the tables' planes, clipped at the last table; stored by the lanes themselves, 2 bytes to
-// a lane and 32 addresses to a unit, a tile took 22,000 cycles (2048 tokens: the whole build 4.4 ms).
+// a lane and 32 addresses to a unit, a tile took 22,000 cycles (a run of one step, 2048 x 1: 7.33 -> 4.62 ms; 512 x 5: 2.63 -> 2.47).
 __device__ __forceinline__ void pair_unit(const GemmDesc& g, const CUtensorMap* mo, float* st, int rbase, int c0, const float (&v)[32]) {
     const int q = rbase / (g.ktiles * kBM), k0 = rbase % (g.ktiles * kBM), l = lane_id(), k = k0 + l;
     if (q < g.nreal && k0 < g.npreal) {
@@ -359,7 +359,7 @@ __device__ __forceinline__ void store_unit(const CUtensorMap* mo, float* st, int
 
 // The epilogue of one 128 x bn accumulator held in TMEM columns [acc, acc + bn), by the eight
 // worker warps: units of 32 output columns alternate between the two groups. Waits for the
-// accumulator itself, after the first unit's global loads are under way.
+// accumulator itself; of a bf16 output with a bias, the first unit's bias is under way by then.
 template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g, const CUtensorMap* mo, uint32_t acc, int row0, int col0,
                                                                uint64_t* tfull, uint32_t tpar, volatile int* abort) {
     const int q = work_quarter(), gp = work_group(), rbase = row0 + q * 32;
@@ -570,8 +570,9 @@ __device__ __forceinline__ unsigned int* flow_cnt(const KP& p, int which) {
 }
 // The calling warp's part of a unit is stored: its lanes' writes (and lane 0's TMA stores, which the
 // caller has waited for) are published with one release add per counter in [c0, c1]. The proxy fence that a
-// TMA read of ordinary stores needs is on the reader's side, behind its acquire (FlowWait, flow_wait): one on
-// the path from the write to the read is enough, and here it would be paid by every warp (0.5 %).
+// TMA read of ordinary stores needs is on the reader's side, behind its acquire (FlowWait::acquire, flow_wait,
+// flow_wait_warp): one on the path from the write to the read is enough, and here it would be paid by every warp (0.5 %).
+// No writer has one, so every wait that a TMA load may follow must keep its own, whatever it costs.
 __device__ __forceinline__ void flow_signal(unsigned int* cnt, int c0, int c1) {
     __syncwarp();
     if (lane_id() == 0) {

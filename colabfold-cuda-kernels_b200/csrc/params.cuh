@@ -44,10 +44,11 @@ struct Bufs {
 };
 // The token blocks run without grid barriers: adaLN -> QKVG -> attention -> WO -> adaLN -> W1 -> W2, and the adaLN
 // rows of the next block (or the final LayerNorm) follow W2 in the same way. A unit of a later operation
-// waits for the units it reads, counted per block of 128 token rows: every worker warp adds one when its part of a
-// unit has been stored (TX0, TX: every adaLN row of the attention's and of the transition's input adds one). The
-// counters are zeroed at the start of a launch and count on through it: a unit of the e-th token block of the
-// launch waits for (e + 1) times what one block adds.
+// waits for the units it reads, counted per block of 128 token rows: a GEMM tile adds the number of worker warps, at
+// once, when the last of them has stored its part; a softmax warp adds one for its rows of an attention item (TO),
+// and every adaLN row of the attention's and of the transition's input adds one (TX0, TX). The counters are zeroed
+// at the start of a launch and count on through it: a unit of the e-th token block of the launch waits for (e + 1)
+// times what one block adds.
 // What a block writes while units of the block before may still be reading: only QKVG and VT, which the attention
 // items of a whole sample read. They alternate between two buffers: what the one of the block before last held
 // has been read when this block's rows exist, since every row went through that block's attention.

@@ -251,7 +251,7 @@ __device__ CCK_PHASE_FN void token_adaln2(const KP& p, Deal& d, int b) {
 // Token rows under the completion counters: every CTA takes one contiguous run of rows, so that it
 // depends on one or two blocks of 128 rows, and a warp starts a row when the tiles of the GEMM that
 // wrote ACT over the row's block are complete (cnt counts on through the launch: target is the
-// count after the GEMM of the current token block). Returns false when the wait gave up.
+// count after the GEMM of the current token block).
 struct FlowRows {
     int r0, r1, ok, step;
     const unsigned int* cnt;

@@ -62,8 +62,8 @@ __device__ __forceinline__ Op flow_next(const Program& prog, const KP& p, Flow& 
 // The schedule state of the calling thread (shared memory). Its address is worked out anew each time, so that the
 // compiler does not hold it in a register over an operation, and so is the parameter's (SmemCtl::launch): a called
 // function that needs all registers saves what its caller holds to local memory and loads it back when it is
-// through, from L2, since every look at a completion counter empties L1. The token attention saved eight registers
-// (ms per step with none: 61 x 5 1.099 -> 1.081, 256 x 5 1.547 -> 1.531, 512 x 5 2.382 -> 2.363, 384 x 1 on barriers 1.367 -> 1.339).
+// through, from L2, since every look at a completion counter empties L1. The token attention saved eight registers (one, by now;
+// ms per step with none: 61 x 5 1.099 -> 1.081, 256 x 5 1.547 -> 1.531, 512 x 5 2.382 -> 2.363, 384 x 1 on barriers 1.367 -> 1.339).
 __device__ __forceinline__ Run& run_state() {
     uint32_t t;
     asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
@@ -252,7 +252,7 @@ __device__ inline GemmDesc gemm_tok(const KP& p, int b, int which) {
 __device__ inline GemmDesc gemm_pair(const KP& p) {
     const int ktiles = cdiv(p.N, kBM);
     GemmDesc g = make_gemm(p, TM_A_PC, TM_B_PLW, 0, p.N * ktiles * kBM, pair_columns(p.nb), p.plc, EPI_PAIR, p.buf.plg, 0);
-    g.map_o = TM_O_PLG, g.fl = GF_NFAST; // (the column tiles of a row tile together: PC, the largest input, is read from HBM once)
+    g.map_o = TM_O_PLG, g.fl = GF_NFAST; // (the column tiles of a row tile together: PC, the largest input, is read from HBM once; a run of one step, 2048 x 1: 4.62 -> 4.54 ms)
     g.np = p.npb, g.ldn = p.Nb, g.ktiles = ktiles, g.nreal = p.N, g.npreal = p.np;
     return g;
 }
