@@ -1,7 +1,9 @@
 """The kernel lookup table, as the reference's tests/test_package.py pins it, for the B200 build."""
 import ctypes
+import json
 import os
 import subprocess
+import sys
 
 import pytest
 
@@ -50,3 +52,13 @@ def test_library_needs_libc_only(product_lib_path):
     out = subprocess.run(["ldd", product_lib_path], capture_output=True, text=True).stdout
     needed = {line.split()[0].split(".so")[0] for line in out.splitlines() if "=>" in line}
     assert needed <= {"libc", "libm", "libdl", "libpthread", "librt"}, out
+
+
+def test_bench_reference_arm_has_no_stand_in():
+    """The reference arm runs the reference or says in one line that it cannot: no number of this repository's own code."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = subprocess.run([sys.executable, os.path.join(root, "bench.py"), "--impl", "reference", "--gpus", "1", "--steps", "2", "--warmup", "1"],
+                         capture_output=True, text=True, cwd=root, timeout=120)
+    assert run.returncode == 0, run.stderr
+    line = json.loads(run.stdout)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
