@@ -390,7 +390,7 @@ template <int E> __device__ __forceinline__ void epilogue_tile(const GemmDesc& g
 #pragma unroll 1
         for (int u = gp; u < units; u += 2) {
             const int oc = oc0 + 32 * u, x = x0 + 32 * u;
-            const bool biased = has_bias && oc < g.bias_cols; // (a unit has a bias or has none: bias_cols is a multiple of 32)
+            const bool biased = has_bias && oc < g.bias_cols; // (a unit has a bias or has none: bias_cols is a multiple of 32. Zeros added instead: 256 x 5 and 512 x 5 0.3 to 0.5 % more, small folds the same)
             if (biased) {
                 __syncwarp();
                 bs[lane_id()] = bnext;
@@ -571,7 +571,7 @@ __device__ __forceinline__ unsigned int* flow_cnt(const KP& p, int which) {
 // The calling warp's part of a unit is stored: its lanes' writes (and lane 0's TMA stores, which the
 // caller has waited for) are published with one release add per counter in [c0, c1]. The proxy fence that a
 // TMA read of ordinary stores needs is on the reader's side, behind its acquire (FlowWait::acquire, flow_wait,
-// flow_wait_warp): one on the path from the write to the read is enough, and here it would be paid by every warp (0.5 %).
+// flow_wait_warp): one on the path from the write to the read is enough, and here it would be paid by every warp (0.1 to 0.3 %).
 // No writer has one, so every wait that a TMA load may follow must keep its own, whatever it costs.
 __device__ __forceinline__ void flow_signal(unsigned int* cnt, int c0, int c1) {
     __syncwarp();
@@ -584,8 +584,8 @@ __device__ __forceinline__ void flow_signal(unsigned int* cnt, int c0, int c1) {
 // The same for a GEMM tile, by the eight worker warps together: each counts itself in shared memory (acquire and
 // release at the CTA's scope), and the one that comes last publishes all eight parts with one release add. A release at
 // the grid's scope waits for the stores in flight and takes some 1500 cycles; eight of them at once got in each
-// other's way (ms per step 256 x 5 1.576 -> 1.547, 512 x 1 1.401 -> 1.364, 512 x 5 2.412 -> 2.367, 61 x 5 1.138 -> 1.114,
-// with the proxy fence out as above). The token attention and the row passes, whose warps finish further apart, lose by it.
+// other's way (ms per step 32 x 1 0.892 -> 0.889, 64 x 5 1.042 -> 1.017, 256 x 5 1.512 -> 1.482, 512 x 1 1.288 -> 1.259,
+// 512 x 5 2.314 -> 2.279, 1024 x 5 0.3 %). The token attention and the row passes, whose warps finish further apart, lose by it.
 // Tile t is counted in slot t % 4: a warp that is through with tile t + 3 has seen its accumulator, whose buffer tile
 // t + 1 held, so that every warp had read that one and, before it, counted itself for tile t.
 __device__ __forceinline__ void flow_signal_tile(unsigned int* cnt, unsigned int* parts) {

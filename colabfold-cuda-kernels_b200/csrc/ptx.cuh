@@ -391,8 +391,8 @@ __device__ __forceinline__ float tanh_approx(float x) {
 }
 // two at a time: a packed instruction costs the pipe what two scalar ones do, but it is one to fetch and to issue. A GEMM's
 // epilogue is run from instructions that are mostly fetched anew (past 32 KB of code 6.5 cycles an instruction, within it
-// 1.5 to 4, measured with straight-line code): with these, and without the addition of a bias that is zero, ms per step
-// 61 x 5 1.102 -> 1.083, 256 x 5 1.528 -> 1.517, 512 x 1 1.333 -> 1.325, 512 x 5 2.340 -> 2.321.
+// 1.5 to 4, measured with straight-line code): ms per step against the scalar forms 32 x 1 0.892 -> 0.889, 64 x 5 1.022 ->
+// 1.017, 256 x 5 1.485 -> 1.482, 512 x 5 2.283 -> 2.279.
 __device__ __forceinline__ float2 tanh2(float2 x) {
     return make_float2(tanh_approx(x.x), tanh_approx(x.y));
 }
